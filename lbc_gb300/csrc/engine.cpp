@@ -99,6 +99,14 @@ Solver::Solver(const CaseDesc &d) : d_(d) {
     if (!check_cuda(cudaStreamCreateWithPriority(&stream_, cudaStreamNonBlocking, hi), "cudaStreamCreate")) return;
     use_retaining_pool();
     if (!build_geometry()) return;
+    // The integer form of the FP64 step has no use for large blocks: 64 x 2
+    // packs the most warps on an SM (1024^2: 74.5 us per step with 64 x 4,
+    // 72.8 with 64 x 2). A grid of at most a warp per SM sub-partition takes
+    // one-warp blocks, so that no two of its warps share one.
+    if (arith_ == ARITH_INT) {
+        const long long warps = (long long)((d_.Nx + 31) / 32) * d_.Ny;
+        block_ = warps <= 4LL * launch::sm_count() ? dim3(32, 1, 1) : dim3(64, 2, 1);
+    }
     ok_ = true;
     set_autotune(tune_default_mode());
 }
@@ -138,6 +146,14 @@ bool Solver::build_geometry() {
     omega0_ = d_.omega ? d_.omega[0] : 1.0;
     if (d_.omega)
         for (size_t n = 1; n < N && uniform; n++) uniform = (d_.omega[n] == omega0_);
+    // The integer form of the FP64 step (fp64_int.cuh) is written for lbc's
+    // weights and needs om 2^-9 exact and om |f - f_eq| finite.
+    auto plain_omega = [](double om) { return om >= 1e-100 && om <= 4.0; };
+    const double lw[9] = {4.0 / 9.0, 1.0 / 9.0, 1.0 / 9.0, 1.0 / 9.0, 1.0 / 9.0, 1.0 / 36.0, 1.0 / 36.0, 1.0 / 36.0, 1.0 / 36.0};
+    bool lbc_int = d_.store == STORE_F64 && !d_.fma64 && std::equal(lw, lw + 9, d_.w) && plain_omega(omega0_);
+    if (!uniform)
+        for (size_t n = 1; n < N && lbc_int; n++) lbc_int = plain_omega(d_.omega[n]);
+    arith_ = d_.fma64 ? ARITH_FMA : lbc_int ? ARITH_INT : ARITH_LBC;
 
     // Stages from the Boundary list.
     bool nonperiodic_seen = false;
@@ -1030,7 +1046,7 @@ bool Solver::launch_step_kernels(int src, int dst, bool collide, bool write_macr
     StepParams p = step_params(src, dst, write_macro, bparity);
     if (!forces) p.mem_partials = nullptr;
     if (d_.store == STORE_F64) {
-        CK(launch::step_exact(p, has_flags_, collide, block_, s, d_.fma64));
+        CK(launch::step_exact(p, has_flags_, collide, block_, s, arith_));
     } else {
         const FastStepParams fp = fast_params(p);
         // The special nodes first, as an ordinary launch, then the clean pairs
@@ -1426,6 +1442,10 @@ Batch::Batch(const std::vector<Solver *> &cases) : cases_(cases) {
             return;
         }
     }
+    // One arithmetic per launch: lbc's sequence when some case needs it (the
+    // integer form gives the same bits).
+    arith_ = cases_[0]->arith();
+    for (Solver *c : cases_) if (c->arith() != arith_) arith_ = ARITH_LBC;
     // FP64 batches (FP64-issue bound, long) run at the lowest stream priority,
     // shifted-storage batches at the highest, so that when both run at once
     // (the server's lanes) free SMs go to the short, memory-bound FP32 steps
@@ -1713,7 +1733,7 @@ bool Batch::build() {
 bool Batch::launch_batched(int sel) {
     if (store_ == STORE_F64) {
         CK(launch::step_batch_exact((const StepParams *)d_sp_, d_tiles_, ntiles_, sel, tws_,
-                                    grid_, stream_, cases_[0]->fma64()));
+                                    grid_, stream_, arith_));
     } else {
         // the clean pairs, then the special nodes overlapping their tail
         CK(launch::step_batch_shifted((const FastStepParams *)d_sp_, d_tiles_, ntiles_, sel, tws_,

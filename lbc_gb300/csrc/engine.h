@@ -134,6 +134,8 @@ class Solver {
     int Ny() const { return d_.Ny; }
     int store() const { return d_.store; }
     bool fma64() const { return d_.fma64; }
+    // ARITH_*: the arithmetic of the FP64 step kernels.
+    int arith() const { return arith_; }
     // The public storage code (lbm_gpu.h), LBM_GPU_F64_FMA included.
     int storage_code() const { return d_.fma64 ? 3 : d_.store; }
     cudaStream_t stream() const { return stream_; }
@@ -266,6 +268,7 @@ class Solver {
     Link *d_links_ = nullptr;
     double *d_omega_ = nullptr;
     double omega0_ = 1.0;
+    int arith_ = ARITH_LBC;
     int *d_colbase_ = nullptr, *d_rowbase_ = nullptr;
     int nslots_ = 0;
     double *d_bandf_ = nullptr;  // FP64 storage
@@ -364,7 +367,7 @@ class Batch {
     bool capture_pair();
 
     std::vector<Solver *> cases_;
-    int store_ = STORE_F64;
+    int store_ = STORE_F64, arith_ = ARITH_LBC;
     bool ok_ = false;
     cudaStream_t stream_ = nullptr;
     long long nodes_ = 0;

@@ -134,7 +134,7 @@ cudaError_t record(const RecordTask *tasks, int n, int store, const void *dst, c
 // FP64 (kernels_exact.cu): lbc's rounding sequence, or with fma set the
 // fused multiply-add arithmetic (moments_fma / collide_fma)
 cudaError_t step_exact(const StepParams &p, bool flags, bool collide, dim3 block, cudaStream_t s,
-                       bool fma = false);
+                       int arith = ARITH_LBC);
 // collide: the finish of fused members applies the collision (false only in
 // the final step of a run, which leaves pre-collision populations).
 // after_bulk (here, stage_batch and force_reduce): the previous launch in s is
@@ -164,7 +164,7 @@ cudaError_t fp64_rate(int blocks, int iters, double *sink, cudaStream_t s);
 // batches of cases (tile list = int4 {case, x0, y0, case has wall links})
 // Tiles of 2^tws x 2^(8 - tws) nodes, tws in [5, 8].
 cudaError_t step_batch_exact(const StepParams *sp, const int4 *tiles, int ntiles,
-                             int sel, int tws, int grid, cudaStream_t s, bool fma = false);
+                             int sel, int tws, int grid, cudaStream_t s, int arith = ARITH_LBC);
 int step_batch_exact_grid();
 // One level of a batch's Boundary lists (n entries): block b steps points
 // blocks[b].y .. + kStageBatchPoints(F64) - 1 of entry blocks[b].x, or, for

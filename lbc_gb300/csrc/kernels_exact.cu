@@ -19,6 +19,7 @@
 #include <cmath>
 #include <cstdio>
 
+#include "fp64_int.cuh"
 #include "kernels.h"
 #include "lbm_device.cuh"
 #include "pdl.cuh"
@@ -37,9 +38,11 @@ namespace lbm {
 // its momentum-exchange terms (src/core/compute_force_mem.c:51-58), computes
 // moments (src/core/compute_macroscopic_fields.c:23-46) and, unless it is written
 // by an edge BC, collides (src/core/collision.c:22-38) and stores.
-// FMA: moments_fma / collide_fma instead of lbc's rounding sequence (the same
-// step to rounding, in 74 FP64 instructions per node instead of 125).
-template <bool FLAGS, bool COLLIDE, bool FMA = false>
+// ARITH: ARITH_LBC, lbc's rounding sequence on the FP64 pipe (125 FP64
+// instructions per node); ARITH_INT, the same bits with 24 of them
+// (fp64_int.cuh; nodes outside its ranges take ARITH_LBC's); ARITH_FMA,
+// moments_fma / collide_fma (the same step to rounding, 74).
+template <bool FLAGS, bool COLLIDE, int ARITH>
 __device__ __forceinline__ void step_node_exact(const StepParams &p, int i, int j, double &mfx,
                                                 double &mfy, bool &link) {
     {
@@ -113,17 +116,22 @@ __device__ __forceinline__ void step_node_exact(const StepParams &p, int i, int 
             }
             if (!(FLAGS && (fl & NF_BCW))) {
                 double rho, ux, uy;
-                if (FMA) moments_fma(f, p.hFx, p.hFy, p.has_force != 0, rho, ux, uy);
-                else moments_exact(f, p.hFx, p.hFy, rho, ux, uy);
+                const double om = COLLIDE ? (p.omega ? p.omega[dn] : p.omega0) : 0.0;
+                bool done = false;
+                if (ARITH == ARITH_INT)
+                    done = fi::step_node<COLLIDE>(f, p.w, p.has_force != 0, p.hFx, p.hFy, om, p.Fx, p.Fy, rho, ux, uy);
+                if (!done) {
+                    if (ARITH == ARITH_FMA) moments_fma(f, p.hFx, p.hFy, p.has_force != 0, rho, ux, uy);
+                    else moments_exact(f, p.hFx, p.hFy, rho, ux, uy);
+                }
                 if (p.write_macro) { p.rho[dn] = rho; p.ux[dn] = ux; p.uy[dn] = uy; }
                 if (slot >= 0) {
                     p.bandm_next[slot] = rho;
                     p.bandm_next[(size_t)p.nslots + slot] = ux;
                     p.bandm_next[2 * (size_t)p.nslots + slot] = uy;
                 }
-                if (COLLIDE) {
-                    const double om = p.omega ? p.omega[dn] : p.omega0;
-                    if (FMA) collide_fma(f, p.w[0], p.w[1], p.w[5], rho, ux, uy, om, p.has_force != 0, p.Fx, p.Fy);
+                if (COLLIDE && !done) {
+                    if (ARITH == ARITH_FMA) collide_fma(f, p.w[0], p.w[1], p.w[5], rho, ux, uy, om, p.has_force != 0, p.Fx, p.Fy);
                     else collide_exact(f, p.w, rho, ux, uy, om, p.has_force != 0, p.Fx, p.Fy);
                 }
 #pragma unroll
@@ -133,14 +141,14 @@ __device__ __forceinline__ void step_node_exact(const StepParams &p, int i, int 
     }
 }
 
-template <bool FLAGS, bool COLLIDE, bool FMA>
-__global__ void __launch_bounds__(256) k_step_exact(const StepParams p) {
+template <bool FLAGS, bool COLLIDE, int ARITH>
+__global__ void __launch_bounds__(256, ARITH == ARITH_INT ? 3 : 1) k_step_exact(const StepParams p) {
     pdl_launch_dependents();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = blockIdx.y * blockDim.y + threadIdx.y;
     double mfx = 0.0, mfy = 0.0;
     bool link = false;
-    if (i < p.Nx && j < p.Ny) step_node_exact<FLAGS, COLLIDE, FMA>(p, i, j, mfx, mfy, link);
+    if (i < p.Nx && j < p.Ny) step_node_exact<FLAGS, COLLIDE, ARITH>(p, i, j, mfx, mfy, link);
     if (FLAGS && p.mem_partials) segment_reduce2_store(mfx, mfy, link, i, j, p.Nx, p.seg_slot, p.mem_partials);
 }
 
@@ -151,8 +159,8 @@ __global__ void __launch_bounds__(256) k_step_exact(const StepParams p) {
 // grids and different geometries share the launch. Force partials go to each
 // case's own segment slots (td.w != 0: the tile contains wall links), reduced
 // per case by k_force_reduce exactly as when the case runs alone.
-template <bool FMA>
-__global__ void __launch_bounds__(256) k_step_batch_exact(const StepParams *__restrict__ sp,
+template <int ARITH>
+__global__ void __launch_bounds__(256, ARITH == ARITH_INT ? 3 : 1) k_step_batch_exact(const StepParams *__restrict__ sp,
                                                           const int4 *__restrict__ tiles, int ntiles,
                                                           int sel, int tws) {
     pdl_launch_dependents();
@@ -165,9 +173,9 @@ __global__ void __launch_bounds__(256) k_step_batch_exact(const StepParams *__re
         bool link = false;
         const bool in = i < p.Nx && j < p.Ny;
         if (p.flags) {
-            if (in) step_node_exact<true, true, FMA>(p, i, j, mfx, mfy, link);
+            if (in) step_node_exact<true, true, ARITH>(p, i, j, mfx, mfy, link);
         } else {
-            if (in) step_node_exact<false, true, FMA>(p, i, j, mfx, mfy, link);
+            if (in) step_node_exact<false, true, ARITH>(p, i, j, mfx, mfy, link);
         }
         if (td.w && p.mem_partials) segment_reduce2_store(mfx, mfy, link, i, j, p.Nx, p.seg_slot, p.mem_partials);
     }
@@ -768,21 +776,22 @@ cudaError_t fp64_rate(int blocks, int iters, double *sink, cudaStream_t s) {
 
 static dim3 grid2(int Nx, int Ny, dim3 b) { return dim3((Nx + b.x - 1) / b.x, (Ny + b.y - 1) / b.y); }
 
-template <bool FMA>
+template <int ARITH>
 static void step_exact_t(const StepParams &p, bool flags, bool collide, dim3 g, dim3 block, cudaStream_t s) {
     if (flags) {
-        if (collide) k_step_exact<true, true, FMA><<<g, block, 0, s>>>(p);
-        else k_step_exact<true, false, FMA><<<g, block, 0, s>>>(p);
+        if (collide) k_step_exact<true, true, ARITH><<<g, block, 0, s>>>(p);
+        else k_step_exact<true, false, ARITH><<<g, block, 0, s>>>(p);
     } else {
-        if (collide) k_step_exact<false, true, FMA><<<g, block, 0, s>>>(p);
-        else k_step_exact<false, false, FMA><<<g, block, 0, s>>>(p);
+        if (collide) k_step_exact<false, true, ARITH><<<g, block, 0, s>>>(p);
+        else k_step_exact<false, false, ARITH><<<g, block, 0, s>>>(p);
     }
 }
 
-cudaError_t step_exact(const StepParams &p, bool flags, bool collide, dim3 block, cudaStream_t s, bool fma) {
+cudaError_t step_exact(const StepParams &p, bool flags, bool collide, dim3 block, cudaStream_t s, int arith) {
     const dim3 g = grid2(p.Nx, p.Ny, block);
-    if (fma) step_exact_t<true>(p, flags, collide, g, block, s);
-    else step_exact_t<false>(p, flags, collide, g, block, s);
+    if (arith == ARITH_FMA) step_exact_t<ARITH_FMA>(p, flags, collide, g, block, s);
+    else if (arith == ARITH_INT) step_exact_t<ARITH_INT>(p, flags, collide, g, block, s);
+    else step_exact_t<ARITH_LBC>(p, flags, collide, g, block, s);
     return cudaGetLastError();
 }
 
@@ -796,11 +805,12 @@ cudaError_t stage_group(const StageGroup &g, int store, bool collide, bool after
 }
 
 cudaError_t step_batch_exact(const StepParams *sp, const int4 *tiles, int ntiles,
-                             int sel, int tws, int grid, cudaStream_t s, bool fma) {
+                             int sel, int tws, int grid, cudaStream_t s, int arith) {
     if (ntiles == 0) return cudaSuccess;
     if (tws < 5 || tws > 8) return cudaErrorInvalidValue;
-    if (fma) k_step_batch_exact<true><<<grid, 256, 0, s>>>(sp, tiles, ntiles, sel, tws);
-    else k_step_batch_exact<false><<<grid, 256, 0, s>>>(sp, tiles, ntiles, sel, tws);
+    if (arith == ARITH_FMA) k_step_batch_exact<ARITH_FMA><<<grid, 256, 0, s>>>(sp, tiles, ntiles, sel, tws);
+    else if (arith == ARITH_INT) k_step_batch_exact<ARITH_INT><<<grid, 256, 0, s>>>(sp, tiles, ntiles, sel, tws);
+    else k_step_batch_exact<ARITH_LBC><<<grid, 256, 0, s>>>(sp, tiles, ntiles, sel, tws);
     return cudaGetLastError();
 }
 

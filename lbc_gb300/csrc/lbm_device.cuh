@@ -94,6 +94,9 @@ __host__ __device__ inline bool bc_is_column(int kind) {
            kind == BC_PRES_OUT_REG;
 }
 
+// Arithmetic of the FP64 step (step_node_exact).
+enum : int { ARITH_LBC = 0, ARITH_FMA = 1, ARITH_INT = 2 };
+
 // Storage policies: FP64 stores f as is; FP32/FP16 store the shifted deviation
 // g_k = f_k - w_k.
 template <typename T> struct Store;
