@@ -150,10 +150,12 @@ bool Solver::build_geometry() {
     // weights and needs om 2^-9 exact and om |f - f_eq| finite.
     auto plain_omega = [](double om) { return om >= 1e-100 && om <= 4.0; };
     const double lw[9] = {4.0 / 9.0, 1.0 / 9.0, 1.0 / 9.0, 1.0 / 9.0, 1.0 / 9.0, 1.0 / 36.0, 1.0 / 36.0, 1.0 / 36.0, 1.0 / 36.0};
-    bool lbc_int = d_.store == STORE_F64 && !d_.fma64 && std::equal(lw, lw + 9, d_.w) && plain_omega(omega0_);
+    bool lbc_int = d_.store == STORE_F64 && std::equal(lw, lw + 9, d_.w) && plain_omega(omega0_);
     if (!uniform)
         for (size_t n = 1; n < N && lbc_int; n++) lbc_int = plain_omega(d_.omega[n]);
-    arith_ = d_.fma64 ? ARITH_FMA : lbc_int ? ARITH_INT : ARITH_LBC;
+    // It serves LBM_GPU_F64_FMA too: lbc's own bits, and faster than the fused
+    // multiply-adds (1531 x 1021: 223 us per step with them, 110 this way).
+    arith_ = lbc_int ? ARITH_INT : d_.fma64 ? ARITH_FMA : ARITH_LBC;
 
     // Stages from the Boundary list.
     bool nonperiodic_seen = false;
@@ -815,7 +817,7 @@ bool Solver::launch_collide(int b, cudaStream_t s) {
     c.Fx = d_.Fx; c.Fy = d_.Fy;
     for (int k = 0; k < 9; k++) c.w[k] = d_.w[k];
     c.from_pops = fields_are_moments_ ? 1 : 0;
-    c.fma = d_.fma64 ? 1 : 0;
+    c.fma = arith_ == ARITH_FMA ? 1 : 0;
     if (d_.store == STORE_F64) CK(launch::collide_exact(c, s));
     else CK(launch::collide_shifted(c, d_.store, s));
     return true;
@@ -830,6 +832,7 @@ StepParams Solver::step_params(int src, int dst, bool write_macro, int bparity) 
     p.flags = d_flags_; p.link_off = d_link_off_; p.links = d_links_;
     p.seg_clean = d_seg_clean_; p.seg_words = seg_words_;
     p.omega = d_omega_; p.omega0 = omega0_;
+    p.fma = arith_ == ARITH_FMA ? 1 : 0;
     p.has_force = (d_.Fx != 0.0 || d_.Fy != 0.0);
     p.Fx = d_.Fx; p.Fy = d_.Fy; p.hFx = 0.5 * d_.Fx; p.hFy = 0.5 * d_.Fy;
     for (int k = 0; k < 9; k++) p.w[k] = d_.w[k];
@@ -1442,10 +1445,11 @@ Batch::Batch(const std::vector<Solver *> &cases) : cases_(cases) {
             return;
         }
     }
-    // One arithmetic per launch: lbc's sequence when some case needs it (the
-    // integer form gives the same bits).
+    // One arithmetic per launch; for a mix, one kernel that asks each case
+    // (the integer form's cases take lbc's sequence there: the same bits).
     arith_ = cases_[0]->arith();
-    for (Solver *c : cases_) if (c->arith() != arith_) arith_ = ARITH_LBC;
+    for (Solver *c : cases_)
+        if (c->arith() != arith_) arith_ = ARITH_MIXED;
     // FP64 batches (FP64-issue bound, long) run at the lowest stream priority,
     // shifted-storage batches at the highest, so that when both run at once
     // (the server's lanes) free SMs go to the short, memory-bound FP32 steps

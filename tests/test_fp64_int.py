@@ -29,3 +29,50 @@ def test_integer_form_matches_fp64(tmp_path, force):
     assert wrong == 0, r.stdout
     # most of the sampled nodes are ordinary ones, which it must accept
     assert refused < nodes // 10, r.stdout
+
+
+def _other_weights():
+    """A periodic flow with weights that keep lbc's pair symmetry but are not
+    lbc's: outside the integer form."""
+    from lbc_gb300 import cases
+    case, st = cases.taylor_green(48, 40, 0.04, 0.56)
+    w = case.w.copy()
+    w[0] += 4e-3
+    w[1:5] -= 1e-3
+    case.w = w
+    f = cases.equilibrium(st.rho, st.u, st.v, w)
+    return case, cases.State(f, f.copy(), st.rho, st.u, st.v)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("storage", ["f64", "f64fma"])
+def test_other_weights_take_the_fp64_pipe(oracle, storage):
+    """Weights the integer form does not serve, alone and in a batch with a
+    case it does: F64 equals the oracle bit for bit, F64_FMA to 1e-12, and each
+    case of the batch equals itself alone."""
+    import numpy as np
+    import casezoo
+    from lbc_gb300 import GpuBatch, GpuSolver, STORAGE
+    built = [_other_weights(), casezoo.build("cylinder_wake_small")[0], _other_weights()]
+    alone, solvers = [], []
+    for case, st in built:
+        s = GpuSolver(case, STORAGE[storage])
+        s.set_state(st)
+        s.run(20)
+        alone.append(s.get_state())
+        s = GpuSolver(case, STORAGE[storage])
+        s.set_state(st)
+        solvers.append(s)
+    GpuBatch(solvers).run(20)
+    for s, a in zip(solvers, alone):
+        got = s.get_state()
+        for fld in ("f", "f_new", "rho", "u", "v"):
+            assert np.array_equal(getattr(got, fld), getattr(a, fld), equal_nan=True), fld
+    case, st = built[0]
+    oracle.run(case, st, 20)
+    for fld in ("f", "f_new", "rho", "u", "v"):
+        a, b = getattr(alone[0], fld), getattr(st, fld)
+        if storage == "f64":
+            assert np.array_equal(a, b), fld
+        else:
+            assert np.max(np.abs(a - b)) <= 1e-12 * np.max(np.abs(b)), fld
