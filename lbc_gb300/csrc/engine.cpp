@@ -116,6 +116,7 @@ Solver::~Solver() {
     if (vtk_ev_) cudaEventDestroy(vtk_ev_);
     if (h_vtk_) cudaFreeHost(h_vtk_);
     if (pair_exec_) cudaGraphExecDestroy(pair_exec_);
+    if (multi_exec_) cudaGraphExecDestroy(multi_exec_);
     for (void *p : allocs_) cudaFreeAsync(p, stream_);
     if (stream_) cudaStreamDestroy(stream_);
 }
@@ -1344,6 +1345,56 @@ void Solver::set_autotune(int mode) {
     }
 }
 
+// Steps per pass of kernels_multi.cu for this case, 0: one at a time. Measured
+// per step (us) against the one-step kernel, Taylor-Green, FP32: 64^2 3.08 ->
+// 2.31, 512^2 5.13 -> 3.60, 1024^2 9.24 -> 6.95, 2048^2 46.4 -> 20.3, 4096^2
+// 173.5 -> 71.4. Four levels, except where the grid gives too few warps to hide
+// four dependent collisions per row: 512 x 256 3.08 with two, 3.60 with four;
+// 768^2 the same with either. FP16's one-step kernel moves half the bytes, so
+// only larger grids gain: 512^2 4.11 -> 4.87, 768^2 6.17 -> 6.43, 1024^2 9.24 ->
+// 8.73, 4096^2 112.5 -> 80.4.
+int Solver::multi_levels() const {
+    const long long n = (long long)d_.Nx * d_.Ny;
+    if (d_.store == STORE_F64 || has_flags_ || d_omega_ || !rec_host_.empty()) return 0;
+    if (d_.Nx < 8 || d_.Ny < 8 || plane_ >= (1LL << 31)) return 0;
+    if (d_.store == STORE_F16) return n >= (1LL << 20) ? 4 : 0;
+    return n >= (1LL << 17) && n < (1LL << 19) ? 2 : 4;
+}
+
+// Warps a pass is split into: 8 per SM while the state is in the L2 cache
+// (1024^2 FP32 6.95 us per step, 7.46 with 12), the 12 that fit beyond that;
+// FP16 keeps more in flight (4096^2: 92 us with 12, 81 with 24).
+int Solver::multi_warps() const {
+    const long long n = (long long)d_.Nx * d_.Ny;
+    return launch::sm_count() * (n < (1LL << 21) ? 8 : d_.store == STORE_F16 ? 24 : 12);
+}
+
+// Two passes (cur -> other -> cur) captured once and replayed.
+bool Solver::capture_multi() {
+    if (multi_exec_ && multi_cur_ == cur_) return true;
+    if (multi_exec_) {
+        cudaGraphExecDestroy(multi_exec_);
+        multi_exec_ = nullptr;
+    }
+    cudaGraph_t g = nullptr;
+    CK(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
+    cudaError_t e = cudaSuccess;
+    for (int b = 0; b < 2 && e == cudaSuccess; b++)
+        e = launch::multi_plain(fast_params(step_params(cur_ ^ b, cur_ ^ b ^ 1, false, 0)), d_.store, multi_levels(),
+                                multi_warps(), stream_);
+    const cudaError_t e2 = cudaStreamEndCapture(stream_, &g);
+    if (e != cudaSuccess || e2 != cudaSuccess) {
+        if (g) cudaGraphDestroy(g);
+        CK(e);
+        CK(e2);
+    }
+    e = cudaGraphInstantiate(&multi_exec_, g, 0);
+    cudaGraphDestroy(g);
+    CK(e);
+    multi_cur_ = cur_;
+    return true;
+}
+
 // One fused step cur -> other, as inside run().
 bool Solver::trial_step() {
     if (!launch_step(cur_, 1 - cur_, true, false, parity_)) return false;
@@ -1402,6 +1453,11 @@ bool Solver::run(int nsteps) {
         const int used = tune_online(remaining);
         if (used < 0) return false;
         remaining -= used;
+    }
+    const int lv = multi_levels();
+    if (lv > 0 && remaining >= 2 * lv) {
+        if (!capture_multi()) return false;
+        for (; remaining >= 2 * lv; remaining -= 2 * lv) CK(cudaGraphLaunch(multi_exec_, stream_));
     }
     if (remaining >= 2) {
         if (!capture_pair()) return false;

@@ -246,6 +246,9 @@ class Solver {
     int nprobes_ = 0, probe_cap_ = 0;
     bool launch_collide(int b, cudaStream_t s = nullptr);
     bool capture_pair();
+    int multi_levels() const;
+    int multi_warps() const;
+    bool capture_multi();
     bool trial_step();
     int tune_online(int avail);
     int tune_mode_ = 0;
@@ -297,6 +300,8 @@ class Solver {
     cudaGraphExec_t pair_exec_ = nullptr;
     int pair_cur_ = -1, pair_parity_ = -1;
     bool graph_valid_ = false;
+    cudaGraphExec_t multi_exec_ = nullptr;
+    int multi_cur_ = -1;
     size_t dev_bytes_ = 0;
     long long steps_done_ = 0;
     std::vector<void *> allocs_;

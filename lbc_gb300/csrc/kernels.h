@@ -122,6 +122,11 @@ struct RecordTask {
     double hFx, hFy;             // half the body force: lbc's u = (j + F / 2) / rho
 };
 
+// Several steps per pass (kernels_multi.cu): threads per block, and the columns
+// a strip of 64 gives up on either side for `levels` steps (even).
+constexpr int kMultiThreads = 128;
+__host__ __device__ constexpr int multi_halo(int levels) { return (levels + 1) / 2 * 2; }
+
 namespace launch {
 // Records of one step: tasks[0 .. n). Alone: the step's populations are at
 // dst. In a batch (spbase set): case cs's are the dst of its step parameters
@@ -139,6 +144,9 @@ cudaError_t step_exact(const StepParams &p, bool flags, bool collide, dim3 block
 // the final step of a run, which leaves pre-collision populations).
 // after_bulk (here, stage_batch and force_reduce): the previous launch in s is
 // a bulk step kernel; the launch overlaps its tail (pdl.cuh).
+// `levels` (2..4) steps of a fully periodic case without a flag word, with one
+// omega, in one pass; warps: how many to split the grid into.
+cudaError_t multi_plain(const FastStepParams &p, int store, int levels, int warps, cudaStream_t s);
 cudaError_t stage_group(const StageGroup &g, int store, bool collide, bool after_bulk, cudaStream_t s);
 cudaError_t collide_exact(const CollideParams &p, cudaStream_t s);
 cudaError_t collide_aos_exact(const CollideAosParams &p, cudaStream_t s);

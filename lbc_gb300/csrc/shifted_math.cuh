@@ -1,0 +1,173 @@
+// shifted_math.cuh -- storage access and arithmetic of the shifted-storage
+// kernels (g_k = f_k - w_k in FP32 or FP16, collision in FP32).
+#pragma once
+#include "lbm_device.cuh"
+
+namespace lbm {
+
+template <typename T> struct SV;
+// rnd: the value as the storage type would hold it. Pre-collision values that
+// are computed rather than loaded (bounce-back interpolation, edge BCs) are
+// rounded to the storage type before the collision, so a run split into
+// chunks (whose boundaries store and reload them) gives the same bits.
+// ld2 / st2: two adjacent nodes of one row (an even column: the pair is 8- or
+// 4-byte aligned because the pitch and the planes are multiples of 64 nodes).
+template <> struct SV<float> {
+    static __device__ __forceinline__ float ld(const float *p) { return __ldg(p); }
+    static __device__ __forceinline__ float ld_plain(const float *p) { return *p; }
+    static __device__ __forceinline__ void st(float *p, float v) { *p = v; }
+    static __device__ __forceinline__ float rnd(float v) { return v; }
+    static __device__ __forceinline__ float2 ld2(const float *p) { return __ldg((const float2 *)p); }
+    static __device__ __forceinline__ void st2(float *p, float2 v) { *(float2 *)p = v; }
+};
+template <> struct SV<__half> {
+    static __device__ __forceinline__ float ld(const __half *p) { return __half2float(__ldg(p)); }
+    static __device__ __forceinline__ float ld_plain(const __half *p) { return __half2float(*p); }
+    static __device__ __forceinline__ void st(__half *p, float v) { *p = __float2half_rn(v); }
+    static __device__ __forceinline__ float rnd(float v) { return __half2float(__float2half_rn(v)); }
+    static __device__ __forceinline__ float2 ld2(const __half *p) { return __half22float2(__ldg((const __half2 *)p)); }
+    static __device__ __forceinline__ void st2(__half *p, float2 v) { *(__half2 *)p = __float22half2_rn(v); }
+};
+
+// ---------------------------------------------------------------- lane math
+// The arithmetic of one node (float) or of two adjacent nodes at once (float2,
+// Blackwell's packed FP32 instructions). Every operation is one correctly
+// rounded IEEE operation with no contraction left to the compiler, so a node
+// gets the same bits whichever form, kernel or launch shape computed it.
+__device__ __forceinline__ float v_add(float a, float b) { return __fadd_rn(a, b); }
+__device__ __forceinline__ float v_sub(float a, float b) { return __fsub_rn(a, b); }
+__device__ __forceinline__ float v_mul(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ float v_fma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+// 1/a correctly rounded for 2^-126 <= a <= 2^125: the hardware's estimate and
+// one Newton step (checked against __frcp_rn on every float of that range; the
+// intrinsic itself has a branch, which keeps the compiler from interleaving the
+// steps of kernels_multi.cu).
+__device__ __forceinline__ float v_rcp_seed(float a) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a));
+    return r;
+}
+__device__ __forceinline__ float v_rcp(float a) {
+    const float r = v_rcp_seed(a);
+    return __fmaf_rn(r, __fmaf_rn(-a, r, 1.0f), r);
+}
+// lbc's floor on the density (compute_macroscopic_fields.c:27), and v_rcp's
+// range above; NaN stays NaN.
+__device__ __forceinline__ float v_floor_rho(float a) {
+    float r;
+    asm("max.NaN.f32 %0, %1, %2;\n\tmin.NaN.f32 %0, %0, %3;" : "=&f"(r) : "f"(a), "f"(1e-16f), "f"(0x1p125f));
+    return r;
+}
+__device__ __forceinline__ float2 v_add(float2 a, float2 b) { return __fadd2_rn(a, b); }
+// a - b rounded once: b * (-1) is exact.
+__device__ __forceinline__ float2 v_sub(float2 a, float2 b) { return __ffma2_rn(b, make_float2(-1.f, -1.f), a); }
+__device__ __forceinline__ float2 v_mul(float2 a, float2 b) { return __fmul2_rn(a, b); }
+__device__ __forceinline__ float2 v_fma(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
+__device__ __forceinline__ float2 v_rcp(float2 a) {
+    const float2 r = make_float2(v_rcp_seed(a.x), v_rcp_seed(a.y));
+    return __ffma2_rn(r, __ffma2_rn(make_float2(-a.x, -a.y), r, make_float2(1.0f, 1.0f)), r);
+}
+__device__ __forceinline__ float2 v_floor_rho(float2 a) { return make_float2(v_floor_rho(a.x), v_floor_rho(a.y)); }
+template <class V> __device__ __forceinline__ V v_splat(float x);
+template <> __device__ __forceinline__ float v_splat<float>(float x) { return x; }
+template <> __device__ __forceinline__ float2 v_splat<float2>(float x) { return make_float2(x, x); }
+
+// h1 = fl(3 w1), h5 = (1 - 2 h1) / 4, as the host computes them.
+__device__ __forceinline__ void shifted_h(float w1, float &h1, float &h5) {
+    h1 = __fmul_rn(3.0f, w1);
+    h5 = __fmul_rn(__fsub_rn(1.0f, __fmul_rn(2.0f, h1)), 0.25f);
+}
+
+// Shifted moments: delta rho = sum g, j = sum c g (sum c w = 0). Jx, Jy are the
+// momentum including half the body force (rho u of lbc); jx, jy without it.
+template <class V>
+__device__ __forceinline__ void moments_v(const V g[9], V hFx, V hFy, V &dr, V &rho, V &ux, V &uy, V &Jx,
+                                          V &Jy, V &jx, V &jy) {
+    dr = v_add(v_add(v_add(v_add(g[0], g[1]), v_add(g[2], g[3])), v_add(v_add(g[4], g[5]), v_add(g[6], g[7]))),
+               g[8]);
+    jx = v_add(v_add(v_sub(g[1], g[3]), v_sub(g[5], g[6])), v_sub(g[8], g[7]));
+    jy = v_sub(v_add(v_sub(g[2], g[4]), v_add(g[5], g[6])), v_add(g[7], g[8]));
+    rho = v_floor_rho(v_add(v_splat<V>(1.0f), dr));
+    const V inv = v_rcp(rho);
+    Jx = v_add(jx, hFx);
+    Jy = v_add(jy, hFy);
+    ux = v_mul(Jx, inv);
+    uy = v_mul(Jy, inv);
+}
+
+// One pair of directions (k, opposite) of the equilibrium: X = w (dr + 4.5 J c
+// - rt) is the even part, h o the odd part, added to X with one rounding
+// (X +- h o as FMAs: rounding h o first doubles the FP32 velocity error of a
+// Taylor-Green run against FP64). The odd part takes the momentum without
+// the half force, o = c.j; the force enters the odd part separately (see
+// collide_v).
+template <class V>
+__device__ __forceinline__ void geq_pair(float w, float h, V dr, V c, V J, V o, V nrt, V &a, V &b) {
+    const V X = v_mul(v_splat<V>(w), v_add(dr, v_fma(v_mul(v_splat<V>(4.5f), J), c, nrt)));
+    a = v_fma(v_splat<V>(h), o, X);
+    b = v_fma(v_splat<V>(-h), o, X);
+}
+
+// BGK + Guo on shifted populations, g' = g + om (geq - g) + (1 - om/2) F_k,
+// with geq_k = w_k (drho + rho (3 c.u + 4.5 (c.u)^2 - 1.5 u.u)) built so that
+// its mass and momentum are the node's own by construction: the odd part of
+// each pair is h (c.J) with FP32 coefficients h1 = fl(3 w1) and
+// h5 = (1 - 2 h1) / 4 whose sum rule 2 h1 + 4 h5 = 1 holds exactly, the linear
+// term uses J = rho u directly (no division), and the rest population closes
+// the mass. Rounded weights would otherwise bias every collision's momentum by
+// ~1e-8 in the same direction, an error that grows linearly with the steps.
+//
+// With a body force, J = j + F/2 would round F/2 (~1e-7) against j: an error of
+// the same sign every step, which drove a forced channel 6.6e-5 away from FP64
+// in 20,000 steps. Instead the odd part relaxes towards h (c.j) and the whole
+// odd forcing, om h c.F/2 + (1 - om/2) 3 w c.F = h c.F (h = 3 w), is added as
+// one small term; the even forcing is (1 - om/2) w S, S = 9 (c.u)(c.F) - 3 u.F.
+// The relaxation and the forcing are summed first (one FMA) and added to g with
+// a single rounding. Channel 256 x 64 against FP64 after 20,000 steps: u L2
+// error 5.0e-7 (6.6e-5 before).
+template <class V, bool FORCE>
+__device__ __forceinline__ void collide_v(V g[9], const float w[9], float h1, float h5, V dr, V ux, V uy,
+                                          V Jx, V Jy, V jx, V jy, V om, bool force, float Fx, float Fy) {
+    const V nrt = v_mul(v_splat<V>(-1.5f), v_fma(Jx, ux, v_mul(Jy, uy)));  // -rho * 1.5 u.u
+    // Without a body force j = J exactly: one set of momenta stays live.
+    const bool forced = FORCE && force;
+    if (!FORCE) {
+        jx = Jx;
+        jy = Jy;
+    }
+    V geq[9];
+    geq_pair(w[1], h1, dr, ux, Jx, jx, nrt, geq[1], geq[3]);
+    geq_pair(w[2], h1, dr, uy, Jy, jy, nrt, geq[2], geq[4]);
+    geq_pair(w[5], h5, dr, v_add(ux, uy), v_add(Jx, Jy), v_add(jx, jy), nrt, geq[5], geq[7]);
+    geq_pair(w[6], h5, dr, v_sub(uy, ux), v_sub(Jy, Jx), v_sub(jy, jx), nrt, geq[6], geq[8]);
+    geq[0] = v_sub(dr, v_add(v_add(v_add(geq[1], geq[3]), v_add(geq[2], geq[4])),
+                             v_add(v_add(geq[5], geq[7]), v_add(geq[6], geq[8]))));
+    if (!forced) {
+        // A force-free case: one FMA per population. Kernels that may see
+        // forced cases (FORCE) take this branch per case at run time, so a
+        // case gets the same bits alone and in any batch.
+#pragma unroll
+        for (int k = 0; k < 9; k++) g[k] = v_fma(om, v_sub(geq[k], g[k]), g[k]);
+        return;
+    }
+    const V Fxv = v_splat<V>(Fx), Fyv = v_splat<V>(Fy);
+    const V gf = v_fma(v_splat<V>(-0.5f), om, v_splat<V>(1.0f));
+    const V n3uF = v_mul(v_splat<V>(-3.0f), v_fma(ux, Fxv, v_mul(uy, Fyv)));  // -3 u.F
+    g[0] = v_add(g[0], v_fma(om, v_sub(geq[0], g[0]), v_mul(gf, v_mul(v_splat<V>(w[0]), n3uF))));
+    const V cu[4] = {ux, uy, v_add(ux, uy), v_sub(uy, ux)};
+    const float cFs[4] = {Fx, Fy, Fx + Fy, Fy - Fx};
+    const float hs[4] = {h1, h1, h5, h5};
+    const int ka[4] = {1, 2, 5, 6}, kb[4] = {3, 4, 7, 8};
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        const V cF = v_splat<V>(cFs[q]);
+        const V S = v_fma(v_mul(v_splat<V>(9.0f), cu[q]), cF, n3uF);
+        const V E = v_mul(gf, v_mul(v_splat<V>(w[ka[q]]), S));
+        const V O = v_splat<V>(hs[q] * cFs[q]);
+        const int a = ka[q], b = kb[q];
+        g[a] = v_add(g[a], v_fma(om, v_sub(geq[a], g[a]), v_add(E, O)));
+        g[b] = v_add(g[b], v_fma(om, v_sub(geq[b], g[b]), v_sub(E, O)));
+    }
+}
+
+}  // namespace lbm
