@@ -117,6 +117,9 @@ Solver::~Solver() {
     if (h_vtk_) cudaFreeHost(h_vtk_);
     if (pair_exec_) cudaGraphExecDestroy(pair_exec_);
     if (multi_exec_) cudaGraphExecDestroy(multi_exec_);
+    if (multi_fork_) cudaEventDestroy(multi_fork_);
+    if (multi_join_) cudaEventDestroy(multi_join_);
+    if (multi_stream_) cudaStreamDestroy(multi_stream_);
     for (void *p : allocs_) cudaFreeAsync(p, stream_);
     if (stream_) cudaStreamDestroy(stream_);
 }
@@ -592,7 +595,7 @@ bool Solver::upload_force_slot() {
 
 bool Solver::set_block(dim3 b) {
     block_ = b;
-    graph_valid_ = false;
+    graph_valid_ = graph_valid_multi_ = false;
     return true;
 }
 
@@ -735,7 +738,7 @@ bool Solver::enable_force_history(int capacity) {
     hist_cap_ = capacity;
     hist_count_ptr_ = cnt;
     hist_written_ = 0;  // a new ring: its records count from its first step
-    graph_valid_ = false;
+    graph_valid_ = graph_valid_multi_ = false;
     return upload_force_slot();
 }
 
@@ -829,7 +832,7 @@ StepParams Solver::step_params(int src, int dst, bool write_macro, int bparity) 
     std::memset(&p, 0, sizeof p);
     p.Nx = d_.Nx; p.Ny = d_.Ny; p.pitch = pitch_; p.plane = plane_;
     p.px = d_.px; p.py = d_.py;
-    p.src = buf_[src]; p.dst = buf_[dst];
+    p.src = buf_[src]; p.dst = buf_[dst]; p.stale = buf_[dst];
     p.flags = d_flags_; p.link_off = d_link_off_; p.links = d_links_;
     p.seg_clean = d_seg_clean_; p.seg_words = seg_words_;
     p.omega = d_omega_; p.omega0 = omega0_;
@@ -985,7 +988,7 @@ bool Solver::set_impedance(int entry, const double *R, const double *m, const do
         st->imp_cos[f] = std::cos(omegas[f]);
         st->imp_sin[f] = std::sin(omegas[f]);
     }
-    graph_valid_ = false;
+    graph_valid_ = graph_valid_multi_ = false;
     // a wall trace reads this array: its record task follows a new allocation
     return st->d_trace ? upload_records() : true;
 }
@@ -1058,10 +1061,16 @@ bool Solver::launch_step_kernels(int src, int dst, bool collide, bool write_macr
         // SMs around the special nodes' latency-bound blocks from the start
         // (the plain kernel of a flag-free grid steps its own odd column).
         // What follows is an ordinary launch, so it sees both.
-        if (special_launch()) CK(launch::special_shifted(fp, d_special_, nspecial_, d_.store, true, collide, false, s));
+        if (special_launch()) CK(launch::special_shifted(fp, d_special_, nspecial_, nspecial_, d_.store, true, collide, false, s));
         CK(launch::step_shifted(fp, d_.store, has_flags_, collide, block_, s, special_launch()));
     }
-    const bool after_bulk = d_.store == STORE_F64;
+    return launch_edges(src, dst, collide, write_macro, bparity, forces, d_.store == STORE_F64, s);
+}
+
+// The Boundary list's launches of a step and its wall force, behind the kernels
+// that stepped the nodes (after_bulk: as their programmatic follower).
+bool Solver::launch_edges(int src, int dst, bool collide, bool write_macro, int bparity, bool forces,
+                          bool after_bulk, cudaStream_t s) {
     if (groups_.empty()) {
         if (forces) CK(launch::force_reduce(d_force_slot_, 1, after_bulk, s));
         return true;
@@ -1128,7 +1137,7 @@ bool Solver::upload_records() {
         r.count = st.trace_count;
         rec_host_.push_back(r);
     }
-    graph_valid_ = false;
+    graph_valid_ = graph_valid_multi_ = false;
     if (rec_host_.empty()) return true;
     if ((int)rec_host_.size() > rec_cap_) {
         if (!dalloc(&d_rec_, rec_host_.size())) return false;
@@ -1355,8 +1364,14 @@ void Solver::set_autotune(int mode) {
 // 8.73, 4096^2 112.5 -> 80.4.
 int Solver::multi_levels() const {
     const long long n = (long long)d_.Nx * d_.Ny;
-    if (d_.store == STORE_F64 || has_flags_ || d_omega_ || !rec_host_.empty()) return 0;
+    if (d_.store == STORE_F64 || d_omega_ || !rec_host_.empty()) return 0;
     if (d_.Nx < 8 || d_.Ny < 8 || plane_ >= (1LL << 31)) return 0;
+    // With a flag word the nodes near walls and edges go step by step beside the
+    // pass, a chain of launches that bounds small grids. Cavity 512^2 7.22 ->
+    // 6.80 with two levels, 1024^2 11.3 -> 9.98 (10.6 with four), 2048^2 50.4 ->
+    // 36.8 and 25.6 with four, 4096^2 184 -> 85; channel 1024 x 256 6.21 -> 5.23
+    // (7.04); cylinder 2048 x 512 16.5 -> 14.6 (13.5).
+    if (has_flags_) return n < (1LL << 18) ? 0 : n < (1LL << 21) ? 2 : 4;
     if (d_.store == STORE_F16) return n >= (1LL << 20) ? 4 : 0;
     return n >= (1LL << 17) && n < (1LL << 19) ? 2 : 4;
 }
@@ -1369,30 +1384,172 @@ int Solver::multi_warps() const {
     return launch::sm_count() * (n < (1LL << 21) ? 8 : d_.store == STORE_F16 ? 24 : 12);
 }
 
+// A case with a flag word in passes of several steps. Nodes at least `levels`
+// nodes away from every special node step by the pass kernel (multi_geo), which
+// reads the state before the pass and writes the one after it. The nodes near
+// special ones cannot: they go step by step, as a list per step (the special
+// nodes, then every node that the following steps of the list pull from) in
+// buffers 2 and 3, with the Boundary list after each step, on a stream of their
+// own beside the pass kernel. multi_swap moves what lbc's two buffers keep in
+// solid nodes and off-grid slots between the buffers' roles.
+bool Solver::multi_setup() {
+    if (multi_state_) return multi_state_ > 0;
+    multi_state_ = -1;
+    const int Nx = d_.Nx, Ny = d_.Ny, lv = multi_levels();
+    const size_t N = (size_t)Nx * Ny;
+    if (nspecial_ == 0 || (size_t)nspecial_ > N / 8) return false;
+    for (const Stage &st : stages_)  // these read post-collision values of the opposite edge
+        if (st.kind == BC_PERIODIC_X || st.kind == BC_PERIODIC_Y) return false;
+    size_t freeb = 0, total = 0;
+    const size_t need = (size_t)(lv > 2 ? 2 : 1) * 9 * (size_t)plane_ * esize_;
+    if (cudaMemGetInfo(&freeb, &total) != cudaSuccess || freeb / 4 < need) return false;
+    // Distance to the nearest special node (the larger of |dx|, |dy|), up to m,
+    // by runs of special nodes along a row.
+    const int m = 2 * lv - 1;
+    std::vector<uint8_t> dist(N, 255);
+    for (int q = 0; q < nspecial_;) {
+        const int y = special_host_[q].y, i0 = special_host_[q].x & ~kSpecialSolid;
+        int i1 = i0;
+        for (q++; q < nspecial_ && special_host_[q].y == y && (special_host_[q].x & ~kSpecialSolid) == i1 + 1; q++) i1++;
+        for (int dy = -m; dy <= m; dy++) {
+            int j = y + dy;
+            if (!wrap(j, Ny, d_.py)) continue;
+            uint8_t *row = &dist[(size_t)j * Nx];
+            const uint8_t ady = (uint8_t)std::abs(dy);
+            for (int i = i0; i <= i1; i++) row[i] = std::min(row[i], ady);
+            for (int dx = 1; dx <= m; dx++) {
+                const uint8_t d = std::max(ady, (uint8_t)dx);
+                int l = i0 - dx, r = i1 + dx;
+                if (wrap(l, Nx, d_.px)) row[l] = std::min(row[l], d);
+                if (wrap(r, Nx, d_.px)) row[r] = std::min(row[r], d);
+            }
+        }
+    }
+    // Deep pairs, both nodes lv or more away: every pair of the grid, then the
+    // near ones taken out as they join the lists.
+    const int halo = multi_halo(lv), width = 64 - 2 * halo, strips = (Nx + width - 1) / width;
+    std::vector<uint32_t> deep((size_t)strips * Ny);
+    for (int st = 0; st < strips; st++) {
+        uint32_t all = 0;
+        for (int c = 0; c < width && st * width + c + 1 < Nx; c += 2) all |= 1u << ((c + halo) / 2);
+        std::fill(deep.begin() + (size_t)st * Ny, deep.begin() + (size_t)(st + 1) * Ny, all);
+    }
+    std::vector<std::vector<int2>> list(lv, special_host_);
+    for (std::vector<int2> &l : list)
+        while (l.size() % 32) l.push_back(make_int2(-1, -1));
+    for (int j = 0; j < Ny; j++) {
+        const uint8_t *row = &dist[(size_t)j * Nx];
+        for (int i = 0; i < Nx; i += 2) {
+            uint64_t eight;
+            if (i + 8 <= Nx && (std::memcpy(&eight, row + i, 8), eight == ~0ull)) {
+                i += 6;
+                continue;
+            }
+            const bool two = i + 1 < Nx;
+            const bool is_deep = two && row[i] >= lv && row[i + 1] >= lv;
+            if (!is_deep) deep[(size_t)(i / width) * Ny + j] &= ~(1u << ((i % width + halo) / 2));
+            // step q + 1 of the list needs the nodes within 2 lv - (q + 1) of a
+            // special one; the last, every node that is not deep
+            for (int h = 0; h < (two ? 2 : 1); h++) {
+                const int d = row[i + h];
+                if (d == 0) continue;
+                for (int q = 0; q < lv - 1; q++)
+                    if (d < 2 * lv - q) list[q].push_back(make_int2(i + h, j));
+                if (!is_deep) list[lv - 1].push_back(make_int2(i + h, j));
+            }
+        }
+    }
+    if (!dalloc(&d_deep_, deep.size())) return false;
+    CK(cudaMemcpyAsync(d_deep_, deep.data(), deep.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, stream_));
+    for (int q = 0; q < lv; q++) {
+        int2 *l = nullptr;
+        if (!dalloc(&l, list[q].size())) return false;
+        CK(cudaMemcpyAsync(l, list[q].data(), list[q].size() * sizeof(int2), cudaMemcpyHostToDevice, stream_));
+        d_multi_list_[q] = l;
+        multi_count_[q] = (int)list[q].size();
+    }
+    for (int b = 2; b < (lv > 2 ? 4 : 3); b++) {
+        char *q = nullptr;
+        if (!dalloc(&q, 9 * (size_t)plane_ * esize_)) return false;
+        buf_[b] = q;
+    }
+    int lo = 0, hi = 0;
+    cudaDeviceGetStreamPriorityRange(&lo, &hi);
+    CK(cudaStreamCreateWithPriority(&multi_stream_, cudaStreamNonBlocking, lo));
+    CK(cudaEventCreateWithFlags(&multi_fork_, cudaEventDisableTiming));
+    CK(cudaEventCreateWithFlags(&multi_join_, cudaEventDisableTiming));
+    CK(cudaStreamSynchronize(stream_));
+    multi_state_ = 1;
+    return true;
+}
+
+// One pass of `lv` steps, cur -> other.
+bool Solver::launch_multi(int cur, int other, int lv) {
+    const FastStepParams whole = fast_params(step_params(cur, other, false, 0));
+    if (!has_flags_) {
+        CK(launch::multi_plain(whole, d_.store, lv, multi_warps(), stream_));
+        return true;
+    }
+    CK(cudaEventRecord(multi_fork_, stream_));
+    CK(cudaStreamWaitEvent(multi_stream_, multi_fork_, 0));
+    CK(launch::multi_geo(whole, d_.store, lv, d_deep_, multi_warps(), multi_stream_));
+    CK(cudaEventRecord(multi_join_, multi_stream_));
+    const bool forces = has_mem_ && hist_cap_ > 0;
+    int at[5] = {cur, 2, 3, 2, other};  // the buffer of each step's state
+    at[lv] = other;
+    for (int q = 0; q < lv; q++) {
+        const int par = parity_ ^ (q & 1);
+        StepParams p = step_params(at[q], at[q + 1], false, par);
+        if (q & 1) p.stale = buf_[at[q - 1]];  // even states: two steps before
+        if (!forces) p.mem_partials = nullptr;
+        CK(launch::special_shifted(fast_params(p), d_multi_list_[q], multi_count_[q], (nspecial_ + 31) / 32 * 32, d_.store,
+                                   true, true, false, stream_));
+        if (!launch_edges(at[q], at[q + 1], true, false, par, forces, true, stream_)) return false;
+    }
+    CK(cudaStreamWaitEvent(stream_, multi_join_, 0));
+    return true;
+}
+
 // Two passes (cur -> other -> cur) captured once and replayed.
 bool Solver::capture_multi() {
-    if (multi_exec_ && multi_cur_ == cur_) return true;
+    if (multi_exec_ && multi_cur_ == cur_ && multi_parity_ == parity_ && graph_valid_multi_) return true;
     if (multi_exec_) {
         cudaGraphExecDestroy(multi_exec_);
         multi_exec_ = nullptr;
     }
     cudaGraph_t g = nullptr;
     CK(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
-    cudaError_t e = cudaSuccess;
-    for (int b = 0; b < 2 && e == cudaSuccess; b++)
-        e = launch::multi_plain(fast_params(step_params(cur_ ^ b, cur_ ^ b ^ 1, false, 0)), d_.store, multi_levels(),
-                                multi_warps(), stream_);
-    const cudaError_t e2 = cudaStreamEndCapture(stream_, &g);
-    if (e != cudaSuccess || e2 != cudaSuccess) {
+    const int lv = multi_levels();
+    const bool okk = launch_multi(cur_, 1 - cur_, lv) && launch_multi(1 - cur_, cur_, lv);
+    cudaError_t e = cudaStreamEndCapture(stream_, &g);
+    if (!okk) {
         if (g) cudaGraphDestroy(g);
-        CK(e);
-        CK(e2);
+        return false;
     }
+    CK(e);
     e = cudaGraphInstantiate(&multi_exec_, g, 0);
     cudaGraphDestroy(g);
     CK(e);
     multi_cur_ = cur_;
+    multi_parity_ = parity_;
+    graph_valid_multi_ = true;
     return true;
+}
+
+// As many of `avail` steps as whole double passes take; -1 on an error.
+int Solver::run_multi(int avail) {
+    const int lv = multi_levels();
+    if (lv == 0 || avail < 2 * lv || (has_flags_ && (avail < 8 * lv || !multi_setup()))) return 0;
+    auto swap = [&](bool enter) {
+        return !has_flags_ || check_cuda(launch::multi_swap(d_special_, nspecial_, d_flags_, pitch_, plane_, d_.store,
+                                                            buf_[cur_], buf_[1 - cur_], buf_[2], lv > 2 ? buf_[3] : nullptr,
+                                                            enter, stream_), "multi_swap");
+    };
+    if (!capture_multi() || !swap(true)) return -1;
+    int used = 0;
+    for (; avail - used >= 2 * lv; used += 2 * lv)
+        if (!check_cuda(cudaGraphLaunch(multi_exec_, stream_), "cudaGraphLaunch")) return -1;
+    return swap(false) ? used : -1;
 }
 
 // One fused step cur -> other, as inside run().
@@ -1454,11 +1611,9 @@ bool Solver::run(int nsteps) {
         if (used < 0) return false;
         remaining -= used;
     }
-    const int lv = multi_levels();
-    if (lv > 0 && remaining >= 2 * lv) {
-        if (!capture_multi()) return false;
-        for (; remaining >= 2 * lv; remaining -= 2 * lv) CK(cudaGraphLaunch(multi_exec_, stream_));
-    }
+    const int used = run_multi(remaining);
+    if (used < 0) return false;
+    remaining -= used;
     if (remaining >= 2) {
         if (!capture_pair()) return false;
         while (remaining >= 2) {

@@ -235,6 +235,8 @@ class Solver {
     bool alloc();
     bool launch_step(int src, int dst, bool collide, bool write_macro, int bparity,
                      cudaStream_t s = nullptr);
+    bool launch_edges(int src, int dst, bool collide, bool write_macro, int bparity, bool forces, bool after_bulk,
+                      cudaStream_t s);
     bool launch_step_kernels(int src, int dst, bool collide, bool write_macro, int bparity, cudaStream_t s);
     bool upload_records();
     std::vector<RecordTask> rec_host_;
@@ -248,7 +250,10 @@ class Solver {
     bool capture_pair();
     int multi_levels() const;
     int multi_warps() const;
+    bool multi_setup();
+    bool launch_multi(int cur, int other, int lv);
     bool capture_multi();
+    int run_multi(int avail);
     bool trial_step();
     int tune_online(int avail);
     int tune_mode_ = 0;
@@ -262,7 +267,7 @@ class Solver {
     int pitch_ = 0;
     long long plane_ = 0;
     size_t esize_ = 8;
-    void *buf_[2] = {nullptr, nullptr};
+    void *buf_[4] = {nullptr, nullptr, nullptr, nullptr};  // 2, 3: passes of several steps (multi_setup)
     int cur_ = 0;
     int parity_ = 0;
     bool has_flags_ = false, has_links_ = false, has_mem_ = false;
@@ -301,7 +306,14 @@ class Solver {
     int pair_cur_ = -1, pair_parity_ = -1;
     bool graph_valid_ = false;
     cudaGraphExec_t multi_exec_ = nullptr;
-    int multi_cur_ = -1;
+    int multi_cur_ = -1, multi_parity_ = -1;
+    bool graph_valid_multi_ = false;
+    int multi_state_ = 0;                 // 0: not tried, 1: set up, -1: not for this case
+    uint32_t *d_deep_ = nullptr;
+    int2 *d_multi_list_[4] = {nullptr, nullptr, nullptr, nullptr};
+    int multi_count_[4] = {0, 0, 0, 0};
+    cudaStream_t multi_stream_ = nullptr;
+    cudaEvent_t multi_fork_ = nullptr, multi_join_ = nullptr;
     size_t dev_bytes_ = 0;
     long long steps_done_ = 0;
     std::vector<void *> allocs_;

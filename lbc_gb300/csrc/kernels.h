@@ -144,9 +144,18 @@ cudaError_t step_exact(const StepParams &p, bool flags, bool collide, dim3 block
 // the final step of a run, which leaves pre-collision populations).
 // after_bulk (here, stage_batch and force_reduce): the previous launch in s is
 // a bulk step kernel; the launch overlaps its tail (pdl.cuh).
-// `levels` (2..4) steps of a fully periodic case without a flag word, with one
+// `levels` (2 or 4) steps of a fully periodic case without a flag word, with one
 // omega, in one pass; warps: how many to split the grid into.
 cudaError_t multi_plain(const FastStepParams &p, int store, int levels, int warps, cudaStream_t s);
+// The same for the nodes of a case with a flag word that are `levels` or more
+// nodes away from any special node: deep[strip * Ny + row], a bit per lane's
+// pair (strips of 64 - 2 multi_halo(levels) columns).
+cudaError_t multi_geo(const FastStepParams &p, int store, int levels, const uint32_t *deep, int warps, cudaStream_t s);
+// Before a run of such passes and after it: the special nodes' populations of
+// odd steps move from `other` to `odd` and back; solid nodes of `other` (and of
+// `even2`, when there is one) take cur's, as the buffers change roles.
+cudaError_t multi_swap(const int2 *nodes, int n, const uint16_t *flags, int pitch, long long plane, int store,
+                       const void *cur, void *other, void *odd, void *even2, bool enter, cudaStream_t s);
 cudaError_t stage_group(const StageGroup &g, int store, bool collide, bool after_bulk, cudaStream_t s);
 cudaError_t collide_exact(const CollideParams &p, cudaStream_t s);
 cudaError_t collide_aos_exact(const CollideAosParams &p, cudaStream_t s);
@@ -189,8 +198,9 @@ cudaError_t step_shifted(const FastStepParams &p, int store, bool flags, bool co
 // The special nodes of a case (nodes[0 .. n)) on the per-node path; flags: the
 // case has a flag word. after_bulk: the programmatic follower of the kernel
 // before it (a case alone launches it first, without the attribute, and the
-// clean pairs as its follower: step_shifted's after).
-cudaError_t special_shifted(const FastStepParams &p, const int2 *nodes, int n, int store, bool flags, bool collide,
+// clean pairs as its follower: step_shifted's after). The first nforce entries
+// (a multiple of 32, or all) sum their wall-link force by chunks.
+cudaError_t special_shifted(const FastStepParams &p, const int2 *nodes, int n, int nforce, int store, bool flags, bool collide,
                             bool after_bulk, cudaStream_t s);
 // The special nodes of a batch: nodes[q] = (case, i, j, chunk), n a multiple
 // of 32 (each case's list padded to 32 entries, i = -1); links: some case has

@@ -94,8 +94,11 @@ template <typename T> struct Rows {
     P up2[3];     // 2, 5, 6 of the row before that
 };
 
-template <typename T, int LV, bool FORCE, bool EDGE>
-__device__ __forceinline__ void walk_strip(const FastStepParams &fp, int cb, int keep0, int keep1, int y0, int y1) {
+// deep: null, or a word per row whose bit l says that lane l's pair is stored
+// (a case with a flag word; the others are garbage near special nodes).
+template <typename T, int LV, bool FORCE, bool EDGE, bool DEEP>
+__device__ __forceinline__ void walk_strip(const FastStepParams &fp, const uint32_t *deep, int cb, int keep0, int keep1,
+                                           int y0, int y1) {
     using PO = PairOf<T>;
     using P = typename PO::P;
     const StepParams &p = fp.s;
@@ -105,13 +108,19 @@ __device__ __forceinline__ void walk_strip(const FastStepParams &fp, int cb, int
     const int lane = (int)(threadIdx.x & 31);
     const int v0 = cb + 2 * lane;  // this lane's columns v0, v0 + 1, before wrapping
     int c0 = v0, c1 = v0 + 1;
-    if (EDGE) {
+    // Wrapped on periodic axes; clamped otherwise, where the values loaded
+    // reach no node that is stored.
+    if (EDGE && p.px) {
         c0 = (c0 + p.Nx) % p.Nx;
         c1 = (c1 + p.Nx) % p.Nx;
+    } else if (EDGE) {
+        c0 = min(max(c0, 0), p.Nx - 1);
+        c1 = min(max(c1, 0), p.Nx - 1);
     }
     const bool st0 = v0 >= keep0 && v0 < keep1, st1 = v0 + 1 >= keep0 && v0 + 1 < keep1;
 
     auto row_of = [&](int r) {
+        if (DEEP && !p.py) return (uint32_t)min(max(r, 0), p.Ny - 1) * (uint32_t)p.pitch;
         r = r < 0 ? r + p.Ny : r;
         return (uint32_t)(r >= p.Ny ? r - p.Ny : r) * (uint32_t)p.pitch;
     };
@@ -162,13 +171,16 @@ __device__ __forceinline__ void walk_strip(const FastStepParams &fp, int cb, int
         const int row = r - (LV - 1);
         if (row >= y0) {
             const size_t o = (size_t)row * (size_t)p.pitch;
+            const bool pair = DEEP ? (__ldg(deep + row) >> lane) & 1u : st0;
 #pragma unroll
             for (int k = 0; k < 9; k++) {
                 T *d = D + k * pl + o;
-                if (EDGE) {
+                if (DEEP) {
+                    if (pair) PO::store(d + v0, f[k]);
+                } else if (EDGE) {
                     if (st0) PO::store1(d + v0, f[k], 0);
                     if (st1) PO::store1(d + v0 + 1, f[k], 1);
-                } else if (st0) {
+                } else if (pair) {
                     PO::store(d + v0, f[k]);
                 }
             }
@@ -185,11 +197,89 @@ __global__ void __launch_bounds__(kMultiThreads) k_multi_plain(const FastStepPar
     if (y0 >= y1) return;
     const int halo = multi_halo(LV), width = 64 - 2 * halo;
     const int keep0 = strip * width, keep1 = min(keep0 + width, fp.s.Nx), cb = keep0 - halo;
-    if (cb >= 0 && cb + 64 <= fp.s.Nx) walk_strip<T, LV, FORCE, false>(fp, cb, keep0, keep1, y0, y1);
-    else walk_strip<T, LV, FORCE, true>(fp, cb, keep0, keep1, y0, y1);
+    if (cb >= 0 && cb + 64 <= fp.s.Nx) walk_strip<T, LV, FORCE, false, false>(fp, nullptr, cb, keep0, keep1, y0, y1);
+    else walk_strip<T, LV, FORCE, true, false>(fp, nullptr, cb, keep0, keep1, y0, y1);
+}
+
+// A case with a flag word and one omega: the nodes at least LV nodes away from
+// any special node (the others are the list kernels', which run beside it:
+// its blocks leave registers free on every SM). Cavity 4096^2: 184 us per step
+// one at a time, 85 with four levels; 2048^2 50.4 -> 25.6.
+template <typename T, int LV, bool FORCE>
+__global__ void __launch_bounds__(kMultiThreads) k_multi_geo(const FastStepParams fp, const uint32_t *deep, int strips,
+                                                             int height) {
+    const int w = (int)(blockIdx.x * (kMultiThreads / 32) + threadIdx.x / 32);
+    const int chunk = w / strips, strip = w - chunk * strips;
+    const int y0 = chunk * height, y1 = min(y0 + height, fp.s.Ny);
+    if (y0 >= y1) return;
+    const int halo = multi_halo(LV), width = 64 - 2 * halo;
+    const int keep0 = strip * width, keep1 = min(keep0 + width, fp.s.Nx), cb = keep0 - halo;
+    deep += (size_t)strip * (size_t)fp.s.Ny;
+    if (cb >= 0 && cb + 64 <= fp.s.Nx) walk_strip<T, LV, FORCE, false, true>(fp, deep, cb, keep0, keep1, y0, y1);
+    else walk_strip<T, LV, FORCE, true, true>(fp, deep, cb, keep0, keep1, y0, y1);
+}
+
+// One thread per special node (launch::multi_swap).
+template <typename T>
+__global__ void k_multi_swap(const int2 *__restrict__ nodes, int n, const uint16_t *__restrict__ flags, int pitch,
+                             long long plane, const T *cur, T *other, T *odd, T *even2, int enter) {
+    const int q = (int)(blockIdx.x * blockDim.x + threadIdx.x);
+    if (q >= n) return;
+    const long long o = (long long)nodes[q].y * pitch + (nodes[q].x & ~kSpecialSolid);
+    const bool solid = (flags[o] & NF_SOLID) != 0;
+#pragma unroll
+    for (int k = 0; k < 9; k++) {
+        const long long at = k * plane + o;
+        if (enter) {
+            odd[at] = other[at];
+            if (solid) {
+                other[at] = cur[at];
+                if (even2) even2[at] = cur[at];
+            }
+        } else {
+            other[at] = odd[at];
+        }
+    }
 }
 
 namespace launch {
+
+template <typename T, int LV>
+static cudaError_t multi_geo_tl(const FastStepParams &p, const uint32_t *deep, int warps_wanted, cudaStream_t s) {
+    const int width = 64 - 2 * multi_halo(LV);
+    const int strips = (p.s.Nx + width - 1) / width;
+    const int chunks = std::max(1, std::min(p.s.Ny / 4, warps_wanted / strips));
+    const int height = (p.s.Ny + chunks - 1) / chunks;
+    const long long warps = (long long)strips * ((p.s.Ny + height - 1) / height);
+    const unsigned blocks = (unsigned)((warps + kMultiThreads / 32 - 1) / (kMultiThreads / 32));
+    if (p.s.has_force) k_multi_geo<T, LV, true><<<blocks, kMultiThreads, 0, s>>>(p, deep, strips, height);
+    else k_multi_geo<T, LV, false><<<blocks, kMultiThreads, 0, s>>>(p, deep, strips, height);
+    return cudaGetLastError();
+}
+
+cudaError_t multi_geo(const FastStepParams &p, int store, int levels, const uint32_t *deep, int warps, cudaStream_t s) {
+    if (store == STORE_F32) {
+        if (levels == 2) return multi_geo_tl<float, 2>(p, deep, warps, s);
+        if (levels == 4) return multi_geo_tl<float, 4>(p, deep, warps, s);
+    } else {
+        if (levels == 2) return multi_geo_tl<__half, 2>(p, deep, warps, s);
+        if (levels == 4) return multi_geo_tl<__half, 4>(p, deep, warps, s);
+    }
+    return cudaErrorInvalidValue;
+}
+
+cudaError_t multi_swap(const int2 *nodes, int n, const uint16_t *flags, int pitch, long long plane, int store,
+                       const void *cur, void *other, void *odd, void *even2, bool enter, cudaStream_t s) {
+    if (n == 0) return cudaSuccess;
+    const unsigned g = (unsigned)((n + 127) / 128);
+    if (store == STORE_F32)
+        k_multi_swap<float><<<g, 128, 0, s>>>(nodes, n, flags, pitch, plane, (const float *)cur, (float *)other,
+                                              (float *)odd, (float *)even2, enter ? 1 : 0);
+    else
+        k_multi_swap<__half><<<g, 128, 0, s>>>(nodes, n, flags, pitch, plane, (const __half *)cur, (__half *)other,
+                                               (__half *)odd, (__half *)even2, enter ? 1 : 0);
+    return cudaGetLastError();
+}
 
 template <typename T, int LV>
 static cudaError_t multi_plain_tl(const FastStepParams &p, int warps_wanted, cudaStream_t s) {
@@ -208,13 +298,11 @@ cudaError_t multi_plain(const FastStepParams &p, int store, int levels, int warp
     if (store == STORE_F32) {
         switch (levels) {
         case 2: return multi_plain_tl<float, 2>(p, warps, s);
-        case 3: return multi_plain_tl<float, 3>(p, warps, s);
         case 4: return multi_plain_tl<float, 4>(p, warps, s);
         }
     } else {
         switch (levels) {
         case 2: return multi_plain_tl<__half, 2>(p, warps, s);
-        case 3: return multi_plain_tl<__half, 3>(p, warps, s);
         case 4: return multi_plain_tl<__half, 4>(p, warps, s);
         }
     }

@@ -34,9 +34,9 @@ __device__ __noinline__ void solid_node_outputs(const StepParams &p, int slot, l
     if (fl & NF_BAND) {
         // A BC may read a solid neighbour: lbc sees the untouched buffer
         // content and NaN moments there.
-        const T *Dst = (const T *)p.dst;
+        const T *Old = (const T *)p.stale;
 #pragma unroll
-        for (int k = 0; k < 9; k++) p.bandg[(size_t)k * p.nslots + slot] = SV<T>::ld_plain(Dst + k * p.plane + node);
+        for (int k = 0; k < 9; k++) p.bandg[(size_t)k * p.nslots + slot] = SV<T>::ld_plain(Old + k * p.plane + node);
         p.bandm_next[slot] = NAN;
         p.bandm_next[(size_t)p.nslots + slot] = NAN;
         p.bandm_next[2 * (size_t)p.nslots + slot] = NAN;
@@ -92,6 +92,7 @@ __device__ __forceinline__ void step_node_shifted(const FastStepParams &fp, int 
     const size_t dn = (size_t)j * (size_t)p.Nx + (size_t)i;
     const T *S = (const T *)p.src;
     T *Dst = (T *)p.dst;
+    const T *Old = (const T *)p.stale;
     const I pl = (I)p.plane;
     // The loads come in three waves of independent loads, not one chain: (1)
     // the flag word, the nine pulled populations, the node's eight own
@@ -132,7 +133,7 @@ __device__ __forceinline__ void step_node_shifted(const FastStepParams &fp, int 
             for (int k = 1; k < 9; k++) {
                 const int si = i - cxk(k), sj = j - cyk(k);
                 off[k] = (!p.px && (si < 0 || si >= p.Nx)) || (!p.py && (sj < 0 || sj >= p.Ny));
-                if (off[k]) g[k] = SV<T>::ld_plain(Dst + (I)k * pl + node);
+                if (off[k]) g[k] = SV<T>::ld_plain(Old + (I)k * pl + node);
             }
         }
     }
@@ -161,7 +162,7 @@ __device__ __forceinline__ void step_node_shifted(const FastStepParams &fp, int 
             behind[k] = 0.f;
             if (!(fl & (1u << k))) continue;
             if (off[k]) {
-                if (LINKS) g[k] = SV<T>::ld_plain(Dst + (I)k * pl + node);
+                if (LINKS) g[k] = SV<T>::ld_plain(Old + (I)k * pl + node);
             } else if (has_links) {
                 if (L[k].mode == LINK_IBB_LO) behind[k] = SV<T>::ld(S + (I)oppk(k) * pl + (I)L[k].behind);
                 else if (L[k].mode == LINK_IBB_HI) behind[k] = SV<T>::ld(S + (I)k * pl + (I)L[k].behind);
@@ -318,7 +319,8 @@ __global__ void __launch_bounds__(256, 5) k_step_shifted_geo(const FastStepParam
     if (i0 < fp.s.Nx && j < fp.s.Ny) step_pair_clean<T, I, true, COLLIDE, FORCE>(fp, i0, j);
 }
 
-// The special nodes of a case, one per thread, on the per-node path (same
+// The special nodes of a case (and, in passes of several steps, the nodes near
+// them), one per thread, on the per-node path (same
 // arithmetic as the pair path, so a node's bits do not depend on which path
 // steps it). Wall-link force terms are summed per 32-entry chunk of the list.
 // It reads and writes nothing the clean-pair kernel touches: a case alone
@@ -329,17 +331,19 @@ __global__ void __launch_bounds__(256, 5) k_step_shifted_geo(const FastStepParam
 // no-op.)
 template <typename T, typename I, bool FLAGS, bool COLLIDE, bool FORCE, bool LINKS>
 __global__ void __launch_bounds__(128) k_step_special_shifted(const FastStepParams fp,
-                                                              const int2 *__restrict__ nodes, int n) {
+                                                              const int2 *__restrict__ nodes, int n, int nforce) {
     pdl_launch_dependents();
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
     float mx = 0.f, my = 0.f;
     bool link = false;
     if (q < n) {
         const int2 ij = nodes[q];
-        if (ij.x & kSpecialSolid) solid_nan(fp.s, ij.x & ~kSpecialSolid, ij.y);
+        if (ij.x < 0) {  // padding
+        } else if (ij.x & kSpecialSolid) solid_nan(fp.s, ij.x & ~kSpecialSolid, ij.y);
         else step_node_shifted<T, I, FLAGS, COLLIDE, FORCE, LINKS>(fp, ij.x, ij.y, mx, my, link);
     }
-    if (fp.s.mem_partials)
+    // (the first nforce entries are the special nodes, whose chunks have slots)
+    if (fp.s.mem_partials && (q & ~31) < nforce)
         chunk_reduce2_store((double)mx, (double)my, link, q >> 5, fp.s.chunk_slot, fp.s.mem_partials);
     pdl_wait();
 }
@@ -645,46 +649,46 @@ cudaError_t step_shifted(const FastStepParams &p, int store, bool flags, bool co
 }
 
 template <typename T, typename I, bool FORCE, bool LINKS>
-static cudaError_t special_shifted_tifl(const FastStepParams &p, const int2 *nodes, int n, bool flags, bool collide,
+static cudaError_t special_shifted_tifl(const FastStepParams &p, const int2 *nodes, int n, int nforce, bool flags, bool collide,
                                         bool after_bulk, cudaStream_t s) {
     const dim3 g((n + 127) / 128), b(128);
     if (flags) {
         if (collide)
             return launch_follower(after_bulk, k_step_special_shifted<T, I, true, true, FORCE, LINKS>, g, b, s, p,
-                                   nodes, n);
+                                   nodes, n, nforce);
         return launch_follower(after_bulk, k_step_special_shifted<T, I, true, false, FORCE, LINKS>, g, b, s, p, nodes,
-                               n);
+                               n, nforce);
     }
     if (collide)
         return launch_follower(after_bulk, k_step_special_shifted<T, I, false, true, FORCE, LINKS>, g, b, s, p, nodes,
-                               n);
-    return launch_follower(after_bulk, k_step_special_shifted<T, I, false, false, FORCE, LINKS>, g, b, s, p, nodes, n);
+                               n, nforce);
+    return launch_follower(after_bulk, k_step_special_shifted<T, I, false, false, FORCE, LINKS>, g, b, s, p, nodes, n, nforce);
 }
 
 template <typename T, typename I, bool FORCE>
-static cudaError_t special_shifted_tif(const FastStepParams &p, const int2 *nodes, int n, bool flags, bool collide,
+static cudaError_t special_shifted_tif(const FastStepParams &p, const int2 *nodes, int n, int nforce, bool flags, bool collide,
                                        bool after_bulk, cudaStream_t s) {
-    if (p.s.links) return special_shifted_tifl<T, I, FORCE, true>(p, nodes, n, flags, collide, after_bulk, s);
-    return special_shifted_tifl<T, I, FORCE, false>(p, nodes, n, flags, collide, after_bulk, s);
+    if (p.s.links) return special_shifted_tifl<T, I, FORCE, true>(p, nodes, n, nforce, flags, collide, after_bulk, s);
+    return special_shifted_tifl<T, I, FORCE, false>(p, nodes, n, nforce, flags, collide, after_bulk, s);
 }
 
 template <typename T>
-static cudaError_t special_shifted_t(const FastStepParams &p, const int2 *nodes, int n, bool flags, bool collide,
+static cudaError_t special_shifted_t(const FastStepParams &p, const int2 *nodes, int n, int nforce, bool flags, bool collide,
                                      bool after_bulk, cudaStream_t s) {
     const bool wide = 9LL * p.s.plane >= (1LL << 31);
     if (p.s.has_force) {
-        if (wide) return special_shifted_tif<T, long long, true>(p, nodes, n, flags, collide, after_bulk, s);
-        return special_shifted_tif<T, int, true>(p, nodes, n, flags, collide, after_bulk, s);
+        if (wide) return special_shifted_tif<T, long long, true>(p, nodes, n, nforce, flags, collide, after_bulk, s);
+        return special_shifted_tif<T, int, true>(p, nodes, n, nforce, flags, collide, after_bulk, s);
     }
-    if (wide) return special_shifted_tif<T, long long, false>(p, nodes, n, flags, collide, after_bulk, s);
-    return special_shifted_tif<T, int, false>(p, nodes, n, flags, collide, after_bulk, s);
+    if (wide) return special_shifted_tif<T, long long, false>(p, nodes, n, nforce, flags, collide, after_bulk, s);
+    return special_shifted_tif<T, int, false>(p, nodes, n, nforce, flags, collide, after_bulk, s);
 }
 
-cudaError_t special_shifted(const FastStepParams &p, const int2 *nodes, int n, int store, bool flags, bool collide,
+cudaError_t special_shifted(const FastStepParams &p, const int2 *nodes, int n, int nforce, int store, bool flags, bool collide,
                             bool after_bulk, cudaStream_t s) {
     if (n == 0) return cudaSuccess;
-    if (store == STORE_F32) return special_shifted_t<float>(p, nodes, n, flags, collide, after_bulk, s);
-    return special_shifted_t<__half>(p, nodes, n, flags, collide, after_bulk, s);
+    if (store == STORE_F32) return special_shifted_t<float>(p, nodes, n, nforce, flags, collide, after_bulk, s);
+    return special_shifted_t<__half>(p, nodes, n, nforce, flags, collide, after_bulk, s);
 }
 
 template <typename T, bool FORCE, bool LINKS>

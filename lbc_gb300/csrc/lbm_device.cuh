@@ -548,7 +548,9 @@ struct StepParams {
     int px, py;
     long long plane;          // pitch * Ny
     const void *src;          // post-collision populations of step n (planes)
-    void *dst;                // output populations (also holds the stale slots)
+    void *dst;                // output populations
+    const void *stale;        // where a slot that is not streamed into keeps its content from (the populations
+                              // of two steps before: dst's own, except in passes of several steps)
     const uint16_t *flags;    // [Ny * pitch] or null (fully periodic, no solids, no BCs)
     const uint32_t *seg_clean; // bit per 64-node row segment whose 32 pairs are all clean; words per row: seg_words
     int seg_words;

@@ -50,3 +50,65 @@ def test_probes_see_every_step():
     assert h.shape == (40, 2, 3) and len(np.unique(h[:, 0, 1])) > 30
     for fld in FIELDS:
         assert np.array_equal(getattr(a.get_state(), fld), getattr(b.get_state(), fld)), fld
+
+
+def _walls(name):
+    from lbc_gb300 import impedance as imp
+    if name == "wake":
+        return cases.cylinder_wake(1029, 257, D=20.0, xc=270.0, yc=127.0, u_max=0.05, Re=60.0, seed=3), None
+    if name == "wake4":
+        return cases.cylinder_wake(2050, 1026, D=64.0, xc=520.0, yc=500.0, u_max=0.05, Re=60.0, seed=3), None
+    if name == "cavity":
+        return cases.cavity_moving_wall(513, 0.1, 300.0), None
+    if name == "cavity4":
+        return cases.cavity_moving_wall(1450, 0.1, 300.0), None
+    if name == "box":
+        return cases.all_regularized_box(600, 450), None
+    if name == "golden":
+        return cases.cylinder_golden(17)[:2], None
+    if name == "blocks":  # obstacles across both periodic edges, body force
+        case, st = cases.taylor_green(641, 450)
+        for i, j in ((0, 0), (300, 449), (640, 200), (100, 100), (101, 109)):
+            case.solid_mask[j:j + 6, i:i + 8] = 1
+        case.Fx, case.Fy = 1e-6, -2e-6
+        return (case, st), None
+    p = imp.LinerParams(2100, 130, 0.2, 1.0 * imp.CS, 5e-3, 0.05)
+    return imp.liner_duct(p), p
+
+
+@pytest.mark.parametrize("storage", ["f32", "f16"])
+@pytest.mark.parametrize("name", ["wake", "wake4", "cavity", "cavity4", "box", "golden", "blocks", "duct"])
+def test_walls_and_edges_match_single_steps(storage, name):
+    """Cases with a flag word: cut links, moving walls, Zou-He, convective,
+    regularized and impedance edges, slots off open edges, odd sizes, with and
+    without a force history; runs that enter and leave the passes twice."""
+    from lbc_gb300 import GpuSolver, STORAGE, impedance as imp
+    (case, st), duct = _walls(name)
+    if duct is None:
+        st = cases.random_state(case, 7)
+    for hist in (False, True):
+        pair = []
+        for _ in range(2):
+            s = GpuSolver(case, STORAGE[storage])
+            if duct is not None:
+                s.set_impedance_wall(imp.LINER_ENTRY, *imp.liner_arrays(duct), imp.TRACKED_OMEGAS, 1.0, imp.MEAN_RATE, 500)
+            if hist and case.solid_mask.any():
+                s.enable_force_history(100)
+            s.set_state(st)
+            pair.append(s)
+        a, b = pair
+        for n in (41, 2, 44):
+            a.run(n)
+        for _ in range(87):
+            b.run(1)
+        x, y = a.get_state(), b.get_state()
+        for fld in FIELDS:
+            assert np.array_equal(getattr(x, fld), getattr(y, fld), equal_nan=True), (hist, fld)
+        assert a.forces() == b.forces()
+        if hist and case.solid_mask.any():
+            assert np.array_equal(a.force_history(100), b.force_history(100))
+        if duct is not None:
+            for p, q in zip(a.impedance_readback(imp.LINER_ENTRY), b.impedance_readback(imp.LINER_ENTRY)):
+                assert np.array_equal(p, q)
+        a.close()
+        b.close()
