@@ -531,6 +531,9 @@ bool Solver::group_stages(const Solid &solid, const std::vector<int> &colbase, c
         gw.insert(w.begin(), w.end());
         gr.insert(r.begin(), r.end());
     }
+    // (periodic entries read post-collision values of the opposite edge)
+    one_group_ = groups_.size() <= 1;
+    for (const Stage &st : stages_) one_group_ = one_group_ && st.kind != BC_PERIODIC_X && st.kind != BC_PERIODIC_Y;
     return true;
 }
 
@@ -1053,16 +1056,33 @@ bool Solver::launch_step_kernels(int src, int dst, bool collide, bool write_macr
     StepParams p = step_params(src, dst, write_macro, bparity);
     if (!forces) p.mem_partials = nullptr;
     if (d_.store == STORE_F64) {
-        CK(launch::step_exact(p, has_flags_, collide, block_, s, arith_));
+        // A Boundary list of one group goes first and the bulk kernel beside it.
+        const bool edges = collide && !write_macro && one_group_ && !groups_.empty();
+        if (edges) CK(launch::edges_exact(p, stage_group(0, src, dst, write_macro, bparity, false), arith_, s));
+        CK(launch::step_exact(p, has_flags_, collide, block_, s, arith_, edges));
+        if (edges) {
+            if (forces) CK(launch::force_reduce(d_force_slot_, 1, true, s));
+            return true;
+        }
     } else {
         const FastStepParams fp = fast_params(p);
         // The special nodes first, as an ordinary launch, then the clean pairs
         // as its programmatic follower: the grid of clean-pair blocks fills the
         // SMs around the special nodes' latency-bound blocks from the start
         // (the plain kernel of a flag-free grid steps its own odd column).
-        // What follows is an ordinary launch, so it sees both.
-        if (special_launch()) CK(launch::special_shifted(fp, d_special_, nspecial_, nspecial_, d_.store, true, collide, false, s));
+        // What follows is an ordinary launch, so it sees both. A Boundary list
+        // of one group steps with the special nodes (near_shifted).
+        const bool near = collide && !write_macro && special_launch() && one_group_ && !groups_.empty();
+        if (near)
+            CK(launch::near_shifted(fp, d_special_, nspecial_, nspecial_, d_.store,
+                                    stage_group(0, src, dst, write_macro, bparity, false), false, s));
+        else if (special_launch())
+            CK(launch::special_shifted(fp, d_special_, nspecial_, nspecial_, d_.store, true, collide, false, s));
         CK(launch::step_shifted(fp, d_.store, has_flags_, collide, block_, s, special_launch()));
+        if (near) {
+            if (forces) CK(launch::force_reduce(d_force_slot_, 1, false, s));
+            return true;
+        }
     }
     return launch_edges(src, dst, collide, write_macro, bparity, forces, d_.store == STORE_F64, s);
 }
@@ -1077,23 +1097,28 @@ bool Solver::launch_edges(int src, int dst, bool collide, bool write_macro, int 
     }
     // The force (from the bulk kernel's partials) rides in the first stage
     // launch; fused stages finish their nodes (group_stages).
-    const FinishParams f = finish_params(dst, write_macro, bparity);
-    for (size_t gi = 0; gi < groups_.size(); gi++) {
-        const std::vector<int> &g = groups_[gi];
-        StageGroup sg;
-        std::memset(&sg, 0, sizeof sg);
-        sg.n = (int)g.size();
-        for (int q = 0; q < sg.n; q++) {
-            sg.p[q] = stage_params(stages_[g[q]], src, bparity);
-            sg.max_along = std::max(sg.max_along, sg.p[q].along);
-        }
-        sg.fin = f;
-        sg.fs = d_force_slot_;
-        sg.nfs = (gi == 0 && forces) ? 1 : 0;
-        sg.warm = (long long)d_.Nx * d_.Ny < (1LL << 20) ? 1 : 0;
-        CK(launch::stage_group(sg, d_.store, collide, gi == 0 && after_bulk, s));
-    }
+    for (size_t gi = 0; gi < groups_.size(); gi++)
+        CK(launch::stage_group(stage_group((int)gi, src, dst, write_macro, bparity, gi == 0 && forces), d_.store, collide,
+                               gi == 0 && after_bulk, s));
     return true;
+}
+
+// Group gi of the Boundary list for one step.
+StageGroup Solver::stage_group(int gi, int src, int dst, bool write_macro, int bparity, bool forces) const {
+    StageGroup sg;
+    std::memset(&sg, 0, sizeof sg);
+    if (groups_.empty()) return sg;
+    const std::vector<int> &g = groups_[gi];
+    sg.n = (int)g.size();
+    for (int q = 0; q < sg.n; q++) {
+        sg.p[q] = stage_params(stages_[g[q]], src, bparity);
+        sg.max_along = std::max(sg.max_along, sg.p[q].along);
+    }
+    sg.fin = finish_params(dst, write_macro, bparity);
+    sg.fs = d_force_slot_;
+    sg.nfs = forces ? 1 : 0;
+    sg.warm = (long long)d_.Nx * d_.Ny < (1LL << 20) ? 1 : 0;
+    return sg;
 }
 
 // One step (launch_step_kernels), then its records when probes or wall
@@ -1502,8 +1527,15 @@ bool Solver::launch_multi(int cur, int other, int lv) {
         StepParams p = step_params(at[q], at[q + 1], false, par);
         if (q & 1) p.stale = buf_[at[q - 1]];  // even states: two steps before
         if (!forces) p.mem_partials = nullptr;
-        CK(launch::special_shifted(fast_params(p), d_multi_list_[q], multi_count_[q], (nspecial_ + 31) / 32 * 32, d_.store,
-                                   true, true, false, stream_));
+        const int nforce = (nspecial_ + 31) / 32 * 32;
+        if (one_group_) {
+            CK(launch::near_shifted(fast_params(p), d_multi_list_[q], multi_count_[q], nforce, d_.store,
+                                    stage_group(0, at[q], at[q + 1], false, par, false), q > 0 && !forces, stream_));
+            if (forces) CK(launch::force_reduce(d_force_slot_, 1, false, stream_));
+            continue;
+        }
+        CK(launch::special_shifted(fast_params(p), d_multi_list_[q], multi_count_[q], nforce, d_.store, true, true, false,
+                                   stream_));
         if (!launch_edges(at[q], at[q + 1], true, false, par, forces, true, stream_)) return false;
     }
     CK(cudaStreamWaitEvent(stream_, multi_join_, 0));

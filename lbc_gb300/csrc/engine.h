@@ -296,6 +296,8 @@ class Solver {
     int stage_rows_ = 1;
     std::vector<Stage> stages_;
     std::vector<std::vector<int>> groups_;
+    bool one_group_ = false;  // at most one group, no periodic entries (near_shifted, edges_exact)
+    StageGroup stage_group(int gi, int src, int dst, bool write_macro, int bparity, bool forces) const;
     template <class Solid>
     bool group_stages(const Solid &solid, const std::vector<int> &colbase, const std::vector<int> &rowbase);
     // Per band slot: the last stage (index into stages_) that writes the node, -1 for none.

@@ -138,8 +138,12 @@ cudaError_t record(const RecordTask *tasks, int n, int store, const void *dst, c
                    int sel, bool collided, cudaStream_t s);
 // FP64 (kernels_exact.cu): lbc's rounding sequence, or with fma set the
 // fused multiply-add arithmetic (moments_fma / collide_fma)
+// (after: the programmatic follower of edges_exact, which it runs beside)
 cudaError_t step_exact(const StepParams &p, bool flags, bool collide, dim3 block, cudaStream_t s,
-                       int arith = ARITH_LBC);
+                       int arith = ARITH_LBC, bool after = false);
+// A step's whole Boundary list (one group, no periodic entries) from the
+// post-collision state: needs nothing of the step's bulk kernel. Collides.
+cudaError_t edges_exact(const StepParams &p, const StageGroup &g, int arith, cudaStream_t s);
 // collide: the finish of fused members applies the collision (false only in
 // the final step of a run, which leaves pre-collision populations).
 // after_bulk (here, stage_batch and force_reduce): the previous launch in s is
@@ -202,6 +206,12 @@ cudaError_t step_shifted(const FastStepParams &p, int store, bool flags, bool co
 // (a multiple of 32, or all) sum their wall-link force by chunks.
 cudaError_t special_shifted(const FastStepParams &p, const int2 *nodes, int n, int nforce, int store, bool flags, bool collide,
                             bool after_bulk, cudaStream_t s);
+// A step's special nodes (or a longer list of nodes, as special_shifted) and its
+// Boundary list, when that is one group without periodic entries, in one
+// launch; collides. g.nfs is not looked at (the force is reduced on its own).
+// after: the programmatic follower of the same launch of the step before.
+cudaError_t near_shifted(const FastStepParams &p, const int2 *nodes, int n, int nforce, int store, const StageGroup &g,
+                         bool after, cudaStream_t s);
 // The special nodes of a batch: nodes[q] = (case, i, j, chunk), n a multiple
 // of 32 (each case's list padded to 32 entries, i = -1); links: some case has
 // cut-link records.

@@ -236,33 +236,40 @@ __device__ __forceinline__ void stage_point(const StageParams &p, const StagePre
     bc_apply(a, p.w, kind, p.Nx, p.Ny, p.index, t, c.v1, c.v2);
 }
 
-// Moments and collision of a node an edge BC wrote (band slot `slot`).
-// live = false: the same instructions without their stores (warm-up pass);
-// band populations are read at L2, never from a possibly stale L1 line.
+// Moments and collision of a node an edge BC wrote (band slot `slot`), from its
+// pre-collision populations f.
+// live = false: the same instructions without their stores (warm-up pass).
 template <bool COLLIDE>
-__device__ __forceinline__ void finish_node_exact(const FinishParams &p, int2 ij, int slot, bool live) {
-    double f[9];
-#pragma unroll
-    for (int k = 0; k < 9; k++) f[k] = __ldcg(p.bandf + (size_t)k * p.nslots + slot);
+__device__ __forceinline__ void finish_pops_exact(const FinishParams &p, int2 ij, int slot, double f[9], int arith,
+                                                  bool live) {
     double rho, ux, uy;
-    moments_exact(f, p.hFx, p.hFy, rho, ux, uy);
     const size_t dn = (size_t)ij.y * p.Nx + ij.x;
+    const double om = COLLIDE ? (p.omega ? p.omega[dn] : p.omega0) : 0.0;
+    const bool done = arith == ARITH_INT && fi::step_node<COLLIDE>(f, p.w, p.has_force != 0, p.hFx, p.hFy, om, p.Fx, p.Fy,
+                                                                   rho, ux, uy);
+    if (!done) moments_exact(f, p.hFx, p.hFy, rho, ux, uy);
     if (live) {
         if (p.write_macro) { p.rho[dn] = rho; p.ux[dn] = ux; p.uy[dn] = uy; }
         p.bandm_next[slot] = rho;
         p.bandm_next[(size_t)p.nslots + slot] = ux;
         p.bandm_next[2 * (size_t)p.nslots + slot] = uy;
     }
-    if (COLLIDE) {
-        const double om = p.omega ? p.omega[dn] : p.omega0;
-        collide_exact(f, p.w, rho, ux, uy, om, p.has_force != 0, p.Fx, p.Fy);
-    }
+    if (COLLIDE && !done) collide_exact(f, p.w, rho, ux, uy, om, p.has_force != 0, p.Fx, p.Fy);
     double *D = (double *)p.dst;
     const long long node = (long long)ij.y * p.pitch + ij.x;
     if (live) {
 #pragma unroll
         for (int k = 0; k < 9; k++) D[k * p.plane + node] = f[k];
     }
+}
+
+// The same from the band, read at L2, never from a possibly stale L1 line.
+template <bool COLLIDE>
+__device__ __forceinline__ void finish_node_exact(const FinishParams &p, int2 ij, int slot, bool live) {
+    double f[9];
+#pragma unroll
+    for (int k = 0; k < 9; k++) f[k] = __ldcg(p.bandf + (size_t)k * p.nslots + slot);
+    finish_pops_exact<COLLIDE>(p, ij, slot, f, ARITH_LBC, live);
 }
 
 // One stage thread, specialised on the entry's kind; with warm set, a
@@ -299,6 +306,109 @@ __device__ __forceinline__ void stage_dispatch(const StageParams &p, const Finis
     LBM_STAGE_KIND(BC_VEL_BOT_ZH_FIX)
 #undef LBM_STAGE_KIND
     default: pdl_wait(); break;
+    }
+}
+
+// ---- edges beside the bulk kernel
+//
+// When the whole Boundary list is one group, an entry's thread pulls the node
+// that its BC reads itself and needs nothing of the bulk kernel's step
+// (near_shifted in kernels_shifted.cu does the same). The edge launch then goes
+// first and the bulk kernel runs beside it: a BC and its finish are a chain of
+// a few hundred FP64 instructions, 64 cycles each, which the bulk kernel's
+// blocks hide. Cylinder 1024 x 256 41.1 -> 26.7 us per step, 1000 x 400 with
+// Zou-He and convective edges 43.7 -> 35.1, cavity 129^2 17.8 -> 15.4.
+
+// The pre-collision populations of one node, as step_node_exact pulls them.
+__device__ __forceinline__ void pull_node_exact(const StepParams &p, int i, int j, double f[9]) {
+    const double *S = (const double *)p.src, *Old = (const double *)p.stale;
+    const long long pl = p.plane, node = (long long)j * p.pitch + i;
+    int im = i - 1, ip = i + 1, jm = j - 1, jp = j + 1;
+    if (p.px) { if (im < 0) im += p.Nx; if (ip >= p.Nx) ip -= p.Nx; }
+    else { im = max(im, 0); ip = min(ip, p.Nx - 1); }
+    if (p.py) { if (jm < 0) jm += p.Ny; if (jp >= p.Ny) jp -= p.Ny; }
+    else { jm = max(jm, 0); jp = min(jp, p.Ny - 1); }
+    const long long r0 = (long long)j * p.pitch, rm = (long long)jm * p.pitch, rp = (long long)jp * p.pitch;
+    const long long so[9] = {r0 + i, r0 + im, rm + i, r0 + ip, rp + i, rm + im, rm + ip, rp + ip, rp + im};
+    const uint16_t fl = p.flags[node];
+#pragma unroll
+    for (int k = 0; k < 9; k++) f[k] = S[k * pl + so[k]];
+    if (!(fl & (NF_SPECIAL_MASK | NF_SOLID))) return;
+    const Link *lk = (fl & NF_LINKS) ? p.links + p.link_off[node] : nullptr;
+#pragma unroll
+    for (int k = 0; k < 9; k++) {
+        if (fl & NF_SOLID) {
+            f[k] = Old[k * pl + node];
+            continue;
+        }
+        if (!(fl & (1u << k))) continue;
+        const int si = i - cxk(k), sj = j - cyk(k);
+        if ((!p.px && (si < 0 || si >= p.Nx)) || (!p.py && (sj < 0 || sj >= p.Ny))) {
+            f[k] = Old[k * pl + node];
+            continue;
+        }
+        const int ko = oppk(k);
+        const double own = S[ko * pl + node];
+        double val = own;
+        if (lk) {
+            const Link L = *lk++;
+            if (L.mode == LINK_IBB_LO) val = L.c1 * own + L.c2 * S[ko * pl + L.behind];
+            else if (L.mode == LINK_IBB_HI) val = L.c1 * own + L.c2 * S[k * pl + L.behind];
+            else if (L.mode == LINK_MOVING) val = own - L.c2;
+        }
+        f[k] = val;
+    }
+}
+
+struct EdgeAccessorExact {
+    const StagePre &c;
+    const double *f;   // the node that the entry reads
+    double *out;       // the node that it writes
+    __device__ double get(int, int, int k) const { return f[k]; }
+    __device__ void set(int, int, int k, double v) const { out[k] = v; }
+    __device__ double rho(int, int) const { return c.nrho; }
+    __device__ double ux(int, int) const { return c.nux; }
+    __device__ double uy(int, int) const { return c.nuy; }
+    __device__ double post(int, int, int) const { return 0.0; }  // periodic entries: not here
+    __device__ bool solid(int, int) const { return c.solid; }
+};
+
+template <int KIND>
+__device__ __forceinline__ void edge_thread_exact(const StepParams &sp, const StageParams &p, const FinishParams &f,
+                                                  int arith, int t) {
+    const StagePre c = stage_preload(p, t, KIND);
+    if (c.solid) return;
+    double in[9], out[9];
+    const int2 at = edge_reads_neighbour(KIND) ? c.nij : c.ij;
+    pull_node_exact(sp, at.x, at.y, in);
+#pragma unroll
+    for (int k = 0; k < 9; k++) out[k] = in[k];
+    EdgeAccessorExact a{c, in, out};
+    if (KIND == BC_VEL_BOT_REG && c.imp)
+        bc_regularized(a, p.w, t, p.index, t, p.index + 1, false, c.v1, c.v2);
+    else
+        bc_apply(a, p.w, KIND, p.Nx, p.Ny, p.index, t, c.v1, c.v2);
+    finish_pops_exact<true>(f, c.ij, c.slot, out, arith, true);
+}
+
+// `per` blocks of 32 threads per Boundary entry.
+__global__ void __launch_bounds__(32) k_edges_exact(const StepParams sp, int per, int arith, const StageGroup g) {
+    pdl_launch_dependents();
+    const StageParams &p = g.p[blockIdx.x / per];
+    const int t = (int)(blockIdx.x % per) * 32 + (int)threadIdx.x;
+    if (t >= p.along) return;
+    switch (p.kind) {
+#define LBM_EDGE_KIND(K) \
+    case K: edge_thread_exact<K>(sp, p, g.fin, arith, t); break;
+    LBM_EDGE_KIND(BC_VEL_IN_ZH) LBM_EDGE_KIND(BC_VEL_OUT_ZH) LBM_EDGE_KIND(BC_VEL_TOP_ZH)
+    LBM_EDGE_KIND(BC_VEL_BOT_ZH) LBM_EDGE_KIND(BC_PRES_IN_ZH) LBM_EDGE_KIND(BC_PRES_OUT_ZH)
+    LBM_EDGE_KIND(BC_CONV_IN) LBM_EDGE_KIND(BC_CONV_OUT)
+    LBM_EDGE_KIND(BC_VEL_IN_REG) LBM_EDGE_KIND(BC_VEL_OUT_REG)
+    LBM_EDGE_KIND(BC_VEL_TOP_REG) LBM_EDGE_KIND(BC_VEL_BOT_REG) LBM_EDGE_KIND(BC_PRES_IN_REG)
+    LBM_EDGE_KIND(BC_PRES_OUT_REG) LBM_EDGE_KIND(BC_PRES_TOP_REG) LBM_EDGE_KIND(BC_PRES_BOT_REG)
+    LBM_EDGE_KIND(BC_VEL_BOT_ZH_FIX)
+#undef LBM_EDGE_KIND
+    default: break;
     }
 }
 
@@ -785,21 +895,26 @@ cudaError_t fp64_rate(int blocks, int iters, double *sink, cudaStream_t s) {
 static dim3 grid2(int Nx, int Ny, dim3 b) { return dim3((Nx + b.x - 1) / b.x, (Ny + b.y - 1) / b.y); }
 
 template <int ARITH>
-static void step_exact_t(const StepParams &p, bool flags, bool collide, dim3 g, dim3 block, cudaStream_t s) {
+static cudaError_t step_exact_t(const StepParams &p, bool flags, bool collide, bool after, dim3 g, dim3 block,
+                                cudaStream_t s) {
     if (flags) {
-        if (collide) k_step_exact<true, true, ARITH><<<g, block, 0, s>>>(p);
-        else k_step_exact<true, false, ARITH><<<g, block, 0, s>>>(p);
-    } else {
-        if (collide) k_step_exact<false, true, ARITH><<<g, block, 0, s>>>(p);
-        else k_step_exact<false, false, ARITH><<<g, block, 0, s>>>(p);
+        if (collide) return launch_follower(after, k_step_exact<true, true, ARITH>, g, block, s, p);
+        return launch_follower(after, k_step_exact<true, false, ARITH>, g, block, s, p);
     }
+    if (collide) return launch_follower(after, k_step_exact<false, true, ARITH>, g, block, s, p);
+    return launch_follower(after, k_step_exact<false, false, ARITH>, g, block, s, p);
 }
 
-cudaError_t step_exact(const StepParams &p, bool flags, bool collide, dim3 block, cudaStream_t s, int arith) {
+cudaError_t step_exact(const StepParams &p, bool flags, bool collide, dim3 block, cudaStream_t s, int arith, bool after) {
     const dim3 g = grid2(p.Nx, p.Ny, block);
-    if (arith == ARITH_FMA) step_exact_t<ARITH_FMA>(p, flags, collide, g, block, s);
-    else if (arith == ARITH_INT) step_exact_t<ARITH_INT>(p, flags, collide, g, block, s);
-    else step_exact_t<ARITH_LBC>(p, flags, collide, g, block, s);
+    if (arith == ARITH_FMA) return step_exact_t<ARITH_FMA>(p, flags, collide, after, g, block, s);
+    if (arith == ARITH_INT) return step_exact_t<ARITH_INT>(p, flags, collide, after, g, block, s);
+    return step_exact_t<ARITH_LBC>(p, flags, collide, after, g, block, s);
+}
+
+cudaError_t edges_exact(const StepParams &p, const StageGroup &g, int arith, cudaStream_t s) {
+    const int per = (g.max_along + 31) / 32;
+    k_edges_exact<<<g.n * per, 32, 0, s>>>(p, per, arith, g);
     return cudaGetLastError();
 }
 

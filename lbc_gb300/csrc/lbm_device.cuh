@@ -669,6 +669,13 @@ __host__ __device__ __forceinline__ int2 stage_neighbour(int kind, int2 ij) {
     }
 }
 
+// Whether an entry of this kind reads its interior neighbour's populations.
+__host__ __device__ constexpr bool edge_reads_neighbour(int kind) {
+    return kind == BC_CONV_IN || kind == BC_CONV_OUT || kind == BC_VEL_IN_REG || kind == BC_VEL_OUT_REG ||
+           kind == BC_VEL_TOP_REG || kind == BC_VEL_BOT_REG || kind == BC_PRES_IN_REG || kind == BC_PRES_OUT_REG ||
+           kind == BC_PRES_TOP_REG || kind == BC_PRES_BOT_REG;
+}
+
 // What stage thread t reads that the bulk kernel of the same step does not
 // write: its node's solid flag and band slot, the neighbour's slot and
 // previous-step moments, the entry's values at t, whether it finishes the
