@@ -63,6 +63,16 @@ __device__ __forceinline__ float2 v_add(float2 a, float2 b) { return __fadd2_rn(
 __device__ __forceinline__ float2 v_sub(float2 a, float2 b) { return __ffma2_rn(b, make_float2(-1.f, -1.f), a); }
 __device__ __forceinline__ float2 v_mul(float2 a, float2 b) { return __fmul2_rn(a, b); }
 __device__ __forceinline__ float2 v_fma(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
+// A product that an addition follows. ptxas 13.0 contracts a packed multiply
+// and add into one multiply-add although both are written with their own
+// rounding (seen in one of the forced kernels: one ulp off in a node of 10^5),
+// so the packed product is a multiply-add of -0, which it does not know: 0x8000'0000
+// plus a block depth of one less one.
+__device__ __forceinline__ float v_mul_alone(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ float2 v_mul_alone(float2 a, float2 b) {
+    const float nz = __uint_as_float(0x80000000u + (blockDim.z - 1u));
+    return __ffma2_rn(a, b, make_float2(nz, nz));
+}
 __device__ __forceinline__ float2 v_rcp(float2 a) {
     const float2 r = make_float2(v_rcp_seed(a.x), v_rcp_seed(a.y));
     return __ffma2_rn(r, __ffma2_rn(make_float2(-a.x, -a.y), r, make_float2(1.0f, 1.0f)), r);
@@ -91,8 +101,8 @@ __device__ __forceinline__ void moments_v(const V g[9], V hFx, V hFy, V &dr, V &
     const V inv = v_rcp(rho);
     Jx = v_add(jx, hFx);
     Jy = v_add(jy, hFy);
-    ux = v_mul(Jx, inv);
-    uy = v_mul(Jy, inv);
+    ux = v_mul_alone(Jx, inv);
+    uy = v_mul_alone(Jy, inv);
 }
 
 // One pair of directions (k, opposite) of the equilibrium: X = w (dr + 4.5 J c
@@ -162,7 +172,7 @@ __device__ __forceinline__ void collide_v(V g[9], const float w[9], float h1, fl
     for (int q = 0; q < 4; q++) {
         const V cF = v_splat<V>(cFs[q]);
         const V S = v_fma(v_mul(v_splat<V>(9.0f), cu[q]), cF, n3uF);
-        const V E = v_mul(gf, v_mul(v_splat<V>(w[ka[q]]), S));
+        const V E = v_mul_alone(gf, v_mul(v_splat<V>(w[ka[q]]), S));
         const V O = v_splat<V>(hs[q] * cFs[q]);
         const int a = ka[q], b = kb[q];
         g[a] = v_add(g[a], v_fma(om, v_sub(geq[a], g[a]), v_add(E, O)));
