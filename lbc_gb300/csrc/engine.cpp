@@ -1313,7 +1313,11 @@ void Solver::advance(int nsteps) {
     }
 }
 
-// Two fused steps (cur -> other -> cur) captured once and replayed.
+// kGraphPairs pairs of fused steps (cur -> other -> cur) captured once and
+// replayed. A graph launch costs the device about 2 us beyond its kernels, which
+// a pair of small steps does not hide: Taylor-Green 64^2 FP32 3.10 us per step
+// with one pair per graph, 2.10 with four, 2.00 with sixteen; channel 256 x 64
+// FP64 9.25, 8.49, 8.27.
 bool Solver::capture_pair() {
     if (graph_valid_ && pair_cur_ == cur_ && pair_parity_ == parity_) return true;
     if (pair_exec_) {
@@ -1322,8 +1326,9 @@ bool Solver::capture_pair() {
     }
     cudaGraph_t g = nullptr;
     CK(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
-    bool okk = launch_step(cur_, 1 - cur_, true, false, parity_) &&
-               launch_step(1 - cur_, cur_, true, false, parity_ ^ 1);
+    bool okk = true;
+    for (int q = 0; q < kGraphPairs && okk; q++)
+        okk = launch_step(cur_, 1 - cur_, true, false, parity_) && launch_step(1 - cur_, cur_, true, false, parity_ ^ 1);
     cudaError_t e = cudaStreamEndCapture(stream_, &g);
     if (!okk) {
         if (g) cudaGraphDestroy(g);
@@ -1380,33 +1385,37 @@ void Solver::set_autotune(int mode) {
 }
 
 // Steps per pass of kernels_multi.cu for this case, 0: one at a time. Measured
-// per step (us) against the one-step kernel, Taylor-Green, FP32: 64^2 3.08 ->
-// 2.31, 512^2 5.13 -> 3.60, 1024^2 9.24 -> 6.95, 2048^2 46.4 -> 20.3, 4096^2
-// 173.5 -> 71.4. Four levels, except where the grid gives too few warps to hide
-// four dependent collisions per row: 512 x 256 3.08 with two, 3.60 with four;
-// 768^2 the same with either. FP16's one-step kernel moves half the bytes, so
-// only larger grids gain: 512^2 4.11 -> 4.87, 768^2 6.17 -> 6.43, 1024^2 9.24 ->
-// 8.73, 4096^2 112.5 -> 80.4.
+// per step (us) against the one-step kernels, both from captured graphs.
+// Periodic FP32: 256^2 2.31 against 2.83 with two levels and 2.72 with four;
+// 512^2 4.01, 3.34, 3.88; 1024 x 768 6.43, 6.42, 5.65; 1024^2 8.21, 7.98, 6.75;
+// 2048^2 46.4, 31.6, 20.3; 4096^2 173.5, 111.5, 71.4: small grids have too few
+// warps to hide the dependent collisions of a row. FP16's one-step kernel moves
+// half the bytes: 1500 x 1100 11.1 against 12.0 with four levels, 2048^2 31.0
+// against 24.6, 4096^2 112.5 against 80.4.
 int Solver::multi_levels() const {
     const long long n = (long long)d_.Nx * d_.Ny;
     if (d_.store == STORE_F64 || d_omega_ || !rec_host_.empty()) return 0;
     if (d_.Nx < 8 || d_.Ny < 8 || plane_ >= (1LL << 31)) return 0;
     // With a flag word the nodes near walls and edges go step by step beside the
-    // pass, a chain of launches that bounds small grids. Cavity 512^2 7.22 ->
-    // 6.80 with two levels, 1024^2 11.3 -> 9.98 (10.6 with four), 2048^2 50.4 ->
-    // 36.8 and 25.6 with four, 4096^2 184 -> 85; channel 1024 x 256 6.21 -> 5.23
-    // (7.04); cylinder 2048 x 512 16.5 -> 14.6 (13.5).
-    if (has_flags_) return n < (1LL << 18) ? 0 : n < (1LL << 21) ? 2 : 4;
-    if (d_.store == STORE_F16) return n >= (1LL << 20) ? 4 : 0;
-    return n >= (1LL << 17) && n < (1LL << 19) ? 2 : 4;
+    // pass, a chain of launches that bounds small grids. FP32: cylinder 1024 x
+    // 256 8.30 against 7.78 with two levels and 8.00 with four, 2048 x 512 10.9,
+    // 10.2, 10.2; cavity 1024^2 10.6, 9.85, 9.07, 2048^2 49.1, 35.7, 25.4, 4096^2
+    // 184, 131, 85. FP16: cavity 1024^2 9.6, 10.5, 9.6, 2048^2 34.2, 27.7, 26.5;
+    // channel 3000 x 750 21.0, 20.2, 22.3.
+    if (has_flags_ && d_.store == STORE_F16) return n < (1LL << 21) ? 0 : n < (3LL << 20) ? 2 : 4;
+    if (has_flags_) return n < (1LL << 18) ? 0 : n < (1LL << 20) ? 2 : 4;
+    if (d_.store == STORE_F16) return n >= (1LL << 21) ? 4 : 0;
+    return n < (1LL << 18) ? 0 : n < (1LL << 19) ? 2 : 4;
 }
 
 // Warps a pass is split into: 8 per SM while the state is in the L2 cache
-// (1024^2 FP32 6.95 us per step, 7.46 with 12), the 12 that fit beyond that;
-// FP16 keeps more in flight (4096^2: 92 us with 12, 81 with 24).
+// (1024^2 FP32 6.95 us per step, 7.46 with 12; the lists beside a pass also find
+// room: cylinder 2048 x 512 10.2, 12.2 with 12), the 12 that fit beyond that
+// (cavity 2048^2 25.5, 28.4 with 8). FP16 keeps more in flight (4096^2: 92 us
+// with 12, 81 with 24; cavity 96 with 12, 88 with 16, 91 with 20).
 int Solver::multi_warps() const {
     const long long n = (long long)d_.Nx * d_.Ny;
-    return launch::sm_count() * (n < (1LL << 21) ? 8 : d_.store == STORE_F16 ? 24 : 12);
+    return launch::sm_count() * (n < (1LL << 21) ? 8 : d_.store == STORE_F32 ? 12 : has_flags_ ? 16 : 24);
 }
 
 // A case with a flag word in passes of several steps. Nodes at least `levels`
@@ -1542,7 +1551,7 @@ bool Solver::launch_multi(int cur, int other, int lv) {
     return true;
 }
 
-// Two passes (cur -> other -> cur) captured once and replayed.
+// kGraphPairs / 2 double passes (cur -> other -> cur) captured once and replayed.
 bool Solver::capture_multi() {
     if (multi_exec_ && multi_cur_ == cur_ && multi_parity_ == parity_ && graph_valid_multi_) return true;
     if (multi_exec_) {
@@ -1552,7 +1561,8 @@ bool Solver::capture_multi() {
     cudaGraph_t g = nullptr;
     CK(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
     const int lv = multi_levels();
-    const bool okk = launch_multi(cur_, 1 - cur_, lv) && launch_multi(1 - cur_, cur_, lv);
+    bool okk = true;
+    for (int q = 0; q < kGraphPairs / 2 && okk; q++) okk = launch_multi(cur_, 1 - cur_, lv) && launch_multi(1 - cur_, cur_, lv);
     cudaError_t e = cudaStreamEndCapture(stream_, &g);
     if (!okk) {
         if (g) cudaGraphDestroy(g);
@@ -1577,14 +1587,20 @@ int Solver::run_multi(int avail) {
                                                             buf_[cur_], buf_[1 - cur_], buf_[2], lv > 2 ? buf_[3] : nullptr,
                                                             enter, stream_), "multi_swap");
     };
-    if (!capture_multi() || !swap(true)) return -1;
+    if (!swap(true)) return -1;
     int used = 0;
+    const int whole = kGraphPairs * lv;
+    if (avail >= whole) {
+        if (!capture_multi()) return -1;
+        for (; avail - used >= whole; used += whole)
+            if (!check_cuda(cudaGraphLaunch(multi_exec_, stream_), "cudaGraphLaunch")) return -1;
+    }
     for (; avail - used >= 2 * lv; used += 2 * lv)
-        if (!check_cuda(cudaGraphLaunch(multi_exec_, stream_), "cudaGraphLaunch")) return -1;
+        if (!launch_multi(cur_, 1 - cur_, lv) || !launch_multi(1 - cur_, cur_, lv)) return -1;
     return swap(false) ? used : -1;
 }
 
-// One fused step cur -> other, as inside run().
+// One fused step cur -> other.
 bool Solver::trial_step() {
     if (!launch_step(cur_, 1 - cur_, true, false, parity_)) return false;
     cur_ ^= 1;
@@ -1646,18 +1662,12 @@ bool Solver::run(int nsteps) {
     const int used = run_multi(remaining);
     if (used < 0) return false;
     remaining -= used;
-    if (remaining >= 2) {
+    if (remaining >= 2 * kGraphPairs) {
         if (!capture_pair()) return false;
-        while (remaining >= 2) {
-            CK(cudaGraphLaunch(pair_exec_, stream_));
-            remaining -= 2;
-        }
+        for (; remaining >= 2 * kGraphPairs; remaining -= 2 * kGraphPairs) CK(cudaGraphLaunch(pair_exec_, stream_));
     }
-    if (remaining == 1) {
-        if (!launch_step(cur_, 1 - cur_, true, false, parity_)) return false;
-        cur_ ^= 1;
-        parity_ ^= 1;
-    }
+    for (; remaining > 0; remaining--)
+        if (!trial_step()) return false;
     if (!launch_step(cur_, 1 - cur_, false, true, parity_)) return false;
     cur_ ^= 1;
     parity_ ^= 1;
@@ -2011,7 +2021,8 @@ bool Batch::capture_pair() {
     if (pair_exec_) return true;
     cudaGraph_t g = nullptr;
     CK(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
-    const bool okk = launch_batched(0) && launch_batched(1);
+    bool okk = true;
+    for (int q = 0; q < kGraphPairs && okk; q++) okk = launch_batched(0) && launch_batched(1);
     const cudaError_t e = cudaStreamEndCapture(stream_, &g);
     if (!okk) {
         if (g) cudaGraphDestroy(g);
@@ -2098,8 +2109,9 @@ bool Batch::run(int nsteps) {
             okk = used >= 0;
             pairs -= std::max(used, 0);
         }
-        if (okk && pairs > 0) okk = capture_pair();
-        for (; okk && pairs > 0; pairs--) okk = check_cuda(cudaGraphLaunch(pair_exec_, stream_), "graph");
+        if (okk && pairs >= kGraphPairs) okk = capture_pair();
+        for (; okk && pairs >= kGraphPairs; pairs -= kGraphPairs) okk = check_cuda(cudaGraphLaunch(pair_exec_, stream_), "graph");
+        for (; okk && pairs > 0; pairs--) okk = launch_batched(0) && launch_batched(1);
         if (okk && (mid & 1)) okk = launch_batched(0);
         for (Solver *c : cases_) {
             c->advance(mid);

@@ -89,6 +89,9 @@ struct Stage {
     unsigned long long trace_written = 0;
 };
 
+// Step pairs per captured graph.
+constexpr int kGraphPairs = 4;
+
 // Most probes a solver records (one block of a record launch walks them).
 constexpr int kMaxProbes = 4096;
 
