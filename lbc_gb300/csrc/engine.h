@@ -323,6 +323,10 @@ class Solver {
     long long steps_done_ = 0;
     std::vector<void *> allocs_;
     bool needs_old_dst_ = true;
+    // FP64 storage: the nodes the step may leave old content in (solid, or a
+    // source solid or off the grid), for the drop-in's step
+    std::vector<int2> old_host_;
+    int2 *d_old_nodes_ = nullptr;
     bool fields_are_moments_ = false;  // stored rho/u/v are the moments of the current populations
     std::vector<uint8_t> link_node_;
     mutable std::map<int, std::vector<int4>> tile_cache_;

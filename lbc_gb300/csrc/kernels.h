@@ -165,6 +165,9 @@ cudaError_t collide_exact(const CollideParams &p, cudaStream_t s);
 cudaError_t collide_aos_exact(const CollideAosParams &p, cudaStream_t s);
 cudaError_t aos_to_soa(const double *aos, void *soa, int store, int Nx, int Ny, int pitch,
                        long long plane, const double w[9], cudaStream_t s);
+// FP64, the listed nodes only.
+cudaError_t aos_to_soa_nodes(const double *aos, double *soa, const int2 *nodes, int n, int Nx, int pitch,
+                             long long plane, cudaStream_t s);
 cudaError_t soa_to_aos(const void *soa, double *aos, int store, int Nx, int Ny, int pitch,
                        long long plane, const double w[9], cudaStream_t s);
 cudaError_t seed_band(const int2 *nodes, const int *slots, int n, int Nx, const double *rho,

@@ -534,6 +534,17 @@ __global__ void k_aos_to_soa(const double *__restrict__ aos, T *__restrict__ soa
     }
 }
 
+// The same for a list of nodes, FP64: a thread per population, so that a node's
+// 72 bytes cross the host link together.
+__global__ void k_aos_to_soa_nodes(const double *__restrict__ aos, double *__restrict__ soa,
+                                   const int2 *__restrict__ nodes, int n, int Nx, int pitch, long long plane) {
+    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= 9LL * n) return;
+    const int2 ij = nodes[t / 9];
+    const int k = (int)(t % 9);
+    soa[k * plane + (long long)ij.y * pitch + ij.x] = aos[((long long)ij.y * Nx + ij.x) * 9 + k];
+}
+
 template <typename T>
 __global__ void k_soa_to_aos(const T *__restrict__ soa, double *__restrict__ aos, int Nx, int Ny,
                              int pitch, long long plane, Wt w) {
@@ -979,6 +990,13 @@ cudaError_t aos_to_soa(const double *aos, void *soa, int store, int Nx, int Ny, 
     if (store == STORE_F64) k_aos_to_soa<double><<<g, 256, 0, s>>>(aos, (double *)soa, Nx, Ny, pitch, plane, wt);
     else if (store == STORE_F32) k_aos_to_soa<float><<<g, 256, 0, s>>>(aos, (float *)soa, Nx, Ny, pitch, plane, wt);
     else k_aos_to_soa<__half><<<g, 256, 0, s>>>(aos, (__half *)soa, Nx, Ny, pitch, plane, wt);
+    return cudaGetLastError();
+}
+
+cudaError_t aos_to_soa_nodes(const double *aos, double *soa, const int2 *nodes, int n, int Nx, int pitch,
+                             long long plane, cudaStream_t s) {
+    if (n == 0) return cudaSuccess;
+    k_aos_to_soa_nodes<<<(unsigned)((9LL * n + 255) / 256), 256, 0, s>>>(aos, soa, nodes, n, Nx, pitch, plane);
     return cudaGetLastError();
 }
 
