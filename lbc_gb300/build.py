@@ -4,6 +4,7 @@ Translation units are compiled in parallel with nvcc:
   kernels_exact.cu    --fmad=false (lbc's FP64 rounding sequence, bit for bit)
   kernels_shifted.cu  FP32/FP16 shifted-storage kernels (--fmad=false as well: FMAs
                       are written out, so every kernel rounds a node the same way)
+  kernels_near.cu     the same arithmetic, special nodes and edges in one launch
   kernels_multi.cu    the same arithmetic, several time steps per pass
   engine.cpp, dropin.cpp  host code (-ffp-contract=off: same host arithmetic on
                           x86-64 and aarch64)
@@ -25,6 +26,7 @@ ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 UNITS = [
     ("kernels_exact.cu", ["-O3", "-lineinfo", "--fmad=false"] + ARCH),
     ("kernels_shifted.cu", ["-O3", "-lineinfo", "--fmad=false"] + ARCH),
+    ("kernels_near.cu", ["-O3", "-lineinfo", "--fmad=false"] + ARCH),
     ("kernels_multi.cu", ["-O3", "-lineinfo", "--fmad=false"] + ARCH),
     ("engine.cpp", ["-O2"]),
     ("dropin.cpp", ["-O2"]),

@@ -894,6 +894,7 @@ StageParams Solver::stage_params(const Stage &st, int src, int bparity) const {
     s.flags = d_flags_; s.colbase = d_colbase_; s.rowbase = d_rowbase_; s.nslots = nslots_;
     s.bandf = d_bandf_; s.bandg = d_bandg_; s.bandm_prev = d_bandm_[bparity];
     s.src = buf_[src];
+    s.step = nullptr;
     for (int k = 0; k < 9; k++) {
         s.w[k] = d_.w[k];
         s.wf[k] = (float)d_.w[k];
@@ -1085,12 +1086,12 @@ bool Solver::launch_step_kernels(int src, int dst, bool collide, bool write_macr
         // (the plain kernel of a flag-free grid steps its own odd column).
         // What follows is an ordinary launch, so it sees both. A Boundary list
         // of one group steps with the special nodes (near_shifted).
-        const bool near = collide && !write_macro && special_launch() && one_group_ && !groups_.empty();
+        const bool near = collide && !write_macro && special_launch() && one_group_ && !groups_.empty() && !wide();
         if (near)
-            CK(launch::near_shifted(fp, d_special_, nspecial_, nspecial_, d_.store,
+            CK(launch::near_shifted(fp, d_special_, nspecial_, nullptr, 0, d_.store,
                                     stage_group(0, src, dst, write_macro, bparity, false), false, s));
         else if (special_launch())
-            CK(launch::special_shifted(fp, d_special_, nspecial_, nspecial_, d_.store, true, collide, false, s));
+            CK(launch::special_shifted(fp, d_special_, nspecial_, d_.store, true, collide, false, s));
         CK(launch::step_shifted(fp, d_.store, has_flags_, collide, block_, s, special_launch()));
         if (near) {
             if (forces) CK(launch::force_reduce(d_force_slot_, 1, false, s));
@@ -1408,7 +1409,7 @@ void Solver::set_autotune(int mode) {
 int Solver::multi_levels() const {
     const long long n = (long long)d_.Nx * d_.Ny;
     if (d_.store == STORE_F64 || d_omega_ || !rec_host_.empty()) return 0;
-    if (d_.Nx < 8 || d_.Ny < 8 || plane_ >= (1LL << 31)) return 0;
+    if (d_.Nx < 8 || d_.Ny < 8 || plane_ >= (1LL << 31) || (has_flags_ && wide())) return 0;
     // With a flag word the nodes near walls and edges go step by step beside the
     // pass, a chain of launches that bounds small grids. FP32: cylinder 1024 x
     // 256 8.30 against 7.78 with two levels and 8.00 with four, 2048 x 512 10.9,
@@ -1431,33 +1432,25 @@ int Solver::multi_warps() const {
     return launch::sm_count() * (n < (1LL << 21) ? 8 : d_.store == STORE_F32 ? 12 : has_flags_ ? 16 : 24);
 }
 
-// A case with a flag word in passes of several steps. Nodes at least `levels`
-// nodes away from every special node step by the pass kernel (multi_geo), which
-// reads the state before the pass and writes the one after it. The nodes near
-// special ones cannot: they go step by step, as a list per step (the special
-// nodes, then every node that the following steps of the list pull from) in
-// buffers 2 and 3, with the Boundary list after each step, on a stream of their
-// own beside the pass kernel. multi_swap moves what lbc's two buffers keep in
-// solid nodes and off-grid slots between the buffers' roles.
-bool Solver::multi_setup() {
-    if (multi_state_) return multi_state_ > 0;
-    multi_state_ = -1;
-    const int Nx = d_.Nx, Ny = d_.Ny, lv = multi_levels();
-    const size_t N = (size_t)Nx * Ny;
-    if (nspecial_ == 0 || (size_t)nspecial_ > N / 8) return false;
-    for (const Stage &st : stages_)  // these read post-collision values of the opposite edge
-        if (st.kind == BC_PERIODIC_X || st.kind == BC_PERIODIC_Y) return false;
-    size_t freeb = 0, total = 0;
-    const size_t need = (size_t)(lv > 2 ? 2 : 1) * 9 * (size_t)plane_ * esize_;
-    if (cudaMemGetInfo(&freeb, &total) != cudaSuccess || freeb / 4 < need) return false;
+// A case with special nodes in passes of `lv` steps. Nodes at least lv nodes
+// away from every special node step by the pass kernel, which reads the state
+// before the pass and writes the one after it (plan.deep: a word per strip and
+// row, a bit per pair). The nodes near special ones cannot: they go step by
+// step (plan.segs: for each step the clean pairs that this or a following step
+// of the list pulls from, as masks over 64 columns of a row) with the special
+// nodes and the Boundary list in buffers 2 and 3, on a stream of their own
+// beside the pass kernel. multi_swap moves what lbc's two buffers keep in solid
+// nodes and off-grid slots between the buffers' roles.
+void Solver::near_plan(int lv, NearPlan &plan) const {
+    const int Nx = d_.Nx, Ny = d_.Ny;
     // Distance to the nearest special node (the larger of |dx|, |dy|), up to m,
     // by runs of special nodes along a row.
-    const int m = 2 * lv - 1;
-    std::vector<uint8_t> dist(N, 255);
-    for (int q = 0; q < nspecial_;) {
+    const int m = 2 * lv - 1, nsp = (int)special_host_.size();
+    std::vector<uint8_t> dist((size_t)Nx * Ny, 255);
+    for (int q = 0; q < nsp;) {
         const int y = special_host_[q].y, i0 = special_host_[q].x & ~kSpecialSolid;
         int i1 = i0;
-        for (q++; q < nspecial_ && special_host_[q].y == y && (special_host_[q].x & ~kSpecialSolid) == i1 + 1; q++) i1++;
+        for (q++; q < nsp && special_host_[q].y == y && (special_host_[q].x & ~kSpecialSolid) == i1 + 1; q++) i1++;
         for (int dy = -m; dy <= m; dy++) {
             int j = y + dy;
             if (!wrap(j, Ny, d_.py)) continue;
@@ -1473,53 +1466,99 @@ bool Solver::multi_setup() {
         }
     }
     // Deep pairs, both nodes lv or more away: every pair of the grid, then the
-    // near ones taken out as they join the lists.
+    // near ones taken out as they join the segments.
     const int halo = multi_halo(lv), width = 64 - 2 * halo, strips = (Nx + width - 1) / width;
-    std::vector<uint32_t> deep((size_t)strips * Ny);
+    plan.deep.resize((size_t)strips * Ny);
     for (int st = 0; st < strips; st++) {
         uint32_t all = 0;
         for (int c = 0; c < width && st * width + c + 1 < Nx; c += 2) all |= 1u << ((c + halo) / 2);
-        std::fill(deep.begin() + (size_t)st * Ny, deep.begin() + (size_t)(st + 1) * Ny, all);
+        std::fill(plan.deep.begin() + (size_t)st * Ny, plan.deep.begin() + (size_t)(st + 1) * Ny, all);
     }
-    std::vector<std::vector<int2>> list(lv, special_host_);
-    for (std::vector<int2> &l : list)
-        while (l.size() % 32) l.push_back(make_int2(-1, -1));
+    plan.segs.assign(lv, std::vector<int4>());
+    plan.near_pairs = 0;
     for (int j = 0; j < Ny; j++) {
         const uint8_t *row = &dist[(size_t)j * Nx];
-        for (int i = 0; i < Nx; i += 2) {
-            uint64_t eight;
-            if (i + 8 <= Nx && (std::memcpy(&eight, row + i, 8), eight == ~0ull)) {
-                i += 6;
-                continue;
+        for (int s0 = 0; s0 < Nx; s0 += 64) {
+            uint32_t mask[4] = {0, 0, 0, 0};
+            bool any = false;
+            for (int l = 0; l < 32 && s0 + 2 * l < Nx; l++) {
+                const int i = s0 + 2 * l;
+                uint64_t eight;
+                if (l % 4 == 0 && i + 8 <= Nx && (std::memcpy(&eight, row + i, 8), eight == ~0ull)) {
+                    l += 3;
+                    continue;
+                }
+                if (i + 1 >= Nx) continue;  // an odd last column is special
+                const int d = std::min(row[i], row[i + 1]);
+                if (d < lv) plan.deep[(size_t)(i / width) * Ny + j] &= ~(1u << ((i % width + halo) / 2));
+                if (d == 0) continue;       // special: both nodes of the pair
+                // step q + 1 of the list needs the nodes within 2 lv - (q + 1) of
+                // a special one; the last, every pair that is not deep
+                for (int q = 0; q < lv; q++)
+                    if (q == lv - 1 ? d < lv : d < 2 * lv - q) {
+                        mask[q] |= 1u << l;
+                        any = true;
+                    }
             }
-            const bool two = i + 1 < Nx;
-            const bool is_deep = two && row[i] >= lv && row[i + 1] >= lv;
-            if (!is_deep) deep[(size_t)(i / width) * Ny + j] &= ~(1u << ((i % width + halo) / 2));
-            // step q + 1 of the list needs the nodes within 2 lv - (q + 1) of a
-            // special one; the last, every node that is not deep
-            for (int h = 0; h < (two ? 2 : 1); h++) {
-                const int d = row[i + h];
-                if (d == 0) continue;
-                for (int q = 0; q < lv - 1; q++)
-                    if (d < 2 * lv - q) list[q].push_back(make_int2(i + h, j));
-                if (!is_deep) list[lv - 1].push_back(make_int2(i + h, j));
-            }
+            for (int q = 0; any && q < lv; q++)
+                if (mask[q]) {
+                    plan.segs[q].push_back(make_int4(0, j, s0, (int)mask[q]));
+                    plan.near_pairs += __builtin_popcount(mask[q]);
+                }
         }
     }
-    if (!dalloc(&d_deep_, deep.size())) return false;
-    CK(cudaMemcpyAsync(d_deep_, deep.data(), deep.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, stream_));
-    for (int q = 0; q < lv; q++) {
-        int2 *l = nullptr;
-        if (!dalloc(&l, list[q].size())) return false;
-        CK(cudaMemcpyAsync(l, list[q].data(), list[q].size() * sizeof(int2), cudaMemcpyHostToDevice, stream_));
-        d_multi_list_[q] = l;
-        multi_count_[q] = (int)list[q].size();
-    }
+}
+
+bool Solver::multi_buffers(int lv) {
     for (int b = 2; b < (lv > 2 ? 4 : 3); b++) {
+        if (buf_[b]) continue;
         char *q = nullptr;
-        if (!dalloc(&q, 9 * (size_t)plane_ * esize_)) return false;
+        if (!dalloc(&q, multi_bytes())) return false;
         buf_[b] = q;
     }
+    return true;
+}
+
+// multi_swap before a run of passes (enter) and after it.
+bool Solver::swap_multi(bool enter, int lv, cudaStream_t s) {
+    if (!has_flags_) return true;
+    CK(launch::multi_swap(d_special_, nspecial_, d_flags_, pitch_, plane_, d_.store, buf_[cur_], buf_[1 - cur_], buf_[2],
+                          lv > 2 ? buf_[3] : nullptr, enter, s));
+    return true;
+}
+
+// The parameters of step q (0 .. lv - 1) of the near nodes in a pass cur -> other.
+StepParams Solver::near_params(int cur, int other, int lv, int q) const {
+    const int src = near_buffer(cur, other, lv, q), dst = near_buffer(cur, other, lv, q + 1);
+    StepParams p = step_params(src, dst, false, parity_ ^ (q & 1));
+    // States of odd steps stay in buffer 2, so it holds its own of two steps
+    // before; those of even steps alternate.
+    if (q & 1) p.stale = buf_[near_buffer(cur, other, lv, q - 1)];
+    p.mem_partials = nullptr;
+    return p;
+}
+
+// Sets a case alone up for passes; false: not this case.
+bool Solver::multi_setup() {
+    if (multi_state_) return multi_state_ > 0;
+    multi_state_ = -1;
+    const int lv = multi_levels();
+    if (nspecial_ == 0 || (long long)nspecial_ > (long long)d_.Nx * d_.Ny / 8) return false;
+    for (const Stage &st : stages_)  // these read post-collision values of the opposite edge
+        if (st.kind == BC_PERIODIC_X || st.kind == BC_PERIODIC_Y) return false;
+    size_t freeb = 0, total = 0;
+    if (cudaMemGetInfo(&freeb, &total) != cudaSuccess || freeb / 4 < (size_t)(lv > 2 ? 2 : 1) * multi_bytes()) return false;
+    NearPlan plan;
+    near_plan(lv, plan);
+    if (!dalloc(&d_deep_, plan.deep.size())) return false;
+    CK(cudaMemcpyAsync(d_deep_, plan.deep.data(), plan.deep.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, stream_));
+    for (int q = 0; q < lv; q++) {
+        if (!dalloc(&d_near_segs_[q], plan.segs[q].size())) return false;
+        CK(cudaMemcpyAsync(d_near_segs_[q], plan.segs[q].data(), plan.segs[q].size() * sizeof(int4),
+                           cudaMemcpyHostToDevice, stream_));
+        near_segs_[q] = (int)plan.segs[q].size();
+    }
+    if (!multi_buffers(lv)) return false;
     int lo = 0, hi = 0;
     cudaDeviceGetStreamPriorityRange(&lo, &hi);
     CK(cudaStreamCreateWithPriority(&multi_stream_, cudaStreamNonBlocking, lo));
@@ -1542,23 +1581,21 @@ bool Solver::launch_multi(int cur, int other, int lv) {
     CK(launch::multi_geo(whole, d_.store, lv, d_deep_, multi_warps(), multi_stream_));
     CK(cudaEventRecord(multi_join_, multi_stream_));
     const bool forces = has_mem_ && hist_cap_ > 0;
-    int at[5] = {cur, 2, 3, 2, other};  // the buffer of each step's state
-    at[lv] = other;
     for (int q = 0; q < lv; q++) {
-        const int par = parity_ ^ (q & 1);
-        StepParams p = step_params(at[q], at[q + 1], false, par);
-        if (q & 1) p.stale = buf_[at[q - 1]];  // even states: two steps before
-        if (!forces) p.mem_partials = nullptr;
-        const int nforce = (nspecial_ + 31) / 32 * 32;
-        if (one_group_) {
-            CK(launch::near_shifted(fast_params(p), d_multi_list_[q], multi_count_[q], nforce, d_.store,
-                                    stage_group(0, at[q], at[q + 1], false, par, false), q > 0 && !forces, stream_));
-            if (forces) CK(launch::force_reduce(d_force_slot_, 1, false, stream_));
-            continue;
+        const int src = near_buffer(cur, other, lv, q), dst = near_buffer(cur, other, lv, q + 1), par = parity_ ^ (q & 1);
+        StepParams p = near_params(cur, other, lv, q);
+        if (forces) p.mem_partials = d_partials_;
+        // (a follower only of the same launch: nothing else in between)
+        StageGroup sg;
+        if (one_group_) sg = stage_group(0, src, dst, false, par, false);
+        else std::memset(&sg, 0, sizeof sg);
+        CK(launch::near_shifted(fast_params(p), d_special_, nspecial_, d_near_segs_[q], near_segs_[q], d_.store, sg,
+                                q > 0 && one_group_ && !forces, stream_));
+        if (!one_group_) {
+            if (!launch_edges(src, dst, true, false, par, forces, true, stream_)) return false;
+        } else if (forces) {
+            CK(launch::force_reduce(d_force_slot_, 1, false, stream_));
         }
-        CK(launch::special_shifted(fast_params(p), d_multi_list_[q], multi_count_[q], nforce, d_.store, true, true, false,
-                                   stream_));
-        if (!launch_edges(at[q], at[q + 1], true, false, par, forces, true, stream_)) return false;
     }
     CK(cudaStreamWaitEvent(stream_, multi_join_, 0));
     return true;
@@ -1595,12 +1632,7 @@ bool Solver::capture_multi() {
 int Solver::run_multi(int avail) {
     const int lv = multi_levels();
     if (lv == 0 || avail < 2 * lv || (has_flags_ && (avail < 8 * lv || !multi_setup()))) return 0;
-    auto swap = [&](bool enter) {
-        return !has_flags_ || check_cuda(launch::multi_swap(d_special_, nspecial_, d_flags_, pitch_, plane_, d_.store,
-                                                            buf_[cur_], buf_[1 - cur_], buf_[2], lv > 2 ? buf_[3] : nullptr,
-                                                            enter, stream_), "multi_swap");
-    };
-    if (!swap(true)) return -1;
+    if (!swap_multi(true, lv, stream_)) return -1;
     int used = 0;
     const int whole = kGraphPairs * lv;
     if (avail >= whole) {
@@ -1610,7 +1642,7 @@ int Solver::run_multi(int avail) {
     }
     for (; avail - used >= 2 * lv; used += 2 * lv)
         if (!launch_multi(cur_, 1 - cur_, lv) || !launch_multi(1 - cur_, cur_, lv)) return -1;
-    return swap(false) ? used : -1;
+    return swap_multi(false, lv, stream_) ? used : -1;
 }
 
 // One fused step cur -> other.
@@ -1732,6 +1764,10 @@ Batch::Batch(const std::vector<Solver *> &cases) : cases_(cases) {
 
 Batch::~Batch() {
     if (pair_exec_) cudaGraphExecDestroy(pair_exec_);
+    if (multi_exec_) cudaGraphExecDestroy(multi_exec_);
+    if (multi_fork_) cudaEventDestroy(multi_fork_);
+    if (multi_join_) cudaEventDestroy(multi_join_);
+    if (multi_stream_) cudaStreamDestroy(multi_stream_);
     if (params_ev_) {
         cudaEventSynchronize(params_ev_);
         cudaEventDestroy(params_ev_);
@@ -2048,6 +2084,150 @@ bool Batch::capture_pair() {
     return true;
 }
 
+// Passes of several steps for the whole batch (Solver::near_plan): per pass one
+// launch of warps over strips and rows of every case, and beside it one launch
+// per step of every case's special nodes, near pairs and edges. Large batches
+// of cases whose Boundary lists are one group, without records.
+bool Batch::multi_setup() {
+    if (multi_state_) return multi_state_ > 0;
+    multi_state_ = -1;
+    const int lv = multi_lv_;
+    if (store_ == STORE_F64 || nodes_ < (store_ == STORE_F32 ? (1LL << 20) : (1LL << 22)) || nrec_ || max_stages_ > 1)
+        return false;
+    size_t need = 0, freeb = 0, total = 0;
+    for (Solver *c : cases_) {
+        if (!c->multi_case()) return false;
+        need += 2 * c->multi_bytes();
+    }
+    if (cudaMemGetInfo(&freeb, &total) != cudaSuccess || freeb / 4 < need) return false;
+    std::vector<uint32_t> deep;
+    std::vector<std::vector<int4>> segs(lv);
+    std::vector<MultiTask> tasks;
+    long long near = 0;
+    const int halo = multi_halo(lv), width = 64 - 2 * halo;
+    for (size_t c = 0; c < cases_.size(); c++) {
+        NearPlan plan;
+        cases_[c]->near_plan(lv, plan);
+        near += 2 * plan.near_pairs;
+        for (int q = 0; q < lv; q++)
+            for (int4 e : plan.segs[q]) segs[q].push_back(make_int4((int)c, e.y, e.z, e.w));
+        // Chunks of about kTaskRows rows: enough tasks to even out cases of
+        // different height, few enough rows walked twice (2 (lv - 1) per chunk).
+        const int Nx = cases_[c]->Nx(), Ny = cases_[c]->Ny(), strips = (Nx + width - 1) / width;
+        const int chunks = std::max(1, (Ny + kTaskRows / 2) / kTaskRows), h = (Ny + chunks - 1) / chunks;
+        for (int y = 0; y < Ny; y += h)
+            for (int st = 0; st < strips; st++)
+                tasks.push_back(MultiTask{(int)c, st, y, std::min(Ny, y + h), (long long)deep.size()});
+        deep.insert(deep.end(), plan.deep.begin(), plan.deep.end());
+    }
+    if (near > nodes_ * lv / 2) return false;
+    for (Solver *c : cases_)  // (allocated on the case's stream, used on this one)
+        if (!c->multi_buffers(lv) || !check_cuda(cudaStreamSynchronize(c->stream()), "multi_buffers")) return false;
+    const int nc = (int)cases_.size(), ne = max_stages_ ? stage_counts_[0] : 0;
+    if (!balloc(allocs_, &d_mdeep_, deep.size(), stream_) || !balloc(allocs_, &d_mtasks_, tasks.size(), stream_) ||
+        !balloc(allocs_, &d_msp_, (size_t)nc * (2 * lv + 2), stream_) || !balloc(allocs_, &d_mfin_, (size_t)nc * 2 * lv, stream_) ||
+        !balloc(allocs_, &d_mlist_, (size_t)std::max(ne, 1) * 2 * lv, stream_))
+        return false;
+    CK(cudaMemcpyAsync(d_mdeep_, deep.data(), deep.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, stream_));
+    CK(cudaMemcpyAsync(d_mtasks_, tasks.data(), tasks.size() * sizeof(MultiTask), cudaMemcpyHostToDevice, stream_));
+    ntasks_ = (int)tasks.size();
+    for (int q = 0; q < lv; q++) {
+        if (!balloc(allocs_, &d_msegs_[q], segs[q].size(), stream_)) return false;
+        CK(cudaMemcpyAsync(d_msegs_[q], segs[q].data(), segs[q].size() * sizeof(int4), cudaMemcpyHostToDevice, stream_));
+        nmsegs_[q] = (int)segs[q].size();
+    }
+    int lo = 0, hi = 0;
+    cudaDeviceGetStreamPriorityRange(&lo, &hi);
+    CK(cudaStreamCreateWithPriority(&multi_stream_, cudaStreamNonBlocking, lo));
+    CK(cudaEventCreateWithFlags(&multi_fork_, cudaEventDisableTiming));
+    CK(cudaEventCreateWithFlags(&multi_join_, cudaEventDisableTiming));
+    CK(cudaStreamSynchronize(stream_));
+    multi_state_ = 1;
+    return true;
+}
+
+// Parameters of two passes (cur -> other -> cur) from each case's state.
+bool Batch::upload_multi() {
+    const int lv = multi_lv_, nc = (int)cases_.size(), nsp = 2 * lv + 2;
+    h_msp_.assign((size_t)nc * nsp, FastStepParams());
+    h_mfin_.assign((size_t)nc * 2 * lv, FinishParams());
+    h_mlist_.clear();
+    for (int c = 0; c < nc; c++) {
+        Solver *s = cases_[c];
+        const int cur = s->current(), par = s->parity();
+        for (int a = 0; a < 2; a++) {
+            const int from = a ? 1 - cur : cur, to = 1 - from;
+            for (int q = 0; q < lv; q++) {
+                h_msp_[(size_t)c * nsp + a * lv + q] = s->fast_params(s->near_params(from, to, lv, q));
+                h_mfin_[(size_t)c * 2 * lv + a * lv + q] =
+                    s->finish_params(Solver::near_buffer(from, to, lv, q + 1), false, par ^ (q & 1));
+            }
+            h_msp_[(size_t)c * nsp + 2 * lv + a] = s->fast_params(s->step_params(from, to, false, par));
+        }
+        if (s->stage_groups().empty()) continue;
+        for (int k : s->stage_groups()[0])
+            for (int m = 0; m < 2 * lv; m++) {
+                StageParams p = s->stage_params(s->stages()[k], cur, par ^ (m & 1));
+                p.fin = d_mfin_ + (size_t)c * 2 * lv + m;
+                p.step = &d_msp_[(size_t)c * nsp + m].s;
+                h_mlist_.push_back(p);
+            }
+    }
+    CK(cudaMemcpyAsync(d_msp_, h_msp_.data(), h_msp_.size() * sizeof(FastStepParams), cudaMemcpyHostToDevice, stream_));
+    CK(cudaMemcpyAsync(d_mfin_, h_mfin_.data(), h_mfin_.size() * sizeof(FinishParams), cudaMemcpyHostToDevice, stream_));
+    if (!h_mlist_.empty())
+        CK(cudaMemcpyAsync(d_mlist_, h_mlist_.data(), h_mlist_.size() * sizeof(StageParams), cudaMemcpyHostToDevice, stream_));
+    return true;
+}
+
+// Pass a (0: cur -> other, 1: back).
+bool Batch::launch_multi(int a) {
+    const int lv = multi_lv_, nsp = 2 * lv + 2;
+    CK(cudaEventRecord(multi_fork_, stream_));
+    CK(cudaStreamWaitEvent(multi_stream_, multi_fork_, 0));
+    CK(launch::multi_batch(d_msp_, nsp, 2 * lv + a, d_mtasks_, ntasks_, d_mdeep_, store_, lv, any_force_, multi_stream_));
+    CK(cudaEventRecord(multi_join_, multi_stream_));
+    for (int q = 0; q < lv; q++) {
+        NearBatch b;
+        std::memset(&b, 0, sizeof b);
+        b.sp = d_msp_; b.nsp = nsp; b.sel = a * lv + q;
+        b.list = d_mlist_; b.nst = 2 * lv;
+        if (max_stages_) {
+            b.eblocks = d_stage_blocks_[0];
+            b.neb = stage_nblocks_[0] - nforce_;  // the force blocks come last
+        }
+        b.nodes = d_special_nf_; b.n = nspecial_nf_;
+        b.segs = d_msegs_[q]; b.nseg = nmsegs_[q];
+        CK(launch::near_batch_shifted(b, store_, any_links_, q > 0, stream_));
+    }
+    CK(cudaStreamWaitEvent(stream_, multi_join_, 0));
+    return true;
+}
+
+// As many of `pairs` step pairs as whole double passes take; -1 on an error.
+int Batch::run_multi(int pairs) {
+    const int lv = multi_lv_;
+    if (forces_ || pairs < 4 * lv || !multi_setup()) return 0;
+    if (!upload_multi()) return -1;
+    for (Solver *c : cases_)
+        if (!c->swap_multi(true, lv, stream_)) return -1;
+    if (!multi_exec_) {
+        cudaGraph_t g = nullptr;
+        if (!check_cuda(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal), "capture")) return -1;
+        const bool okk = launch_multi(0) && launch_multi(1);
+        cudaError_t e = cudaStreamEndCapture(stream_, &g);
+        if (okk && e == cudaSuccess) e = cudaGraphInstantiate(&multi_exec_, g, 0);
+        if (g) cudaGraphDestroy(g);
+        if (!okk || !check_cuda(e, "capture")) return -1;
+    }
+    int used = 0;
+    for (; pairs - used >= lv; used += lv)
+        if (!check_cuda(cudaGraphLaunch(multi_exec_, stream_), "graph")) return -1;
+    for (Solver *c : cases_)
+        if (!c->swap_multi(false, lv, stream_)) return -1;
+    return used;
+}
+
 bool Batch::run(int nsteps) {
     if (!ok_) return false;
     if (nsteps <= 0) return true;
@@ -2122,6 +2302,13 @@ bool Batch::run(int nsteps) {
             okk = used >= 0;
             pairs -= std::max(used, 0);
         }
+        if (okk) {
+            const int used = run_multi(pairs);
+            okk = used >= 0;
+            pairs -= std::max(used, 0);
+        }
+        // (params_ev_ again: the passes' parameter copies are waited for too)
+        if (okk) okk = check_cuda(cudaEventRecord(params_ev_, stream_), "event");
         if (okk && pairs >= kGraphPairs) okk = capture_pair();
         for (; okk && pairs >= kGraphPairs; pairs -= kGraphPairs) okk = check_cuda(cudaGraphLaunch(pair_exec_, stream_), "graph");
         for (; okk && pairs > 0; pairs--) okk = launch_batched(0) && launch_batched(1);

@@ -95,6 +95,16 @@ constexpr int kGraphPairs = 4;
 // Most probes a solver records (one block of a record launch walks them).
 constexpr int kMaxProbes = 4096;
 
+// A case's nodes near special ones in passes of several steps (near_plan).
+struct NearPlan {
+    std::vector<uint32_t> deep;
+    std::vector<std::vector<int4>> segs;
+    long long near_pairs = 0;
+};
+// Rows of a warp's task in a batch's pass (64 ducts: 126 us per step with 32, 122
+// with 64, 120.7 with 96 and 128).
+constexpr int kTaskRows = 96;
+
 // Zero-order-hold update of m v' + R v + K x = p over one lattice step:
 // (x, v) <- A (x, v) + b p. Returns false unless m > 0 and K > 0.
 bool msd_zoh(double R, double m, double K, double A[4], double b[2]);
@@ -230,6 +240,21 @@ class Solver {
     const std::vector<RecordTask> &record_tasks() const { return rec_host_; }
     bool begin_steps(cudaStream_t s);
     bool end_steps(cudaStream_t s);
+    // Passes of several steps, for a case alone and in a batch.
+    bool multi_case() const {
+        return d_.store != STORE_F64 && !d_omega_ && rec_host_.empty() && one_group_ && d_.Nx >= 8 && d_.Ny >= 8 &&
+               !wide() && (long long)special_host_.size() <= (long long)d_.Nx * d_.Ny / 8;
+    }
+    bool wide() const { return 9LL * plane_ >= (1LL << 31); }  // element offsets need 64 bits
+    size_t multi_bytes() const { return 9 * (size_t)plane_ * esize_; }  // of one of its buffers
+    void near_plan(int lv, NearPlan &plan) const;
+    bool multi_buffers(int lv);
+    bool swap_multi(bool enter, int lv, cudaStream_t s);
+    StepParams near_params(int cur, int other, int lv, int q) const;
+    // The buffer of the near nodes' state after q steps of a pass.
+    static int near_buffer(int cur, int other, int lv, int q) {
+        return q == 0 ? cur : q == lv ? other : (q & 1) ? 2 : 3;
+    }
     void advance(int nsteps);
     void add_steps(long long n) { steps_done_ += n; }
 
@@ -315,8 +340,8 @@ class Solver {
     bool graph_valid_multi_ = false;
     int multi_state_ = 0;                 // 0: not tried, 1: set up, -1: not for this case
     uint32_t *d_deep_ = nullptr;
-    int2 *d_multi_list_[4] = {nullptr, nullptr, nullptr, nullptr};
-    int multi_count_[4] = {0, 0, 0, 0};
+    int4 *d_near_segs_[4] = {nullptr, nullptr, nullptr, nullptr};
+    int near_segs_[4] = {0, 0, 0, 0};
     cudaStream_t multi_stream_ = nullptr;
     cudaEvent_t multi_fork_ = nullptr, multi_join_ = nullptr;
     size_t dev_bytes_ = 0;
@@ -391,6 +416,10 @@ class Batch {
     float tuned_us_ = 0.f;
     bool launch_batched(int sel);
     bool capture_pair();
+    bool multi_setup();
+    bool upload_multi();
+    bool launch_multi(int a);
+    int run_multi(int pairs);
 
     std::vector<Solver *> cases_;
     int store_ = STORE_F64, arith_ = ARITH_LBC;
@@ -423,6 +452,20 @@ class Batch {
     int nrec_ = 0;
     cudaGraphExec_t pair_exec_ = nullptr;
     std::vector<void *> allocs_;
+    // passes of several steps (multi_setup)
+    int multi_state_ = 0, multi_lv_ = 4, ntasks_ = 0, nmsegs_[4] = {0, 0, 0, 0};
+    uint32_t *d_mdeep_ = nullptr;
+    MultiTask *d_mtasks_ = nullptr;
+    FastStepParams *d_msp_ = nullptr;
+    FinishParams *d_mfin_ = nullptr;
+    StageParams *d_mlist_ = nullptr;
+    int4 *d_msegs_[4] = {nullptr, nullptr, nullptr, nullptr};
+    std::vector<FastStepParams> h_msp_;
+    std::vector<FinishParams> h_mfin_;
+    std::vector<StageParams> h_mlist_;
+    cudaGraphExec_t multi_exec_ = nullptr;
+    cudaStream_t multi_stream_ = nullptr;
+    cudaEvent_t multi_fork_ = nullptr, multi_join_ = nullptr;
     // host copies of the per-run parameters (kept until their uploads ran)
     std::vector<StepParams> h_sp_;
     std::vector<FastStepParams> h_fsp_;

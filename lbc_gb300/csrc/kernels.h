@@ -127,6 +127,27 @@ struct RecordTask {
 constexpr int kMultiThreads = 128;
 __host__ __device__ constexpr int multi_halo(int levels) { return (levels + 1) / 2 * 2; }
 
+// A warp's part of a batch's pass: rows [y0, y1) of a strip of case cs.
+struct MultiTask {
+    int cs, strip, y0, y1;
+    long long deep;       // the case's first word in `deep`
+};
+
+// One step of a batch's near nodes (launch::near_batch_shifted): parameter set
+// sel of nsp per case and of nst per Boundary entry.
+struct NearBatch {
+    const FastStepParams *sp;
+    int nsp, sel;
+    const StageParams *list;
+    int nst;
+    const int2 *eblocks;
+    int neb;
+    const int4 *nodes;    // (case, i, j, chunk), a multiple of 32 per case
+    int n;
+    const int4 *segs;     // (case, row, first column, mask)
+    int nseg;
+};
+
 namespace launch {
 // Records of one step: tasks[0 .. n). Alone: the step's populations are at
 // dst. In a batch (spbase set): case cs's are the dst of its step parameters
@@ -155,6 +176,10 @@ cudaError_t multi_plain(const FastStepParams &p, int store, int levels, int warp
 // nodes away from any special node: deep[strip * Ny + row], a bit per lane's
 // pair (strips of 64 - 2 multi_halo(levels) columns).
 cudaError_t multi_geo(const FastStepParams &p, int store, int levels, const uint32_t *deep, int warps, cudaStream_t s);
+// The same for every case of a batch: a warp per task, parameter set sel of nsp
+// per case; force: some case has a body force.
+cudaError_t multi_batch(const FastStepParams *sp, int nsp, int sel, const MultiTask *tasks, int ntasks,
+                        const uint32_t *deep, int store, int levels, bool force, cudaStream_t s);
 // Before a run of such passes and after it: the special nodes' populations of
 // odd steps move from `other` to `odd` and back; solid nodes of `other` (and of
 // `even2`, when there is one) take cur's, as the buffers change roles.
@@ -205,16 +230,18 @@ cudaError_t step_shifted(const FastStepParams &p, int store, bool flags, bool co
 // The special nodes of a case (nodes[0 .. n)) on the per-node path; flags: the
 // case has a flag word. after_bulk: the programmatic follower of the kernel
 // before it (a case alone launches it first, without the attribute, and the
-// clean pairs as its follower: step_shifted's after). The first nforce entries
-// (a multiple of 32, or all) sum their wall-link force by chunks.
-cudaError_t special_shifted(const FastStepParams &p, const int2 *nodes, int n, int nforce, int store, bool flags, bool collide,
+// clean pairs as its follower: step_shifted's after).
+cudaError_t special_shifted(const FastStepParams &p, const int2 *nodes, int n, int store, bool flags, bool collide,
                             bool after_bulk, cudaStream_t s);
-// A step's special nodes (or a longer list of nodes, as special_shifted) and its
-// Boundary list, when that is one group without periodic entries, in one
-// launch; collides. g.nfs is not looked at (the force is reduced on its own).
-// after: the programmatic follower of the same launch of the step before.
-cudaError_t near_shifted(const FastStepParams &p, const int2 *nodes, int n, int nforce, int store, const StageGroup &g,
-                         bool after, cudaStream_t s);
+// A step's special nodes, the clean pairs of segs (x unused, row, first column, a
+// bit per pair of 64 columns) and its Boundary list, when that is one group
+// without periodic entries, in one launch; collides. g.nfs is not looked at
+// (the force is reduced on its own). after: the programmatic follower of the
+// same launch of the step before. The nine planes hold less than 2^31 elements.
+cudaError_t near_shifted(const FastStepParams &p, const int2 *nodes, int n, const int4 *segs, int nseg, int store,
+                         const StageGroup &g, bool after, cudaStream_t s);
+// The same for a batch.
+cudaError_t near_batch_shifted(const NearBatch &b, int store, bool links, bool after, cudaStream_t s);
 // The special nodes of a batch: nodes[q] = (case, i, j, chunk), n a multiple
 // of 32 (each case's list padded to 32 entries, i = -1); links: some case has
 // cut-link records.

@@ -219,6 +219,22 @@ __global__ void __launch_bounds__(kMultiThreads) k_multi_geo(const FastStepParam
     else walk_strip<T, LV, FORCE, true, true>(fp, deep, cb, keep0, keep1, y0, y1);
 }
 
+// Every case of a batch: a warp per task.
+template <typename T, int LV, bool FORCE>
+__global__ void __launch_bounds__(kMultiThreads) k_multi_batch(const FastStepParams *__restrict__ sp, int nsp, int sel,
+                                                               const MultiTask *__restrict__ tasks, int ntasks,
+                                                               const uint32_t *__restrict__ deep) {
+    const int w = (int)(blockIdx.x * (kMultiThreads / 32) + threadIdx.x / 32);
+    if (w >= ntasks) return;
+    const MultiTask t = tasks[w];
+    const FastStepParams &fp = sp[nsp * t.cs + sel];
+    const int halo = multi_halo(LV), width = 64 - 2 * halo;
+    const int keep0 = t.strip * width, keep1 = min(keep0 + width, fp.s.Nx), cb = keep0 - halo;
+    const uint32_t *d = deep + t.deep + (size_t)t.strip * (size_t)fp.s.Ny;
+    if (cb >= 0 && cb + 64 <= fp.s.Nx) walk_strip<T, LV, FORCE, false, true>(fp, d, cb, keep0, keep1, t.y0, t.y1);
+    else walk_strip<T, LV, FORCE, true, true>(fp, d, cb, keep0, keep1, t.y0, t.y1);
+}
+
 // One thread per special node (launch::multi_swap).
 template <typename T>
 __global__ void k_multi_swap(const int2 *__restrict__ nodes, int n, const uint16_t *__restrict__ flags, int pitch,
@@ -264,6 +280,27 @@ cudaError_t multi_geo(const FastStepParams &p, int store, int levels, const uint
     } else {
         if (levels == 2) return multi_geo_tl<__half, 2>(p, deep, warps, s);
         if (levels == 4) return multi_geo_tl<__half, 4>(p, deep, warps, s);
+    }
+    return cudaErrorInvalidValue;
+}
+
+template <typename T, int LV>
+static cudaError_t multi_batch_tl(const FastStepParams *sp, int nsp, int sel, const MultiTask *tasks, int ntasks,
+                                  const uint32_t *deep, bool force, cudaStream_t s) {
+    const unsigned blocks = (unsigned)((ntasks + kMultiThreads / 32 - 1) / (kMultiThreads / 32));
+    if (force) k_multi_batch<T, LV, true><<<blocks, kMultiThreads, 0, s>>>(sp, nsp, sel, tasks, ntasks, deep);
+    else k_multi_batch<T, LV, false><<<blocks, kMultiThreads, 0, s>>>(sp, nsp, sel, tasks, ntasks, deep);
+    return cudaGetLastError();
+}
+
+cudaError_t multi_batch(const FastStepParams *sp, int nsp, int sel, const MultiTask *tasks, int ntasks,
+                        const uint32_t *deep, int store, int levels, bool force, cudaStream_t s) {
+    if (store == STORE_F32) {
+        if (levels == 2) return multi_batch_tl<float, 2>(sp, nsp, sel, tasks, ntasks, deep, force, s);
+        if (levels == 4) return multi_batch_tl<float, 4>(sp, nsp, sel, tasks, ntasks, deep, force, s);
+    } else {
+        if (levels == 2) return multi_batch_tl<__half, 2>(sp, nsp, sel, tasks, ntasks, deep, force, s);
+        if (levels == 4) return multi_batch_tl<__half, 4>(sp, nsp, sel, tasks, ntasks, deep, force, s);
     }
     return cudaErrorInvalidValue;
 }

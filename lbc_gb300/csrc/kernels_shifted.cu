@@ -14,244 +14,9 @@
 #include "lbm_device.cuh"
 #include "pdl.cuh"
 #include "reduce.cuh"
-#include "shifted_math.cuh"
+#include "shifted_node.cuh"
 
 namespace lbm {
-
-// Scalar entry points used by the per-node paths.
-__device__ __forceinline__ void moments_shifted(const float g[9], float hFx, float hFy, float &dr,
-                                                float &rho, float &ux, float &uy, float &Jx,
-                                                float &Jy, float &jx, float &jy) {
-    moments_v<float>(g, hFx, hFy, dr, rho, ux, uy, Jx, Jy, jx, jy);
-}
-
-// Rare per-node outputs, kept out of line so the compiler cannot hoist their
-// FP64 conversions into every thread's path (FP64 issue is slow on GB300).
-template <typename T>
-__device__ __noinline__ void solid_node_outputs(const StepParams &p, int slot, long long node, size_t dn,
-                                                uint16_t fl) {
-    if (p.write_macro) { p.rho[dn] = NAN; p.ux[dn] = NAN; p.uy[dn] = NAN; }
-    if (fl & NF_BAND) {
-        // A BC may read a solid neighbour: lbc sees the untouched buffer
-        // content and NaN moments there.
-        const T *Old = (const T *)p.stale;
-#pragma unroll
-        for (int k = 0; k < 9; k++) p.bandg[(size_t)k * p.nslots + slot] = SV<T>::ld_plain(Old + k * p.plane + node);
-        p.bandm_next[slot] = NAN;
-        p.bandm_next[(size_t)p.nslots + slot] = NAN;
-        p.bandm_next[2 * (size_t)p.nslots + slot] = NAN;
-    }
-}
-
-
-// A solid node off the edge band (kSpecialSolid entries): NaN moments on steps
-// that write the fields, as solid_node_outputs writes them.
-__device__ __forceinline__ void solid_nan(const StepParams &p, int i, int j) {
-    if (!p.write_macro) return;
-    const size_t dn = (size_t)j * (size_t)p.Nx + (size_t)i;
-    p.rho[dn] = NAN;
-    p.ux[dn] = NAN;
-    p.uy[dn] = NAN;
-}
-
-__device__ __noinline__ void macro_store(const StepParams &p, size_t dn, int slot, float dr, float ux,
-                                         float uy) {
-    if (p.write_macro) { p.rho[dn] = 1.0 + (double)dr; p.ux[dn] = ux; p.uy[dn] = uy; }
-    if (slot >= 0) {
-        p.bandm_next[slot] = 1.0 + (double)dr;
-        p.bandm_next[(size_t)p.nslots + slot] = ux;
-        p.bandm_next[2 * (size_t)p.nslots + slot] = uy;
-    }
-}
-
-__device__ __noinline__ void macro_store_pair(const StepParams &p, size_t dn, float2 dr, float2 ux, float2 uy) {
-    p.rho[dn] = 1.0 + (double)dr.x;
-    p.rho[dn + 1] = 1.0 + (double)dr.y;
-    p.ux[dn] = ux.x;
-    p.ux[dn + 1] = ux.y;
-    p.uy[dn] = uy.x;
-    p.uy[dn + 1] = uy.y;
-}
-
-__device__ __noinline__ float2 omega_pair(const double *omega, size_t dn) {
-    return make_float2((float)omega[dn], (float)omega[dn + 1]);
-}
-
-// One node of the fused step in shifted storage (solids, bounce-back links,
-// stale slots, edge-BC band: everything). I is the element-offset type: int
-// whenever all nine planes fit in 2^31 elements (fewer address instructions),
-// long long otherwise. LINKS = false: no case of the launch has cut-link
-// records (plain bounce-back on every solid link), and the record path is
-// left out (measured: 116 -> 64 registers for the batched special-node
-// kernel, twice the resident warps).
-template <typename T, typename I, bool FLAGS, bool COLLIDE, bool FORCE, bool LINKS = true>
-__device__ __forceinline__ void step_node_shifted(const FastStepParams &fp, int i, int j,
-                                                  float &mfx, float &mfy, bool &link) {
-    const StepParams &p = fp.s;
-    const I node = (I)j * (I)p.pitch + (I)i;
-    const size_t dn = (size_t)j * (size_t)p.Nx + (size_t)i;
-    const T *S = (const T *)p.src;
-    T *Dst = (T *)p.dst;
-    const T *Old = (const T *)p.stale;
-    const I pl = (I)p.plane;
-    // The loads come in three waves of independent loads, not one chain: (1)
-    // the flag word, the nine pulled populations, the node's eight own
-    // opposite populations, its cut-link offset, its band bases and (without
-    // cut-link records) the stale slots of off-grid sources, which the
-    // position alone decides; (2) the cut-link records of its flagged
-    // directions; (3) the populations behind interpolated links (and the
-    // stale slots, with records). Source neighbours are wrapped on periodic axes and
-    // clamped otherwise, so that every load of wave 1 is in bounds whatever
-    // the flags say. (Measured: the own populations loaded in wave 2, for
-    // flagged directions only, cost the channel and the cylinder 2-4 %.)
-    int im = i - 1, ip = i + 1, jm = j - 1, jp = j + 1;
-    if (p.px) { if (im < 0) im += p.Nx; if (ip >= p.Nx) ip -= p.Nx; }
-    else { im = max(im, 0); ip = min(ip, p.Nx - 1); }
-    if (p.py) { if (jm < 0) jm += p.Ny; if (jp >= p.Ny) jp -= p.Ny; }
-    else { jm = max(jm, 0); jp = min(jp, p.Ny - 1); }
-    const I r0 = (I)j * (I)p.pitch, rm = (I)jm * (I)p.pitch, rp = (I)jp * (I)p.pitch;
-    const I so[9] = {r0 + i, r0 + im, rm + i, r0 + ip, rp + i, rm + im, rm + ip, rp + ip, rp + im};
-    const uint16_t fl = FLAGS ? p.flags[node] : (uint16_t)0;
-    float g[9];
-#pragma unroll
-    for (int k = 0; k < 9; k++) g[k] = SV<T>::ld(S + (I)k * pl + so[k]);
-    int lo = 0, cb = -1, rb = -1;
-    float own[9];
-    bool off[9];
-    if (FLAGS) {
-#pragma unroll
-        for (int k = 1; k < 9; k++) own[k] = SV<T>::ld(S + (I)oppk(k) * pl + node);
-        if (LINKS && p.link_off) lo = p.link_off[node];
-        // Without cut-link records, also the band bases and the stale slots
-        // of off-grid sources (this node's own destination slots, written by
-        // no other thread). With records they stay in the later waves: their
-        // registers (96 -> 116 for the per-case kernel) cost more than the
-        // latency saved.
-        if (!LINKS && p.colbase) { cb = p.colbase[i]; rb = p.rowbase[j]; }
-        if (!LINKS) {
-#pragma unroll
-            for (int k = 1; k < 9; k++) {
-                const int si = i - cxk(k), sj = j - cyk(k);
-                off[k] = (!p.px && (si < 0 || si >= p.Nx)) || (!p.py && (sj < 0 || sj >= p.Ny));
-                if (off[k]) g[k] = SV<T>::ld_plain(Old + (I)k * pl + node);
-            }
-        }
-    }
-    int slot = -1;
-    if (FLAGS && (fl & NF_BAND)) slot = LINKS ? band_slot(p.colbase, p.rowbase, i, j) : (cb >= 0 ? cb + j : rb + i);
-    if (FLAGS && (fl & NF_SOLID)) {
-        solid_node_outputs<T>(p, slot, (long long)node, dn, fl);
-        return;
-    }
-    if (FLAGS && (fl & NF_SPECIAL_MASK)) {
-        const bool has_links = LINKS && (fl & NF_LINKS) != 0;
-        Link L[9];
-        int m = 0;
-#pragma unroll
-        for (int k = 1; k < 9; k++) {
-            if (LINKS) {
-                const int si = i - cxk(k), sj = j - cyk(k);
-                off[k] = (!p.px && (si < 0 || si >= p.Nx)) || (!p.py && (sj < 0 || sj >= p.Ny));
-            }
-            // link records in direction order, one per flagged on-grid direction
-            if ((fl & (1u << k)) && !off[k] && has_links) L[k] = p.links[lo + m++];
-        }
-        float behind[9];
-#pragma unroll
-        for (int k = 1; k < 9; k++) {
-            behind[k] = 0.f;
-            if (!(fl & (1u << k))) continue;
-            if (off[k]) {
-                if (LINKS) g[k] = SV<T>::ld_plain(Old + (I)k * pl + node);
-            } else if (has_links) {
-                if (L[k].mode == LINK_IBB_LO) behind[k] = SV<T>::ld(S + (I)oppk(k) * pl + (I)L[k].behind);
-                else if (L[k].mode == LINK_IBB_HI) behind[k] = SV<T>::ld(S + (I)k * pl + (I)L[k].behind);
-            }
-        }
-#pragma unroll
-        for (int k = 1; k < 9; k++) {
-            if (!(fl & (1u << k)) || off[k]) continue;
-            float val = own[k];
-            if (has_links) {
-                if (L[k].mode == LINK_IBB_LO || L[k].mode == LINK_IBB_HI)
-                    val = (float)L[k].c1 * own[k] + (float)L[k].c2 * behind[k];
-                else if (L[k].mode == LINK_MOVING)
-                    val = own[k] - (float)L[k].c2;
-            }
-            g[k] = SV<T>::rnd(val);
-            // Per-node link sum in FP32 (a few terms); chunk and case sums are FP64.
-            const float df = (own[k] + val) + 2.0f * fp.wf[k];
-            mfx -= df * cxk(k);
-            mfy -= df * cyk(k);
-            link = true;
-        }
-    }
-    if (FLAGS && (fl & NF_BAND)) {
-#pragma unroll
-        for (int k = 0; k < 9; k++) p.bandg[(size_t)k * p.nslots + slot] = g[k];
-    }
-    if (FLAGS && (fl & NF_BCW)) return;
-    float dr, rho, ux, uy, Jx, Jy, jx, jy;
-    moments_v<float>(g, fp.hFxf, fp.hFyf, dr, rho, ux, uy, Jx, Jy, jx, jy);
-    if (p.write_macro || slot >= 0) macro_store(p, dn, slot, dr, ux, uy);
-    if (COLLIDE) {
-        const float om = p.omega ? (float)p.omega[dn] : fp.omega0f;
-        collide_v<float, FORCE>(g, fp.wf, fp.h1f, fp.h5f, dr, ux, uy, Jx, Jy, jx, jy, om, p.has_force != 0,
-                                fp.Fxf, fp.Fyf);
-    }
-#pragma unroll
-    for (int k = 0; k < 9; k++) SV<T>::st(Dst + (I)k * pl + node, g[k]);
-}
-
-// Two adjacent nodes (i0, i0 + 1) of one row, neither of them special (no
-// solid, link, stale slot, band or BC node): pair loads where the pull sources
-// are adjacent (c_x = 0), a pair and a single load otherwise (c_x = +-1), packed
-// FP32 arithmetic, pair stores. im = source column of i0 - 1, ip2 of i0 + 2
-// (wrapped or clamped like the per-node path), so every load is in bounds
-// whatever the nodes' flags say.
-template <typename T, typename I>
-__device__ __forceinline__ void load_pair_shifted(const StepParams &p, int i0, int j, int im, int ip2, int jm,
-                                                  int jp, float2 g[9]) {
-    const T *S = (const T *)p.src;
-    const I pl = (I)p.plane;
-    const I r0 = (I)j * (I)p.pitch + (I)i0, rm = (I)jm * (I)p.pitch, rp = (I)jp * (I)p.pitch;
-    const I m0 = rm + (I)i0, p0 = rp + (I)i0;
-    float2 a;
-    g[0] = SV<T>::ld2(S + r0);
-    a = SV<T>::ld2(S + pl + r0);
-    g[1] = make_float2(SV<T>::ld(S + pl + (r0 - (I)i0 + (I)im)), a.x);
-    g[2] = SV<T>::ld2(S + 2 * pl + m0);
-    a = SV<T>::ld2(S + 3 * pl + r0);
-    g[3] = make_float2(a.y, SV<T>::ld(S + 3 * pl + (r0 - (I)i0 + (I)ip2)));
-    g[4] = SV<T>::ld2(S + 4 * pl + p0);
-    a = SV<T>::ld2(S + 5 * pl + m0);
-    g[5] = make_float2(SV<T>::ld(S + 5 * pl + rm + (I)im), a.x);
-    a = SV<T>::ld2(S + 6 * pl + m0);
-    g[6] = make_float2(a.y, SV<T>::ld(S + 6 * pl + rm + (I)ip2));
-    a = SV<T>::ld2(S + 7 * pl + p0);
-    g[7] = make_float2(a.y, SV<T>::ld(S + 7 * pl + rp + (I)ip2));
-    a = SV<T>::ld2(S + 8 * pl + p0);
-    g[8] = make_float2(SV<T>::ld(S + 8 * pl + rp + (I)im), a.x);
-}
-
-template <typename T, typename I, bool COLLIDE, bool FORCE>
-__device__ __forceinline__ void collide_store_pair_shifted(const FastStepParams &fp, int i0, int j, float2 g[9]) {
-    const StepParams &p = fp.s;
-    T *Dst = (T *)p.dst;
-    const I pl = (I)p.plane;
-    const I r0 = (I)j * (I)p.pitch + (I)i0;
-    float2 dr, rho, ux, uy, Jx, Jy, jx, jy;
-    moments_v<float2>(g, v_splat<float2>(fp.hFxf), v_splat<float2>(fp.hFyf), dr, rho, ux, uy, Jx, Jy, jx, jy);
-    const size_t dn = (size_t)j * (size_t)p.Nx + (size_t)i0;
-    if (p.write_macro) macro_store_pair(p, dn, dr, ux, uy);
-    if (COLLIDE) {
-        const float2 om = p.omega ? omega_pair(p.omega, dn) : v_splat<float2>(fp.omega0f);
-        collide_v<float2, FORCE>(g, fp.wf, fp.h1f, fp.h5f, dr, ux, uy, Jx, Jy, jx, jy, om, p.has_force != 0,
-                                 fp.Fxf, fp.Fyf);
-    }
-#pragma unroll
-    for (int k = 0; k < 9; k++) SV<T>::st2(Dst + (I)k * pl + r0, g[k]);
-}
 
 // Flag bits that take a node off the pair path: a solid or off-grid pull
 // source, solid, edge-BC band or BC-written, cut links.
@@ -319,8 +84,7 @@ __global__ void __launch_bounds__(256, 5) k_step_shifted_geo(const FastStepParam
     if (i0 < fp.s.Nx && j < fp.s.Ny) step_pair_clean<T, I, true, COLLIDE, FORCE>(fp, i0, j);
 }
 
-// The special nodes of a case (and, in passes of several steps, the nodes near
-// them), one per thread, on the per-node path (same
+// The special nodes of a case, one per thread, on the per-node path (same
 // arithmetic as the pair path, so a node's bits do not depend on which path
 // steps it). Wall-link force terms are summed per 32-entry chunk of the list.
 // It reads and writes nothing the clean-pair kernel touches: a case alone
@@ -331,19 +95,17 @@ __global__ void __launch_bounds__(256, 5) k_step_shifted_geo(const FastStepParam
 // no-op.)
 template <typename T, typename I, bool FLAGS, bool COLLIDE, bool FORCE, bool LINKS>
 __global__ void __launch_bounds__(128) k_step_special_shifted(const FastStepParams fp,
-                                                              const int2 *__restrict__ nodes, int n, int nforce) {
+                                                              const int2 *__restrict__ nodes, int n) {
     pdl_launch_dependents();
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
     float mx = 0.f, my = 0.f;
     bool link = false;
     if (q < n) {
         const int2 ij = nodes[q];
-        if (ij.x < 0) {  // padding
-        } else if (ij.x & kSpecialSolid) solid_nan(fp.s, ij.x & ~kSpecialSolid, ij.y);
+        if (ij.x & kSpecialSolid) solid_nan(fp.s, ij.x & ~kSpecialSolid, ij.y);
         else step_node_shifted<T, I, FLAGS, COLLIDE, FORCE, LINKS>(fp, ij.x, ij.y, mx, my, link);
     }
-    // (the first nforce entries are the special nodes, whose chunks have slots)
-    if (fp.s.mem_partials && (q & ~31) < nforce)
+    if (fp.s.mem_partials)
         chunk_reduce2_store((double)mx, (double)my, link, q >> 5, fp.s.chunk_slot, fp.s.mem_partials);
     pdl_wait();
 }
@@ -403,38 +165,8 @@ __global__ void __launch_bounds__(128) k_step_batch_special_shifted(const FastSt
     pdl_wait();
 }
 
-// Moments and collision of a node that an edge BC wrote: pre-collision
-// populations f (rounded to the storage type here).
-template <typename T, bool COLLIDE>
-__device__ __forceinline__ void finish_pops_shifted(const FinishParams &p, int2 ij, int slot, const float f[9]) {
-    float g[9], wf[9];
-#pragma unroll
-    for (int k = 0; k < 9; k++) {
-        g[k] = SV<T>::rnd(f[k]);
-        wf[k] = p.wf[k];
-    }
-    float dr, rho, ux, uy, Jx, Jy, jx, jy;
-    moments_shifted(g, p.hFxf, p.hFyf, dr, rho, ux, uy, Jx, Jy, jx, jy);
-    const size_t dn = (size_t)ij.y * p.Nx + ij.x;
-    if (p.write_macro) { p.rho[dn] = 1.0 + (double)dr; p.ux[dn] = ux; p.uy[dn] = uy; }
-    p.bandm_next[slot] = 1.0 + (double)dr;
-    p.bandm_next[(size_t)p.nslots + slot] = ux;
-    p.bandm_next[2 * (size_t)p.nslots + slot] = uy;
-    if (COLLIDE) {
-        const float om = p.omega ? (float)p.omega[dn] : p.omega0f;
-        float h1, h5;
-        shifted_h(wf[1], h1, h5);
-        if (p.has_force) collide_v<float, true>(g, wf, h1, h5, dr, ux, uy, Jx, Jy, jx, jy, om, true, p.Fxf, p.Fyf);
-        else collide_v<float, false>(g, wf, h1, h5, dr, ux, uy, Jx, Jy, jx, jy, om, false, 0.f, 0.f);
-    }
-    T *D = (T *)p.dst;
-    const long long node = (long long)ij.y * p.pitch + ij.x;
-#pragma unroll
-    for (int k = 0; k < 9; k++) SV<T>::st(D + k * p.plane + node, g[k]);
-}
-
-// The same from the band, read at L2 (__ldcg), never from a possibly stale L1
-// line.
+// finish_pops_shifted from the band, read at L2 (__ldcg), never from a possibly
+// stale L1 line.
 template <typename T, bool COLLIDE>
 __device__ __forceinline__ void finish_node_shifted(const FinishParams &p, int2 ij, int slot) {
     float f[9];
@@ -559,136 +291,6 @@ __device__ __forceinline__ void stage_dispatch_s(const StageParams &p, const Fin
     }
 }
 
-// ---- a step's special nodes and its edges in one launch
-//
-// When the whole Boundary list is one group (no entry reads or writes a node
-// that another writes), an entry's thread need not wait for the band: it pulls
-// the node that its BC reads itself (its own for Zou-He, the interior
-// neighbour's for the others), and edges run beside the special nodes. That
-// takes the edge launch, and what it waits for, off every step: cylinder
-// 2048 x 512 16.5 -> 11.9 us, 256 x 64 12.4 -> 8.3, liner duct 1500 x 200 13.4 ->
-// 7.3.
-
-// The pre-collision populations of one node: what step_node_shifted leaves in
-// the band for it.
-template <typename T, typename I, bool LINKS>
-__device__ __forceinline__ void pull_node(const StepParams &p, int i, int j, float g[9]) {
-    const T *S = (const T *)p.src, *Old = (const T *)p.stale;
-    const I pl = (I)p.plane, node = (I)j * (I)p.pitch + (I)i;
-    int im = i - 1, ip = i + 1, jm = j - 1, jp = j + 1;
-    if (p.px) { if (im < 0) im += p.Nx; if (ip >= p.Nx) ip -= p.Nx; }
-    else { im = max(im, 0); ip = min(ip, p.Nx - 1); }
-    if (p.py) { if (jm < 0) jm += p.Ny; if (jp >= p.Ny) jp -= p.Ny; }
-    else { jm = max(jm, 0); jp = min(jp, p.Ny - 1); }
-    const I r0 = (I)j * (I)p.pitch, rm = (I)jm * (I)p.pitch, rp = (I)jp * (I)p.pitch;
-    const I so[9] = {r0 + i, r0 + im, rm + i, r0 + ip, rp + i, rm + im, rm + ip, rp + ip, rp + im};
-    const uint16_t fl = p.flags[node];
-#pragma unroll
-    for (int k = 0; k < 9; k++) g[k] = SV<T>::ld(S + (I)k * pl + so[k]);
-    if (!(fl & (NF_SPECIAL_MASK | NF_SOLID))) return;
-    if (fl & NF_SOLID) {
-#pragma unroll
-        for (int k = 0; k < 9; k++) g[k] = SV<T>::ld_plain(Old + (I)k * pl + node);
-        return;
-    }
-    const Link *lk = LINKS && (fl & NF_LINKS) ? p.links + p.link_off[node] : nullptr;
-#pragma unroll
-    for (int k = 1; k < 9; k++) {
-        if (!(fl & (1u << k))) continue;
-        const int si = i - cxk(k), sj = j - cyk(k);
-        if ((!p.px && (si < 0 || si >= p.Nx)) || (!p.py && (sj < 0 || sj >= p.Ny))) {
-            g[k] = SV<T>::ld_plain(Old + (I)k * pl + node);
-            continue;
-        }
-        const float own = SV<T>::ld(S + (I)oppk(k) * pl + node);
-        float val = own;
-        if (lk) {
-            const Link L = *lk++;
-            if (L.mode == LINK_IBB_LO) val = (float)L.c1 * own + (float)L.c2 * SV<T>::ld(S + (I)oppk(k) * pl + (I)L.behind);
-            else if (L.mode == LINK_IBB_HI) val = (float)L.c1 * own + (float)L.c2 * SV<T>::ld(S + (I)k * pl + (I)L.behind);
-            else if (L.mode == LINK_MOVING) val = own - (float)L.c2;
-        }
-        g[k] = SV<T>::rnd(val);
-    }
-}
-
-struct EdgeAccessor {
-    const StagePre &c;
-    const float *g;   // the node that the entry reads
-    float *out;       // the node that it writes
-    __device__ float get(int, int, int k) const { return g[k]; }
-    __device__ void set(int, int, int k, float v) const { out[k] = v; }
-    __device__ float drho(int, int) const { return (float)(c.nrho - 1.0); }
-    __device__ float ux(int, int) const { return (float)c.nux; }
-    __device__ float uy(int, int) const { return (float)c.nuy; }
-    __device__ float post(int, int, int) const { return 0.f; }  // periodic entries: not here
-    __device__ bool solid(int, int) const { return c.solid; }
-};
-
-template <typename T, typename I, bool LINKS, int KIND>
-__device__ __forceinline__ void edge_thread(const StepParams &sp, const StageParams &p, const FinishParams &f, int t) {
-    const StagePre c = stage_preload<true>(p, t, KIND);
-    if (c.solid) return;
-    float g[9], out[9], w[9];
-    const int2 at = edge_reads_neighbour(KIND) ? c.nij : c.ij;
-    pull_node<T, I, LINKS>(sp, at.x, at.y, g);
-#pragma unroll
-    for (int k = 0; k < 9; k++) {
-        out[k] = g[k];
-        w[k] = p.wf[k];
-    }
-    EdgeAccessor a{c, g, out};
-    if (KIND == BC_VEL_BOT_REG && c.imp)
-        bc_regularized_s(a, w, t, p.index, t, p.index + 1, false, (float)c.v1, (float)c.v2);
-    else
-        bc_apply_s(a, w, KIND, p.Nx, p.Ny, p.index, t, c.v1, c.v2);
-    finish_pops_shifted<T, true>(f, c.ij, c.slot, out);
-}
-
-template <typename T, typename I, bool LINKS>
-__device__ __forceinline__ void edge_dispatch(const StepParams &sp, const StageParams &p, const FinishParams &f, int t) {
-    switch (p.kind) {
-#define LBM_EDGE_KIND(K) \
-    case K: edge_thread<T, I, LINKS, K>(sp, p, f, t); break;
-    LBM_EDGE_KIND(BC_VEL_IN_ZH) LBM_EDGE_KIND(BC_VEL_OUT_ZH) LBM_EDGE_KIND(BC_VEL_TOP_ZH)
-    LBM_EDGE_KIND(BC_VEL_BOT_ZH) LBM_EDGE_KIND(BC_PRES_IN_ZH) LBM_EDGE_KIND(BC_PRES_OUT_ZH)
-    LBM_EDGE_KIND(BC_CONV_IN) LBM_EDGE_KIND(BC_CONV_OUT)
-    LBM_EDGE_KIND(BC_VEL_IN_REG) LBM_EDGE_KIND(BC_VEL_OUT_REG)
-    LBM_EDGE_KIND(BC_VEL_TOP_REG) LBM_EDGE_KIND(BC_VEL_BOT_REG) LBM_EDGE_KIND(BC_PRES_IN_REG)
-    LBM_EDGE_KIND(BC_PRES_OUT_REG) LBM_EDGE_KIND(BC_PRES_TOP_REG) LBM_EDGE_KIND(BC_PRES_BOT_REG)
-    LBM_EDGE_KIND(BC_VEL_BOT_ZH_FIX)
-#undef LBM_EDGE_KIND
-    default: break;
-    }
-}
-
-// Blocks [0, g.n * per): `per` blocks of each Boundary entry; then the node
-// list, as k_step_special_shifted. The wait at the start lets it follow the
-// same kernel of the step before.
-template <typename T, typename I, bool FORCE, bool LINKS>
-__global__ void __launch_bounds__(128) k_near_shifted(const FastStepParams fp, const int2 *__restrict__ nodes, int n,
-                                                      int nforce, int per, const StageGroup g) {
-    pdl_launch_dependents();
-    pdl_wait();
-    const int eb = g.n * per;
-    if ((int)blockIdx.x < eb) {
-        const StageParams &p = g.p[blockIdx.x / per];
-        const int t = (int)(blockIdx.x % per) * 128 + (int)threadIdx.x;
-        if (t < p.along) edge_dispatch<T, I, LINKS>(fp.s, p, g.fin, t);
-        return;
-    }
-    const int q = ((int)blockIdx.x - eb) * 128 + (int)threadIdx.x;
-    float mx = 0.f, my = 0.f;
-    bool link = false;
-    if (q < n) {
-        const int2 ij = nodes[q];
-        if (ij.x >= 0 && !(ij.x & kSpecialSolid))
-            step_node_shifted<T, I, true, true, FORCE, LINKS>(fp, ij.x, ij.y, mx, my, link);
-    }
-    if (fp.s.mem_partials && (q & ~31) < nforce)
-        chunk_reduce2_store((double)mx, (double)my, link, q >> 5, fp.s.chunk_slot, fp.s.mem_partials);
-}
-
 // As k_stage_group / k_stage_batch in kernels_exact.cu.
 template <typename T, bool COLLIDE>
 __global__ void k_stage_group_shifted(const StageGroup g) {
@@ -789,74 +391,46 @@ cudaError_t step_shifted(const FastStepParams &p, int store, bool flags, bool co
 }
 
 template <typename T, typename I, bool FORCE, bool LINKS>
-static cudaError_t special_shifted_tifl(const FastStepParams &p, const int2 *nodes, int n, int nforce, bool flags, bool collide,
+static cudaError_t special_shifted_tifl(const FastStepParams &p, const int2 *nodes, int n, bool flags, bool collide,
                                         bool after_bulk, cudaStream_t s) {
     const dim3 g((n + 127) / 128), b(128);
     if (flags) {
         if (collide)
             return launch_follower(after_bulk, k_step_special_shifted<T, I, true, true, FORCE, LINKS>, g, b, s, p,
-                                   nodes, n, nforce);
+                                   nodes, n);
         return launch_follower(after_bulk, k_step_special_shifted<T, I, true, false, FORCE, LINKS>, g, b, s, p, nodes,
-                               n, nforce);
+                               n);
     }
     if (collide)
         return launch_follower(after_bulk, k_step_special_shifted<T, I, false, true, FORCE, LINKS>, g, b, s, p, nodes,
-                               n, nforce);
-    return launch_follower(after_bulk, k_step_special_shifted<T, I, false, false, FORCE, LINKS>, g, b, s, p, nodes, n, nforce);
+                               n);
+    return launch_follower(after_bulk, k_step_special_shifted<T, I, false, false, FORCE, LINKS>, g, b, s, p, nodes, n);
 }
 
 template <typename T, typename I, bool FORCE>
-static cudaError_t special_shifted_tif(const FastStepParams &p, const int2 *nodes, int n, int nforce, bool flags, bool collide,
+static cudaError_t special_shifted_tif(const FastStepParams &p, const int2 *nodes, int n, bool flags, bool collide,
                                        bool after_bulk, cudaStream_t s) {
-    if (p.s.links) return special_shifted_tifl<T, I, FORCE, true>(p, nodes, n, nforce, flags, collide, after_bulk, s);
-    return special_shifted_tifl<T, I, FORCE, false>(p, nodes, n, nforce, flags, collide, after_bulk, s);
+    if (p.s.links) return special_shifted_tifl<T, I, FORCE, true>(p, nodes, n, flags, collide, after_bulk, s);
+    return special_shifted_tifl<T, I, FORCE, false>(p, nodes, n, flags, collide, after_bulk, s);
 }
 
 template <typename T>
-static cudaError_t special_shifted_t(const FastStepParams &p, const int2 *nodes, int n, int nforce, bool flags, bool collide,
+static cudaError_t special_shifted_t(const FastStepParams &p, const int2 *nodes, int n, bool flags, bool collide,
                                      bool after_bulk, cudaStream_t s) {
     const bool wide = 9LL * p.s.plane >= (1LL << 31);
     if (p.s.has_force) {
-        if (wide) return special_shifted_tif<T, long long, true>(p, nodes, n, nforce, flags, collide, after_bulk, s);
-        return special_shifted_tif<T, int, true>(p, nodes, n, nforce, flags, collide, after_bulk, s);
+        if (wide) return special_shifted_tif<T, long long, true>(p, nodes, n, flags, collide, after_bulk, s);
+        return special_shifted_tif<T, int, true>(p, nodes, n, flags, collide, after_bulk, s);
     }
-    if (wide) return special_shifted_tif<T, long long, false>(p, nodes, n, nforce, flags, collide, after_bulk, s);
-    return special_shifted_tif<T, int, false>(p, nodes, n, nforce, flags, collide, after_bulk, s);
+    if (wide) return special_shifted_tif<T, long long, false>(p, nodes, n, flags, collide, after_bulk, s);
+    return special_shifted_tif<T, int, false>(p, nodes, n, flags, collide, after_bulk, s);
 }
 
-cudaError_t special_shifted(const FastStepParams &p, const int2 *nodes, int n, int nforce, int store, bool flags, bool collide,
+cudaError_t special_shifted(const FastStepParams &p, const int2 *nodes, int n, int store, bool flags, bool collide,
                             bool after_bulk, cudaStream_t s) {
     if (n == 0) return cudaSuccess;
-    if (store == STORE_F32) return special_shifted_t<float>(p, nodes, n, nforce, flags, collide, after_bulk, s);
-    return special_shifted_t<__half>(p, nodes, n, nforce, flags, collide, after_bulk, s);
-}
-
-template <typename T, typename I, bool FORCE>
-static cudaError_t near_shifted_tif(const FastStepParams &p, const int2 *nodes, int n, int nforce,
-                                    const StageGroup &g, bool after, cudaStream_t s) {
-    const int per = (g.max_along + 127) / 128;
-    const dim3 grid(g.n * per + (n + 127) / 128), b(128);
-    if (p.s.links) return launch_follower(after, k_near_shifted<T, I, FORCE, true>, grid, b, s, p, nodes, n, nforce, per, g);
-    return launch_follower(after, k_near_shifted<T, I, FORCE, false>, grid, b, s, p, nodes, n, nforce, per, g);
-}
-
-template <typename T>
-static cudaError_t near_shifted_t(const FastStepParams &p, const int2 *nodes, int n, int nforce, const StageGroup &g,
-                                  bool after, cudaStream_t s) {
-    const bool wide = 9LL * p.s.plane >= (1LL << 31);
-    if (p.s.has_force) {
-        if (wide) return near_shifted_tif<T, long long, true>(p, nodes, n, nforce, g, after, s);
-        return near_shifted_tif<T, int, true>(p, nodes, n, nforce, g, after, s);
-    }
-    if (wide) return near_shifted_tif<T, long long, false>(p, nodes, n, nforce, g, after, s);
-    return near_shifted_tif<T, int, false>(p, nodes, n, nforce, g, after, s);
-}
-
-cudaError_t near_shifted(const FastStepParams &p, const int2 *nodes, int n, int nforce, int store, const StageGroup &g,
-                         bool after, cudaStream_t s) {
-    if (n == 0 && g.n == 0) return cudaSuccess;
-    if (store == STORE_F32) return near_shifted_t<float>(p, nodes, n, nforce, g, after, s);
-    return near_shifted_t<__half>(p, nodes, n, nforce, g, after, s);
+    if (store == STORE_F32) return special_shifted_t<float>(p, nodes, n, flags, collide, after_bulk, s);
+    return special_shifted_t<__half>(p, nodes, n, flags, collide, after_bulk, s);
 }
 
 template <typename T, bool FORCE, bool LINKS>

@@ -614,6 +614,7 @@ struct StageParams {
     const short *last;
     int entry;
     const FinishParams *fin;   // batches: the case's finish parameters (solo: by value)
+    const StepParams *step;    // batches in passes of several steps: the case's step
 };
 
 struct FinishParams {

@@ -112,3 +112,49 @@ def test_walls_and_edges_match_single_steps(storage, name):
                 assert np.array_equal(p, q)
         a.close()
         b.close()
+
+
+def _batch_cases(name):
+    from lbc_gb300 import impedance as imp
+    if name == "ducts":
+        return [(imp.liner_duct(p), p) for p in imp.sample_liners(5, 11)]
+    built = [cases.cylinder_wake(1501, 401, D=40.0, xc=400.0, yc=200.0, u_max=0.05, Re=60.0), cases.taylor_green(701, 450),
+             cases.cavity_moving_wall(500, 0.1, 300.0), cases.poiseuille(900, 333, 0.8, 1e-5),
+             cases.cylinder_golden(12)[:2], cases.taylor_green(640, 33)]
+    return [((c, cases.random_state(c, n)), None) for n, (c, _) in enumerate(built)]
+
+
+@pytest.mark.parametrize("name", ["ducts", "mix"])
+def test_batch_passes_match_cases_alone(name):
+    """A batch large enough for passes of several steps (with walls, links,
+    edges, impedance walls, periodic cases of odd width, with and without body
+    forces) leaves every case as single steps alone do, over two runs."""
+    from lbc_gb300 import F32_SHIFTED, GpuBatch, GpuSolver, impedance as imp
+    built = _batch_cases(name)
+    assert sum(c.nodes for (c, _), _ in built) >= 1 << 20
+
+    def solvers():
+        out = []
+        for (case, st), duct in built:
+            s = GpuSolver(case, F32_SHIFTED)
+            if duct is not None:
+                s.set_impedance_wall(imp.LINER_ENTRY, *imp.liner_arrays(duct), imp.TRACKED_OMEGAS, 1.0, imp.MEAN_RATE, 500)
+            s.set_state(st)
+            out.append(s)
+        return out
+
+    mixed, alone = solvers(), solvers()
+    b = GpuBatch(mixed)
+    b.run(47)
+    b.run(38)
+    for n, (x, y, (_, duct)) in enumerate(zip(mixed, alone, built)):
+        for _ in range(85):
+            y.run(1)
+        got, want = x.get_state(), y.get_state()
+        for fld in FIELDS:
+            assert np.array_equal(getattr(got, fld), getattr(want, fld), equal_nan=True), (n, fld)
+        assert x.forces() == y.forces()
+        if duct is not None:
+            for p, q in zip(x.impedance_readback(imp.LINER_ENTRY), y.impedance_readback(imp.LINER_ENTRY)):
+                assert np.array_equal(p, q)
+    b.close()
