@@ -175,12 +175,11 @@ LBM_HD uint64_t negate_if(uint64_t v, uint32_t sgn) {
     const uint64_t s = u64(sgn, sgn);
     return (v ^ s) - s;
 }
-// v 2^-n, bits shifted out kept as a sticky bit 0 (n of 64 or more included).
-// A zero v gives zero; the sticky bit alone is a value no rounding below sees.
+// v 2^-n, bits shifted out kept as a sticky bit 0. 64 or more give zero: below
+// 2^-62 beside numbers near 1 of 53 bits, which no rounding here sees.
 LBM_HD uint64_t shr_sticky(uint64_t v, uint32_t n) {
-    const uint32_t nn = n < 63u ? n : 63u;
-    const uint64_t lost = shl(v, 64u - nn);
-    return shr(v, nn) | (uint64_t)((lo32(lost) | hi32(lost)) != 0u);
+    const uint64_t lost = shl(v, 64u - n);
+    return shr(v, n) | (uint64_t)((lo32(lost) | hi32(lost)) != 0u);
 }
 // a * b: the high 64 bits, with bit 0 set when the low 64 are not zero.
 LBM_HD uint64_t mul_high_sticky(uint64_t a, uint64_t b) {
@@ -338,13 +337,14 @@ LBM_HD Moments moments(const uint64_t F[9], bool force, double hFx, double hFy, 
 // collide_exact rounds them. Br: the bracket, LSB 2^-62, 53 significant bits;
 // wr: w_1 rho, LSB 2^-(65 + sb); n = sb, 2 + sb, 4 + sb for w_0 = 4 w_1, w_1
 // and w_5 = w_1 / 4 (exact in FP64: powers of two apart).
-LBM_HD double relax(uint64_t F, uint64_t wr, uint32_t n, uint64_t Br, double om, double om_m9, uint32_t &bad) {
+// big collects the high words of |f - f_eq|, to be below 2^20 (2^-9).
+LBM_HD double relax(uint64_t F, uint64_t wr, uint32_t n, uint64_t Br, double om, double om_m9, uint32_t &big) {
     // f_eq: product rounded to 53 bits, then to LSB 2^-61 (exact: f_eq >= 2^-8)
     const uint64_t feq = shr(round53(mul_high_sticky(wr, Br)), n);
     const uint64_t d = F - feq;
     const bool neg = (int32_t)hi32(d) < 0;
     const uint64_t a = neg ? 0ull - d : d;  // |f - f_eq|, exact
-    bad |= hi32(a) >> 20 ? 0x80000000u : 0u;
+    big |= hi32(a);
     // 2^-9 + |f - f_eq| is the FP64 number with these mantissa bits
     const double m = make_double(lo32(a), hi32(a) | ((1023u - 9u) << 20));
     const double g = fma(om, m, om_m9);  // omega |f - f_eq|, rounded once
@@ -377,17 +377,16 @@ LBM_HD bool step_node(double f[9], const double w[9], bool force, double hFx, do
     const uint64_t kNinth = 0xE38E38E38E38E000ull;  // the FP64 number 1/9, LSB 2^-67
     const uint64_t wr = round53(mul_high_sticky(kNinth, q.D << 1));
     const Num tn = num_of(mul(1.5, add(mul(ux, ux), mul(uy, uy))));
-    uint32_t far = 0;
+    uint32_t far = 0, big = 0;
     const uint64_t T = shr_sticky(tn.m, tn.e - 62u);
     const uint64_t one = 1ull << 62;
     // -omega 2^-9, exact
     const double om_m9 = make_double(words(om).lo, words(om).hi + 0x80000000u - (9u << 20));
     const Num c[4] = {q.ux, q.uy, num_of(add(ux, uy)), num_of(add(uy, -ux))};
     double r[9];
-    // brackets below 1/4 or from 2 up set bit 31 of far
+    // For |c.u| < 1/4 every bracket is above 1/4.
     const uint64_t b0 = round_low(one - T, 9);  // 3/4 < 1 - T <= 1
-    far |= (hi32(b0) - 0x10000000u) | hi32(b0);
-    r[0] = relax(F[0], wr, q.sb, b0, om, om_m9, bad);
+    r[0] = relax(F[0], wr, q.sb, b0, om, om_m9, big);
 #pragma unroll
     for (int i = 0; i < 4; i++) {
         const int ka = i < 2 ? 1 + i : 3 + i, kb = ka + 2;  // (1,3) (2,4) (5,7) (6,8)
@@ -397,35 +396,43 @@ LBM_HD bool step_node(double f[9], const double w[9], bool force, double hFx, do
         const bool neg = c[i].sgn != 0;
         const uint64_t B = shr_sticky(round53(3u * m) << 8, c[i].e - 65u);
         const uint64_t A = shr_sticky(round53(mul_high_sticky(round53(9u * m) << 7, c[i].m)), 2u * c[i].e - 129u);
-        // 1 + |B| + A in [1, 2) (checked): 10 bits go
+        // 1 + |B| + A in [1, 2) (bit 31 of far otherwise): 10 bits go
         const uint64_t p2 = round_low(round_low(one + B, 10) + A, 10);
         far |= hi32(p2);
         const uint64_t p3 = round53(p2 - T), m3 = round53(round53(round53(one - B) + A) - T);
         const uint64_t bp = neg ? m3 : p3, bm = neg ? p3 : m3;
-        far |= (hi32(bp) - 0x10000000u) | hi32(bp);
-        far |= (hi32(bm) - 0x10000000u) | hi32(bm);
-        r[ka] = relax(F[ka], wr, (i < 2 ? 2u : 4u) + q.sb, bp, om, om_m9, bad);
-        r[kb] = relax(F[kb], wr, (i < 2 ? 2u : 4u) + q.sb, bm, om, om_m9, bad);
+        r[ka] = relax(F[ka], wr, (i < 2 ? 2u : 4u) + q.sb, bp, om, om_m9, big);
+        r[kb] = relax(F[kb], wr, (i < 2 ? 2u : 4u) + q.sb, bm, om, om_m9, big);
     }
-    if (bad > 7u || (far >> 31)) return false;
+    if ((big >> 20) || (far >> 31)) return false;
     if (!force) {
 #pragma unroll
         for (int k = 0; k < 9; k++) f[k] = add(f[k], r[k]);
         return true;
     }
-    // Guo's term (collide_exact): w (3 c.F + 9 (c.u)(c.F) - 3 u.F); the pair's
-    // product (9 c.u)(c.F) is the same for both directions.
-    const double uF3 = mul(3.0, add(mul(ux, Fx), mul(uy, Fy)));
+    // Guo's term (collide_exact): w (3 c.F + 9 (c.u)(c.F) - 3 u.F), in the FP64
+    // sequence. The pair's product (9 c.u)(c.F) is the same for both directions;
+    // a direction across the force has 3 u.F alone, and its w_1 multiple serves
+    // the rest population (w_0 = 4 w_1). Zero terms are left out: x + 0 = x.
+    const bool fx = Fx != 0.0, fy = Fy != 0.0;
+    const double uF = !fy ? mul(ux, Fx) : !fx ? mul(uy, Fy) : add(mul(ux, Fx), mul(uy, Fy));
+    const double uF3 = mul(3.0, uF);
     const double g = add(1.0, -mul(0.5, om));
-    f[0] = add(f[0], add(r[0], mul(g, mul(w[0], -uF3))));
+    const double across = mul(g, mul(w[1], -uF3));
+    f[0] = add(f[0], add(r[0], mul(4.0, across)));
     const double cF[4] = {Fx, Fy, add(Fx, Fy), add(Fy, -Fx)};
 #pragma unroll
     for (int i = 0; i < 4; i++) {
         const int ka = i < 2 ? 1 + i : 3 + i, kb = ka + 2;
-        const double cu = i == 0 ? ux : i == 1 ? uy : i == 2 ? add(ux, uy) : add(uy, -ux);
-        const double L = mul(3.0, cF[i]), X = mul(mul(9.0, cu), cF[i]);
-        f[ka] = add(f[ka], add(r[ka], mul(g, mul(w[ka], add(add(L, X), -uF3)))));
-        f[kb] = add(f[kb], add(r[kb], mul(g, mul(w[kb], add(add(-L, X), -uF3)))));
+        double ta = across, tb = across;
+        if (i == 0 ? fx : i == 1 ? fy : true) {
+            const double cu = i == 0 ? ux : i == 1 ? uy : i == 2 ? add(ux, uy) : add(uy, -ux);
+            const double L = mul(3.0, cF[i]), X = mul(mul(9.0, cu), cF[i]);
+            ta = mul(g, mul(w[ka], add(add(L, X), -uF3)));
+            tb = mul(g, mul(w[kb], add(add(-L, X), -uF3)));
+        }
+        f[ka] = add(f[ka], add(r[ka], ta));
+        f[kb] = add(f[kb], add(r[kb], tb));
     }
     return true;
 }
