@@ -9,7 +9,7 @@ than L2, so no flush is needed between steps.
   value     FP32-shifted fused step, state resident in HBM (lbm_gpu_run), MLUPS
   fp64      the plain FP64 fused kernel (bit-identical to lbc), same workload,
             with its FP64 instructions per node and fraction of the measured
-            FP64 issue rate; fp64.fma the fused multiply-add form (1e-12 of lbc)
+            FP64 issue rate; fp64.fma the F64_FMA storage (1e-12 of lbc)
   fp16      FP16-shifted storage, same workload
   e2e       lbc's own main_lbm call through this library's C ABI with host
             arrays (page-locked): each call reads f, rho, u, v and writes f,
@@ -207,10 +207,11 @@ def taylor_green_decay(storage, n, steps, every=500):
 
 
 def fp64_record(res, hbm, n, fp64_rate):
-    """The FP64 step kernels: lbc's arithmetic bit for bit, and the fused
-    multiply-add form. Both are bound by FP64 issue on GB300, so each reports
-    its FP64 instructions per node (ncu) and the fraction of the measured FP64
-    FMA issue rate it reaches beside its fraction of HBM bandwidth."""
+    """The FP64 step: lbc's arithmetic bit for bit, mostly on the integer pipes
+    (24 FP64 instructions per node), as F64 and as F64_FMA, which steps the same
+    way with lbc's weights. Each reports its FP64 instructions per node (ncu) and
+    the fraction of the measured FP64 FMA issue rate they take beside its
+    fraction of HBM bandwidth."""
     def issue(key, mlups):
         ipn = fp64_inst_per_node(key)
         if ipn is None or not fp64_rate:
@@ -219,13 +220,13 @@ def fp64_record(res, hbm, n, fp64_rate):
 
     f64, fma = res["f64"], res["f64fma"]
     ipn_x, frac_x = issue("exact", f64["mlups"])
-    ipn_f, frac_f = issue("fma", fma["mlups"])
+    ipn_f, frac_f = issue("exact", fma["mlups"])
     return {"value": round(f64["mlups"], 1), "ms_per_step": round(f64["ms_per_step"], 4),
             "achieved_gbs": round(f64["gbs"], 1), "frac_hbm": round(f64["gbs"] / hbm, 4),
             "traffic": traffic_per_launch(f"f64_{n}"), "steps": f64["steps"],
             "fp64_inst_per_node": ipn_x, "frac_fp64_issue": frac_x,
             "fp64_fma_rate_lane_ops_per_s": fp64_rate,
-            "bound": "FP64 issue (GB300 issues about 2 FP64 lane operations per clock per SM)",
+            "bound": "integer issue, then FP64 issue (GB300: about 2 FP64 lane operations per clock per SM)",
             "parity": "bit-identical to lbc's FP64 CPU solver",
             "fma": {"value": round(fma["mlups"], 1), "ms_per_step": round(fma["ms_per_step"], 4),
                     "achieved_gbs": round(fma["gbs"], 1), "frac_hbm": round(fma["gbs"] / hbm, 4),
@@ -316,21 +317,23 @@ def run_ours(a, ws, rank, pg):
         s.run(a.warmup)
         s.sync()
         barrier(pg)
+        before, _ = s.launch_stats()
         ms = s.run_timed(steps)
         barrier(pg)
         ms = allmax(pg, ms)
-        info = s.info()
-        return s, ms, None, info
+        after, per_pass = s.launch_stats()
+        return s, ms, per_pass, after - before
 
     # Clocks are sampled over all timed regions (nvidia-smi samples every 200 ms).
     clk = Clocks()
     clk.start()
     # FP32-shifted: the headline.
-    s32, ms32, _, info32 = timed(lbc_gb300.F32_SHIFTED, a.steps)
+    # (bytes: one read and one write of every population per pass of pass32 steps)
+    s32, ms32, pass32, launches32 = timed(lbc_gb300.F32_SHIFTED, a.steps)
     bytes32 = 2 * 9 * 4 * N
     t_step = ms32 / a.steps / 1e3
     res["f32"] = {"mlups": ws * N * a.steps / (ms32 / 1e3) / 1e6, "ms_per_step": ms32 / a.steps,
-                  "gbs": bytes32 / t_step / 1e9, "launches": 1 + a.steps * info32.launches_per_step}
+                  "gbs": bytes32 / pass32 / t_step / 1e9, "launches": launches32}
     del s32
     # FP64 plain.
     k64 = a.fp64_steps or max(20, a.steps // 5)
@@ -340,7 +343,7 @@ def run_ours(a, ws, rank, pg):
     t64 = ms64 / k64 / 1e3
     res["f64"] = {"mlups": ws * N * k64 / (ms64 / 1e3) / 1e6, "ms_per_step": ms64 / k64,
                   "gbs": bytes64 / t64 / 1e9, "steps": k64}
-    # FP64 storage, fused multiply-add step (lbc's results to rounding).
+    # F64_FMA storage (lbc's results to rounding).
     sfm, msfm, _, _ = timed(lbc_gb300.F64_FMA, k64)
     del sfm
     tfm = msfm / k64 / 1e3
@@ -351,7 +354,7 @@ def run_ours(a, ws, rank, pg):
     rate = C.c_double(0.0)
     fp64_rate = rate.value if lib0.lbm_gpu_fp64_rate(C.byref(rate)) == 0 else None
     # FP16-shifted.
-    s16, ms16, _, _ = timed(lbc_gb300.F16_SHIFTED, a.steps)
+    s16, ms16, pass16, _ = timed(lbc_gb300.F16_SHIFTED, a.steps)
     del s16
     bytes16 = 2 * 9 * 2 * N
     t16 = ms16 / a.steps / 1e3
@@ -415,6 +418,8 @@ def run_ours(a, ws, rank, pg):
             cs.run(a.warmup)
             barrier(pg)
             cms = allmax(pg, cs.run_timed(a.cavity_steps))
+            if storage == lbc_gb300.F32_SHIFTED:
+                cpass = cs.launch_stats()[1]
             cres[name] = (cms, cs.get_fields())
             del cs
         m = ccase.solid_mask == 0
@@ -425,7 +430,8 @@ def run_ours(a, ws, rank, pg):
         c32 = ws * ccase.nodes * a.cavity_steps / (cres["f32"][0] / 1e3) / 1e6
         c64 = ws * ccase.nodes * a.cavity_steps / (cres["f64"][0] / 1e3) / 1e6
         cavity = {"grid": "2048x2048", "steps": a.warmup + a.cavity_steps, "f32_mlups": round(c32, 1),
-                  "f32_frac_hbm": round(c32 * 1e6 * 72 / 1e9 / hbm, 4), "fp64_mlups": round(c64, 1),
+                  "f32_steps_per_pass": cpass,
+                  "f32_frac_hbm": round(c32 * 1e6 * 72 / cpass / 1e9 / hbm, 4), "fp64_mlups": round(c64, 1),
                   "ratio_f32_vs_fp64": round(c32 / c64, 2), "u_l2_rel_f32_vs_fp64": err,
                   "mass_rel_f32_vs_fp64": float(np.sum(r32[m]) / np.sum(r64[m]) - 1.0),
                   "note": "moving-wall bounce-back lid, u 0.1, Re 1000; one replica per rank"}
@@ -443,12 +449,14 @@ def run_ours(a, ws, rank, pg):
             sm = wake.summary(h)
             sm["mlups"] = ws * h["nodes"] * a.wake_steps / (allmax(pg, h["ms"]) / 1e3) / 1e6
             wk[name] = sm
+            wk[name + "_pass"] = h["steps_per_pass"]
         f32w, f64w = wk["f32"], wk["f64"]
         wake_res = {"grid": "2048x512", "steps": a.wake_steps, "D": 64, "Re": 100, "u_max": 0.05,
                     "f64": {k: (round(v, 6) if k != "mlups" else round(v, 1)) for k, v in f64w.items()},
                     "f32": {k: (round(v, 6) if k != "mlups" else round(v, 1)) for k, v in f32w.items()},
                     "f32_rel_err_vs_f64": {q: float(f32w[q] / f64w[q] - 1.0) for q in ("cd_mean", "cl_rms", "st")},
-                    "f32_frac_hbm": round(f32w["mlups"] * 1e6 * 72 / 1e9 / hbm, 4),
+                    "f32_steps_per_pass": wk["f32_pass"],
+                    "f32_frac_hbm": round(f32w["mlups"] * 1e6 * 72 / wk["f32_pass"] / 1e9 / hbm, 4),
                     "ratio_f32_vs_fp64": round(f32w["mlups"] / f64w["mlups"], 2),
                     "note": "statistics over the second half of the run; St from the Hann-windowed FFT peak of Cl; "
                             "one replica per rank"}
@@ -491,7 +499,7 @@ def run_ours(a, ws, rank, pg):
                                        if a.serve_f64 == "fma" else "FP64 storage, lbc's arithmetic bit for bit")}
     clocks = clk.stop()
     res["f16"] = {"mlups": ws * N * a.steps / (ms16 / 1e3) / 1e6, "ms_per_step": ms16 / a.steps,
-                  "gbs": bytes16 / t16 / 1e9}
+                  "gbs": bytes16 / pass16 / t16 / 1e9}
 
     # Accuracy against the FP64 kernel (itself bit-identical to lbc) after E
     # steps on the bench grid.
@@ -612,7 +620,9 @@ def run_ours(a, ws, rank, pg):
         "roofline": {"bound": "hbm", "achieved": round(f32["gbs"], 1), "peak": hbm, "unit": "GB/s",
                      "frac": round(f32["gbs"] / hbm, 4), "peak_kind": peak_kind,
                      "traffic": traffic_per_launch(f"f32_{n}"),
-                     "algorithmic_bytes_per_launch": bytes32},
+                     "algorithmic_bytes_per_launch": bytes32, "steps_per_launch": pass32,
+                     "note": "achieved counts one read and one write of every population per pass of "
+                             "steps_per_launch steps; past one step per pass FP32 issue bounds it, not HBM"},
         "fp64": fp64_record(res, hbm, n, fp64_rate),
         "fp16": {"value": round(res["f16"]["mlups"], 1), "achieved_gbs": round(res["f16"]["gbs"], 1),
                  "frac_hbm": round(res["f16"]["gbs"] / hbm, 4), "traffic": traffic_per_launch(f"f16_{n}")},

@@ -29,11 +29,10 @@ extern "C" {
 
 /* Population storage. F64: lbc's arithmetic, bit for bit. F32/F16_SHIFTED:
  * populations stored as f_k - w_k in FP32 / FP16, collision in FP32.
- * F64_FMA: FP64 storage, the step's moments and collision with fused
- * multiply-adds and the D2Q9 pair symmetry (74 FP64 instructions per node
- * against 125, so 1.6-1.9x faster on a part whose FP64 rate bounds the step);
- * lbc's results to rounding (1e-12 relative), not bit for bit. It needs lbc's
- * weight symmetry (w1 = w2 = w3 = w4, w5 = w6 = w7 = w8). */
+ * F64_FMA: FP64 storage, lbc's results to rounding (1e-12 relative). With lbc's
+ * weights it steps as F64 does (the integer form of the step is the faster);
+ * with other weights of their symmetry (w1 = w2 = w3 = w4, w5 = w6 = w7 = w8,
+ * which it needs) it uses fused multiply-adds. */
 enum { LBM_GPU_F64 = 0, LBM_GPU_F32_SHIFTED = 1, LBM_GPU_F16_SHIFTED = 2, LBM_GPU_F64_FMA = 3 };
 
 typedef struct lbm_gpu_solver lbm_gpu_solver;
@@ -62,14 +61,16 @@ typedef struct {
     int Nx, Ny, pitch, storage;
     int has_geometry;              /* 0: fully periodic, no solids, no edge BCs */
     int edge_stages;               /* Boundary entries run as edge kernels */
-    int launches_per_step;         /* kernel launches per time step in the loop: the bulk
+    int launches_per_step;         /* kernel launches of a time step on its own: the bulk
                                       step; the special-node step (F32/F16 storage with
                                       a flag word); edge_launches, which also finish the
                                       BC-written nodes and reduce the wall force, or,
                                       with wall links but no edge stages, one force
                                       reduction when a force history is enabled (the
-                                      loop's steps reduce the force only then; a run's
-                                      last step always does, for lbm_gpu_forces) */
+                                      last step always does, for lbm_gpu_forces). Inside
+                                      a run a Boundary list of one launch rides with the
+                                      special nodes (F32/F16), and passes of several
+                                      steps take fewer: lbm_gpu_launch_stats counts */
     size_t device_bytes;
     long long steps_done;
     int edge_launches;             /* launches the edge stages take per step: consecutive
@@ -196,6 +197,10 @@ long long lbm_gpu_write_impedance_trace(lbm_gpu_solver *s, int entry, const char
 int lbm_gpu_msd_zoh(double R, double m, double K, double *A, double *b);
 
 int lbm_gpu_get_info(lbm_gpu_solver *s, lbm_gpu_info *info);
+/* The kernels this solver's runs have launched so far (those of replayed graphs
+ * included), and the time steps one pass over the populations takes in a long
+ * run (1, 2 or 4). */
+int lbm_gpu_launch_stats(lbm_gpu_solver *s, long long *launches, int *steps_per_pass);
 /* Thread-block shape of the fused step (bx * by <= 256, bx multiple of 32).
  * No result depends on it: populations, fields and the momentum-exchange force
  * (summed in a fixed order per 32-node row segment in FP64 storage, per

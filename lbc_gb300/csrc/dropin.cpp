@@ -913,6 +913,13 @@ int lbm_gpu_msd_zoh(double R, double m, double K, double *A, double *b) {
     return LBM_GPU_OK;
 }
 
+int lbm_gpu_launch_stats(lbm_gpu_solver *s, long long *launches, int *steps_per_pass) {
+    SOLVER_OR_FAIL(s);
+    if (launches) *launches = s->s->launches();
+    if (steps_per_pass) *steps_per_pass = std::max(1, s->s->multi_levels());
+    return LBM_GPU_OK;
+}
+
 int lbm_gpu_get_info(lbm_gpu_solver *s, lbm_gpu_info *info) {
     SOLVER_OR_FAIL(s);
     info->Nx = s->s->Nx();

@@ -107,6 +107,9 @@ Solver::Solver(const CaseDesc &d) : d_(d) {
         const long long warps = (long long)((d_.Nx + 31) / 32) * d_.Ny;
         block_ = warps <= 4LL * launch::sm_count() ? dim3(32, 1, 1) : dim3(64, 2, 1);
     }
+    // (a failure here shows at the launch)
+    if (multi_levels() > 0 && launch::multi_load(d_.store, multi_levels(), !has_flags_, has_force()) != cudaSuccess)
+        cudaGetLastError();
     ok_ = true;
     set_autotune(tune_default_mode());
 }
@@ -1694,9 +1697,22 @@ int Solver::tune_online(int avail) {
     return used;
 }
 
+// Kernels of one step inside run(), as launch_step launches them.
+int Solver::loop_launches() const {
+    const int force = has_mem_ && hist_cap_ > 0 ? 1 : 0, rec = rec_host_.empty() ? 0 : 1;
+    const int bulk = 1 + (special_launch() ? 1 : 0);
+    if (groups_.empty()) return bulk + force + rec;
+    const bool rides = one_group_ && d_.store != STORE_F64 && special_launch() && !wide();
+    if (rides) return bulk + force + rec;
+    // FP64 with one group reduces the force on its own; otherwise it rides in
+    // the first group's launch
+    return bulk + (int)groups_.size() + (one_group_ && d_.store == STORE_F64 ? force : 0) + rec;
+}
+
 bool Solver::run(int nsteps) {
     if (nsteps <= 0) return true;
     if (!launch_collide(cur_)) return false;
+    launches_ += 1 + launches_per_step();  // the collision, and the last step
     int remaining = nsteps - 1;
     // Tuning takes its trial windows from the steps of this run.
     if (tune_mode_ && !tuned_ && remaining >= 2 + 2 * kNBlockCand) {
@@ -1707,6 +1723,12 @@ bool Solver::run(int nsteps) {
     const int used = run_multi(remaining);
     if (used < 0) return false;
     remaining -= used;
+    launches_ += (long long)(nsteps - 1 - used) * loop_launches();
+    if (used > 0) {
+        const int lv = multi_levels(), force = has_mem_ && hist_cap_ > 0 ? 1 : 0;
+        const int near = 1 + (one_group_ ? force : (int)groups_.size());
+        launches_ += (long long)(used / lv) * (has_flags_ ? 1 + lv * near : 1) + (has_flags_ ? 2 : 0);
+    }
     if (remaining >= 2 * kGraphPairs) {
         if (!capture_pair()) return false;
         for (; remaining >= 2 * kGraphPairs; remaining -= 2 * kGraphPairs) CK(cudaGraphLaunch(pair_exec_, stream_));

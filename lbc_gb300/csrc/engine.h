@@ -160,7 +160,7 @@ class Solver {
     void *buffer(int b) const { return buf_[b]; }
     int current() const { return cur_; }
     long long steps_done() const { return steps_done_; }
-    // Kernel launches per time step inside the loop (for launch counting).
+    // Kernel launches of a time step on its own.
     int launches_per_step() const {
         const int bulk = 1 + (special_launch() ? 1 : 0);
         const int rec = rec_host_.empty() ? 0 : 1;
@@ -168,6 +168,7 @@ class Solver {
         if (groups_.empty()) return bulk + (has_mem_ && hist_cap_ > 0 ? 1 : 0) + rec;
         return bulk + (int)groups_.size() + rec;
     }
+    long long launches() const { return launches_; }
     // Shifted storage: the nodes the clean-pair kernels leave to the
     // special-node kernel (row-major; both nodes of a pair with a special
     // node, and an odd last column). Launched on its own for grids with a
@@ -241,6 +242,7 @@ class Solver {
     bool begin_steps(cudaStream_t s);
     bool end_steps(cudaStream_t s);
     // Passes of several steps, for a case alone and in a batch.
+    int multi_levels() const;
     bool multi_case() const {
         return d_.store != STORE_F64 && !d_omega_ && rec_host_.empty() && one_group_ && d_.Nx >= 8 && d_.Ny >= 8 &&
                !wide() && (long long)special_host_.size() <= (long long)d_.Nx * d_.Ny / 8;
@@ -276,7 +278,6 @@ class Solver {
     int nprobes_ = 0, probe_cap_ = 0;
     bool launch_collide(int b, cudaStream_t s = nullptr);
     bool capture_pair();
-    int multi_levels() const;
     int multi_warps() const;
     bool multi_setup();
     bool launch_multi(int cur, int other, int lv);
@@ -346,6 +347,8 @@ class Solver {
     cudaEvent_t multi_fork_ = nullptr, multi_join_ = nullptr;
     size_t dev_bytes_ = 0;
     long long steps_done_ = 0;
+    long long launches_ = 0;   // kernels launched by run()
+    int loop_launches() const;
     std::vector<void *> allocs_;
     bool needs_old_dst_ = true;
     // FP64 storage: the nodes the step may leave old content in (solid, or a

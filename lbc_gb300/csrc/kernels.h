@@ -176,6 +176,9 @@ cudaError_t multi_plain(const FastStepParams &p, int store, int levels, int warp
 // nodes away from any special node: deep[strip * Ny + row], a bit per lane's
 // pair (strips of 64 - 2 multi_halo(levels) columns).
 cudaError_t multi_geo(const FastStepParams &p, int store, int levels, const uint32_t *deep, int warps, cudaStream_t s);
+// Loads the pass kernel that multi_plain (plain) or multi_geo would launch: CUDA
+// loads a kernel at its first use, which takes this one some milliseconds.
+cudaError_t multi_load(int store, int levels, bool plain, bool force);
 // The same for every case of a batch: a warp per task, parameter set sel of nsp
 // per case; force: some case has a body force.
 cudaError_t multi_batch(const FastStepParams *sp, int nsp, int sel, const MultiTask *tasks, int ntasks,

@@ -261,6 +261,18 @@ __global__ void k_multi_swap(const int2 *__restrict__ nodes, int n, const uint16
 namespace launch {
 
 template <typename T, int LV>
+static cudaError_t multi_load_tl(bool plain, bool force) {
+    cudaFuncAttributes a;
+    if (plain) return force ? cudaFuncGetAttributes(&a, k_multi_plain<T, LV, true>) : cudaFuncGetAttributes(&a, k_multi_plain<T, LV, false>);
+    return force ? cudaFuncGetAttributes(&a, k_multi_geo<T, LV, true>) : cudaFuncGetAttributes(&a, k_multi_geo<T, LV, false>);
+}
+
+cudaError_t multi_load(int store, int levels, bool plain, bool force) {
+    if (store == STORE_F32) return levels == 2 ? multi_load_tl<float, 2>(plain, force) : multi_load_tl<float, 4>(plain, force);
+    return levels == 2 ? multi_load_tl<__half, 2>(plain, force) : multi_load_tl<__half, 4>(plain, force);
+}
+
+template <typename T, int LV>
 static cudaError_t multi_geo_tl(const FastStepParams &p, const uint32_t *deep, int warps_wanted, cudaStream_t s) {
     const int width = 64 - 2 * multi_halo(LV);
     const int strips = (p.s.Nx + width - 1) / width;

@@ -88,6 +88,7 @@ def _bind_ext(lib: C.CDLL) -> None:
         "lbm_gpu_write_impedance_trace": (C.c_longlong, [vp, C.c_int, C.c_char_p, C.c_double, C.c_double,
                                                          C.c_double, C.c_int]),
         "lbm_gpu_get_info": (C.c_int, [vp, C.POINTER(Info)]),
+        "lbm_gpu_launch_stats": (C.c_int, [vp, C.POINTER(C.c_longlong), C.POINTER(C.c_int)]),
         "lbm_gpu_set_block": (C.c_int, [vp, C.c_int, C.c_int]),
         "lbm_gpu_get_block": (C.c_int, [vp, C.POINTER(C.c_int), C.POINTER(C.c_int)]),
         "lbm_gpu_checkpoint_save": (C.c_int, [vp, C.c_char_p]),
@@ -353,6 +354,13 @@ class GpuSolver:
         inf = Info()
         _check(self.lib.lbm_gpu_get_info(self.h, C.byref(inf)), "lbm_gpu_get_info")
         return inf
+
+    def launch_stats(self):
+        """(kernels launched by this solver's runs, time steps per pass over the
+        populations in a long run)."""
+        n, k = C.c_longlong(), C.c_int()
+        _check(self.lib.lbm_gpu_launch_stats(self.h, C.byref(n), C.byref(k)), "lbm_gpu_launch_stats")
+        return n.value, k.value
 
     def set_block(self, bx: int, by: int):
         _check(self.lib.lbm_gpu_set_block(self.h, bx, by), "lbm_gpu_set_block")

@@ -41,7 +41,7 @@ def strouhal(cl: np.ndarray, D: float, u: float) -> float:
 def cylinder_forces(storage: int, steps: int, Nx: int = 2048, Ny: int = 512, D: float = 64.0,
                     u_max: float = 0.05, Re: float = 100.0, seed: int = 0):
     """Run the cylinder case for `steps` steps in one storage type; return the
-    per-step (Cd, Cl) history and the device time."""
+    per-step (Cd, Cl) history, the device time and the steps per pass."""
     case, st = cases.cylinder_wake(Nx, Ny, D=D, xc=Nx / 4.0, yc=Ny / 2.0, u_max=u_max, Re=Re, seed=seed)
     s = GpuSolver(case, storage)
     s.enable_force_history(steps)
@@ -51,7 +51,7 @@ def cylinder_forces(storage: int, steps: int, Nx: int = 2048, Ny: int = 512, D: 
     scale = 2.0 / (1.0 * u_max * u_max * D)
     cd = hist[:, 0] * scale
     cl = hist[:, 1] * scale
-    return {"cd": cd, "cl": cl, "ms": ms, "nodes": case.nodes}
+    return {"cd": cd, "cl": cl, "ms": ms, "nodes": case.nodes, "steps_per_pass": s.launch_stats()[1]}
 
 
 def summary(h, D: float = 64.0, u_max: float = 0.05) -> dict:
