@@ -81,8 +81,8 @@ const char *lbm_gpu_last_error(void);
 int lbm_gpu_device_count(void);
 /* The current device's FP64 fused multiply-add issue rate, measured (thread
  * FMA instructions per second, the fastest of five timed launches of a kernel
- * of independent DFMA chains): the ceiling of the FP64 step kernels, which are
- * bound by FP64 issue on parts with a low FP64 rate such as GB300. */
+ * of independent DFMA chains): about 2 per clock per SM on GB300, which is why
+ * the FP64 step does most of its arithmetic on the integer pipes. */
 int lbm_gpu_fp64_rate(double *lane_ops_per_s);
 /* How kernels can reach host memory at p: 1 page-locked and mapped at the
  * same address, 2 any pageable memory (the device walks the host page tables,

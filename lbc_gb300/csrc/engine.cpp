@@ -1413,6 +1413,9 @@ int Solver::multi_levels() const {
     const long long n = (long long)d_.Nx * d_.Ny;
     if (d_.store == STORE_F64 || d_omega_ || !rec_host_.empty()) return 0;
     if (d_.Nx < 8 || d_.Ny < 8 || plane_ >= (1LL << 31) || (has_flags_ && wide())) return 0;
+    // Narrow grids whose last strip is mostly empty (channel 64 x 8192: 7.8 us one
+    // step at a time, 8.9 in passes; 120 x 4000 7.9 and 5.8).
+    if (n < (1LL << 22) && (d_.Nx + 55) / 56 * 320 > 8 * d_.Nx) return 0;
     // With a flag word the nodes near walls and edges go step by step beside the
     // pass, a chain of launches that bounds small grids. FP32: cylinder 1024 x
     // 256 8.30 against 7.78 with two levels and 8.00 with four, 2048 x 512 10.9,
@@ -1553,6 +1556,11 @@ bool Solver::multi_setup() {
     if (cudaMemGetInfo(&freeb, &total) != cudaSuccess || freeb / 4 < (size_t)(lv > 2 ? 2 : 1) * multi_bytes()) return false;
     NearPlan plan;
     near_plan(lv, plan);
+    // With much of the grid near walls the lists outweigh the pass (channel 16384 x
+    // 64, 16 % near: 12.9 us one step at a time, 13.7 in passes; 32768 x 64 27.8
+    // and 22.0).
+    const long long n = (long long)d_.Nx * d_.Ny;
+    if (n < (1LL << 21) && 16 * plan.near_pairs > n * lv) return false;
     if (!dalloc(&d_deep_, plan.deep.size())) return false;
     CK(cudaMemcpyAsync(d_deep_, plan.deep.data(), plan.deep.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, stream_));
     for (int q = 0; q < lv; q++) {
@@ -2114,7 +2122,7 @@ bool Batch::multi_setup() {
     if (multi_state_) return multi_state_ > 0;
     multi_state_ = -1;
     const int lv = multi_lv_;
-    if (store_ == STORE_F64 || nodes_ < (store_ == STORE_F32 ? (1LL << 20) : (1LL << 22)) || nrec_ || max_stages_ > 1)
+    if (store_ == STORE_F64 || nodes_ < (store_ == STORE_F32 ? (1LL << 22) : (1LL << 23)) || nrec_ || max_stages_ > 1)
         return false;
     size_t need = 0, freeb = 0, total = 0;
     for (Solver *c : cases_) {
@@ -2142,7 +2150,10 @@ bool Batch::multi_setup() {
                 tasks.push_back(MultiTask{(int)c, st, y, std::min(Ny, y + h), (long long)deep.size()});
         deep.insert(deep.end(), plan.deep.begin(), plan.deep.end());
     }
-    if (near > nodes_ * lv / 2) return false;
+    // Measured, one step at a time against passes: 13.5 M nodes 198 -> 125 us, 6.7
+    // M (14 % of the node steps near) 103 -> 81, 3.2 M 50-57 either way, below
+    // that slower: four list launches bound a pass.
+    if (near > nodes_ * lv / 5) return false;
     for (Solver *c : cases_)  // (allocated on the case's stream, used on this one)
         if (!c->multi_buffers(lv) || !check_cuda(cudaStreamSynchronize(c->stream()), "multi_buffers")) return false;
     const int nc = (int)cases_.size(), ne = max_stages_ ? stage_counts_[0] : 0;

@@ -1,6 +1,5 @@
-// pdl.cuh -- programmatic dependent launch between consecutive kernels of a
-// step in the same stream (clean pairs, special nodes, edge stages, force
-// reduction).
+// pdl.cuh -- programmatic dependent launch between consecutive kernels in the
+// same stream (clean pairs, special nodes, edges, force reduction).
 //
 // A kernel signals at its start that the next kernel may be launched
 // (griddepcontrol.launch_dependents); a follower launched with programmatic

@@ -80,8 +80,8 @@ def make_stream(n: int = 2000, seed: int = 2026, rate: float = 50.0, scale: floa
                 max_nodes: int = 2048 * 512, f64_storage: int = F64) -> List[Req]:
     """A seeded Poisson stream of channel / cylinder / liner requests. The 20 %
     of requests that ask for FP64 storage get f64_storage: F64 (lbc's
-    arithmetic, bit for bit) or F64_FMA (the fused multiply-add step, lbc's
-    results to rounding at 1.6-1.9x the speed)."""
+    arithmetic, bit for bit) or F64_FMA (lbc's results to rounding; the same step
+    with lbc's weights)."""
     rng = np.random.default_rng(seed)
     out, t = [], 0.0
     lo, hi = math.log(128 * 32), math.log(min(2048 * 512, max_nodes))
