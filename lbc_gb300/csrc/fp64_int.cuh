@@ -21,7 +21,7 @@
 // ranges of an ordinary flow (checked per node, the flag `ok`); any other node
 // takes moments_exact / collide_exact. Ranges: populations and equilibria in
 // [2^-8, 1) (f_1 .. f_8 below 1/2), 9/16 <= rho < 2, |c.u| < 1/4, |f - f_eq| <
-// 2^-9. Zeros come out with lbc's value; their sign is not kept.
+// 2^-9 (2^-6 where no f or f_eq is below 2^-6). Zeros come out with lbc's value; their sign is not kept.
 //
 // The division by the density is an integer one: a 64-bit reciprocal by Newton
 // steps from the FP32 one, shared by both velocities, and the exact remainder
@@ -72,6 +72,15 @@ LBM_HD uint32_t shl_wide(uint32_t lo, uint32_t hi, uint32_t s) {
 #else
     s &= 31;
     return s ? (hi << s) | (lo >> (32 - s)) : hi;
+#endif
+}
+// low word of hi:lo >> (s mod 32)
+LBM_HD uint32_t shr_wide(uint32_t lo, uint32_t hi, uint32_t s) {
+#ifdef __CUDA_ARCH__
+    return __funnelshift_r(lo, hi, s);
+#else
+    s &= 31;
+    return s ? (lo >> s) | (hi << (32 - s)) : lo;
 #endif
 }
 // Position of the highest set bit, -1 for 0; of the highest bit that differs
@@ -333,23 +342,29 @@ LBM_HD Moments moments(const uint64_t F[9], bool force, double hFx, double hFy, 
     return q;
 }
 
-// -omega (f - f_eq) for f_eq = (w rho) * bracket, both operations rounded as
-// collide_exact rounds them. Br: the bracket, LSB 2^-62, 53 significant bits;
-// wr: w_1 rho, LSB 2^-(65 + sb); n = sb, 2 + sb, 4 + sb for w_0 = 4 w_1, w_1
-// and w_5 = w_1 / 4 (exact in FP64: powers of two apart).
-// big collects the high words of |f - f_eq|, to be below 2^20 (2^-9).
-LBM_HD double relax(uint64_t F, uint64_t wr, uint32_t n, uint64_t Br, double om, double om_m9, uint32_t &big) {
+// f - f_eq for f_eq = (w rho) * bracket, as sign (bit 63) and magnitude of LSB
+// 2^-61, exact. Br: the bracket, LSB 2^-62, 53 significant bits; wr: w_1 rho, LSB
+// 2^-(65 + sb); n = sb, 2 + sb, 4 + sb for w_0 = 4 w_1, w_1 and w_5 = w_1 / 4
+// (exact in FP64: powers of two apart). big and low collect the magnitudes'
+// words.
+LBM_HD uint64_t excess(uint64_t F, uint64_t wr, uint32_t n, uint64_t Br, uint32_t &big, uint32_t &low) {
     // f_eq: product rounded to 53 bits, then to LSB 2^-61 (exact: f_eq >= 2^-8)
-    const uint64_t feq = shr(round53(mul_high_sticky(wr, Br)), n);
-    const uint64_t d = F - feq;
-    const bool neg = (int32_t)hi32(d) < 0;
-    const uint64_t a = neg ? 0ull - d : d;  // |f - f_eq|, exact
+    const uint64_t d = F - shr(round53(mul_high_sticky(wr, Br)), n);
+    const uint64_t a = (int32_t)hi32(d) < 0 ? 0ull - d : d;
     big |= hi32(a);
-    // 2^-9 + |f - f_eq| is the FP64 number with these mantissa bits
-    const double m = make_double(lo32(a), hi32(a) | ((1023u - 9u) << 20));
-    const double g = fma(om, m, om_m9);  // omega |f - f_eq|, rounded once
-    const W2 w = words(g);
-    return make_double(w.lo, neg ? w.hi : w.hi ^ 0x80000000u);
+    low |= lo32(a);
+    return u64(lo32(a), hi32(a) | (hi32(d) & 0x80000000u));
+}
+
+// -omega (f - f_eq), one rounding: 2^(s-9) + |f - f_eq| is the FP64 number whose
+// mantissa is the magnitude (its low s bits, which are zero, dropped), and
+// omega times that minus omega 2^(s-9) is exact but for the multiply-add's own
+// rounding. om_m = -omega 2^(s-9).
+LBM_HD double relax(uint64_t x, uint32_t s, double om, double om_m) {
+    const uint32_t h = hi32(x) & 0x7FFFFFFFu;
+    const double m = make_double(shr_wide(lo32(x), h, s), (h >> s) | ((1023u - 9u + s) << 20));
+    const W2 w = words(fma(om, m, om_m));
+    return make_double(w.lo, w.hi ^ (~hi32(x) & 0x80000000u));
 }
 
 // One node: moments, then (COLLIDE) the collided populations in f. Returns
@@ -377,16 +392,14 @@ LBM_HD bool step_node(double f[9], const double w[9], bool force, double hFx, do
     const uint64_t kNinth = 0xE38E38E38E38E000ull;  // the FP64 number 1/9, LSB 2^-67
     const uint64_t wr = round53(mul_high_sticky(kNinth, q.D << 1));
     const Num tn = num_of(mul(1.5, add(mul(ux, ux), mul(uy, uy))));
-    uint32_t far = 0, big = 0;
+    uint32_t far = 0, big = 0, low = 0;
     const uint64_t T = shr_sticky(tn.m, tn.e - 62u);
     const uint64_t one = 1ull << 62;
-    // -omega 2^-9, exact
-    const double om_m9 = make_double(words(om).lo, words(om).hi + 0x80000000u - (9u << 20));
     const Num c[4] = {q.ux, q.uy, num_of(add(ux, uy)), num_of(add(uy, -ux))};
-    double r[9];
+    uint64_t x[9];
     // For |c.u| < 1/4 every bracket is above 1/4.
     const uint64_t b0 = round_low(one - T, 9);  // 3/4 < 1 - T <= 1
-    r[0] = relax(F[0], wr, q.sb, b0, om, om_m9, big);
+    x[0] = excess(F[0], wr, q.sb, b0, big, low);
 #pragma unroll
     for (int i = 0; i < 4; i++) {
         const int ka = i < 2 ? 1 + i : 3 + i, kb = ka + 2;  // (1,3) (2,4) (5,7) (6,8)
@@ -401,10 +414,17 @@ LBM_HD bool step_node(double f[9], const double w[9], bool force, double hFx, do
         far |= hi32(p2);
         const uint64_t p3 = round53(p2 - T), m3 = round53(round53(round53(one - B) + A) - T);
         const uint64_t bp = neg ? m3 : p3, bm = neg ? p3 : m3;
-        r[ka] = relax(F[ka], wr, (i < 2 ? 2u : 4u) + q.sb, bp, om, om_m9, big);
-        r[kb] = relax(F[kb], wr, (i < 2 ? 2u : 4u) + q.sb, bm, om, om_m9, big);
+        x[ka] = excess(F[ka], wr, (i < 2 ? 2u : 4u) + q.sb, bp, big, low);
+        x[kb] = excess(F[kb], wr, (i < 2 ? 2u : 4u) + q.sb, bm, big, low);
     }
-    if ((big >> 20) || (far >> 31)) return false;
+    // Below 2^-9 as they are; below 2^-6 without their low three bits, which are
+    // zero when f and f_eq are 2^-6 or more.
+    const uint32_t sh = big >> 20 ? 3u : 0u;
+    if ((big >> 23) || (sh && (low & 7u)) || (far >> 31)) return false;
+    const double om_m = make_double(words(om).lo, words(om).hi + 0x80000000u - ((9u - sh) << 20));
+    double r[9];
+#pragma unroll
+    for (int k = 0; k < 9; k++) r[k] = relax(x[k], sh, om, om_m);
     if (!force) {
 #pragma unroll
         for (int k = 0; k < 9; k++) f[k] = add(f[k], r[k]);

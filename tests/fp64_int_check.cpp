@@ -38,8 +38,8 @@ int main(int argc, char **argv) {
     std::uniform_real_distribution<double> U(-1, 1);
     long wrong = 0, refused = 0;
     for (long i = 0; i < n; i++) {
-        // speeds up to 0.2 (some past the range), non-equilibrium from 1e-17 to 1e-3
-        const double amp = std::pow(10.0, -0.7 - 8 * (U(gen) + 1)), ne = std::pow(10.0, -3 - 7 * (U(gen) + 1));
+        // speeds up to 0.2 (some past the range), non-equilibrium from 1e-15 to 0.03
+        const double amp = std::pow(10.0, -0.7 - 8 * (U(gen) + 1)), ne = std::pow(10.0, -1.5 - 7 * (U(gen) + 1));
         double ux = amp * U(gen), uy = amp * U(gen);
         if (i % 17 == 0) uy = 0;
         if (i % 19 == 0) ux = 0;
