@@ -1447,7 +1447,11 @@ int Solver::multi_warps() const {
 // nodes and the Boundary list in buffers 2 and 3, on a stream of their own
 // beside the pass kernel. multi_swap moves what lbc's two buffers keep in solid
 // nodes and off-grid slots between the buffers' roles.
-void Solver::near_plan(int lv, NearPlan &plan) const {
+// Kept per case: a server builds a batch anew whenever a request joins or leaves.
+const NearPlan &Solver::near_plan(int lv) const {
+    if (near_plan_.lv == lv) return near_plan_;
+    NearPlan &plan = near_plan_;
+    plan.lv = lv;
     const int Nx = d_.Nx, Ny = d_.Ny;
     // Distance to the nearest special node (the larger of |dx|, |dy|), up to m,
     // by runs of special nodes along a row.
@@ -1513,6 +1517,7 @@ void Solver::near_plan(int lv, NearPlan &plan) const {
                 }
         }
     }
+    return plan;
 }
 
 bool Solver::multi_buffers(int lv) {
@@ -1554,8 +1559,7 @@ bool Solver::multi_setup() {
         if (st.kind == BC_PERIODIC_X || st.kind == BC_PERIODIC_Y) return false;
     size_t freeb = 0, total = 0;
     if (cudaMemGetInfo(&freeb, &total) != cudaSuccess || freeb / 4 < (size_t)(lv > 2 ? 2 : 1) * multi_bytes()) return false;
-    NearPlan plan;
-    near_plan(lv, plan);
+    const NearPlan &plan = near_plan(lv);
     // With much of the grid near walls the lists outweigh the pass (channel 16384 x
     // 64, 16 % near: 12.9 us one step at a time, 13.7 in passes; 32768 x 64 27.8
     // and 22.0).
@@ -2136,8 +2140,7 @@ bool Batch::multi_setup() {
     long long near = 0;
     const int halo = multi_halo(lv), width = 64 - 2 * halo;
     for (size_t c = 0; c < cases_.size(); c++) {
-        NearPlan plan;
-        cases_[c]->near_plan(lv, plan);
+        const NearPlan &plan = cases_[c]->near_plan(lv);
         near += 2 * plan.near_pairs;
         for (int q = 0; q < lv; q++)
             for (int4 e : plan.segs[q]) segs[q].push_back(make_int4((int)c, e.y, e.z, e.w));

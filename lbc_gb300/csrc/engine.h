@@ -97,6 +97,7 @@ constexpr int kMaxProbes = 4096;
 
 // A case's nodes near special ones in passes of several steps (near_plan).
 struct NearPlan {
+    int lv = 0;
     std::vector<uint32_t> deep;
     std::vector<std::vector<int4>> segs;
     long long near_pairs = 0;
@@ -249,7 +250,7 @@ class Solver {
     }
     bool wide() const { return 9LL * plane_ >= (1LL << 31); }  // element offsets need 64 bits
     size_t multi_bytes() const { return 9 * (size_t)plane_ * esize_; }  // of one of its buffers
-    void near_plan(int lv, NearPlan &plan) const;
+    const NearPlan &near_plan(int lv) const;
     bool multi_buffers(int lv);
     bool swap_multi(bool enter, int lv, cudaStream_t s);
     StepParams near_params(int cur, int other, int lv, int q) const;
@@ -339,6 +340,7 @@ class Solver {
     cudaGraphExec_t multi_exec_ = nullptr;
     int multi_cur_ = -1, multi_parity_ = -1;
     bool graph_valid_multi_ = false;
+    mutable NearPlan near_plan_;
     int multi_state_ = 0;                 // 0: not tried, 1: set up, -1: not for this case
     uint32_t *d_deep_ = nullptr;
     int4 *d_near_segs_[4] = {nullptr, nullptr, nullptr, nullptr};
