@@ -538,9 +538,25 @@ bool Solver::group_stages(const Solid &solid, const std::vector<int> &colbase, c
         gw.insert(w.begin(), w.end());
         gr.insert(r.begin(), r.end());
     }
-    // (periodic entries read post-collision values of the opposite edge)
+    // Edges that pull their node themselves (near_shifted, edges_exact): not
+    // with periodic entries, which read post-collision values of the opposite
+    // edge, nor where an entry's interior neighbour keeps a slot from two steps
+    // before (a source off the grid): the step overwrites it meanwhile. The
+    // entry's own node is its thread's alone, and solid nodes are never written.
     one_group_ = groups_.size() <= 1;
-    for (const Stage &st : stages_) one_group_ = one_group_ && st.kind != BC_PERIODIC_X && st.kind != BC_PERIODIC_Y;
+    for (const Stage &st : stages_) {
+        if (st.kind == BC_PERIODIC_X || st.kind == BC_PERIODIC_Y) {
+            one_group_ = false;
+            continue;
+        }
+        if (!edge_reads_neighbour(st.kind)) continue;
+        for (int t = 0; t < st.along && one_group_; t++) {
+            const int2 at = bc_is_column(st.kind) ? make_int2(st.index, t) : make_int2(t, st.index);
+            const int2 n = stage_neighbour(st.kind, at);
+            if (solid(at.x, at.y) || solid(n.x, n.y)) continue;
+            if ((!d_.px && (n.x == 0 || n.x == Nx - 1)) || (!d_.py && (n.y == 0 || n.y == Ny - 1))) one_group_ = false;
+        }
+    }
     return true;
 }
 

@@ -64,6 +64,14 @@ def _walls(name):
         return cases.cavity_moving_wall(1450, 0.1, 300.0), None
     if name == "box":
         return cases.all_regularized_box(600, 450), None
+    if name == "open":  # inlet and outlet between open rows: neighbours with slots of their own
+        case, st = cases.cylinder_wake(900, 400, D=40.0, xc=300.0, yc=200.0, u_max=0.05, Re=60.0)
+        case.solid_mask[0] = case.solid_mask[-1] = 0
+        return (case, st), None
+    if name == "boxblock":  # several groups of edges around a body
+        case, st = cases.all_regularized_box(610, 450)
+        case.solid_mask[200:240, 300:360] = 1
+        return (case, st), None
     if name == "golden":
         return cases.cylinder_golden(17)[:2], None
     if name == "blocks":  # obstacles across both periodic edges, body force
@@ -77,7 +85,8 @@ def _walls(name):
 
 
 @pytest.mark.parametrize("storage", ["f32", "f16"])
-@pytest.mark.parametrize("name", ["wake", "wake4", "cavity", "cavity4", "box", "golden", "blocks", "duct"])
+@pytest.mark.parametrize("name", ["wake", "wake4", "cavity", "cavity4", "box", "boxblock", "open", "golden", "blocks",
+                                  "duct"])
 def test_walls_and_edges_match_single_steps(storage, name):
     """Cases with a flag word: cut links, moving walls, Zou-He, convective,
     regularized and impedance edges, slots off open edges, odd sizes, with and
