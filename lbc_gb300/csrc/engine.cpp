@@ -120,6 +120,7 @@ Solver::~Solver() {
     if (h_vtk_) cudaFreeHost(h_vtk_);
     if (pair_exec_) cudaGraphExecDestroy(pair_exec_);
     if (multi_exec_) cudaGraphExecDestroy(multi_exec_);
+    if (beside_ev_) cudaEventDestroy(beside_ev_);
     if (multi_fork_) cudaEventDestroy(multi_fork_);
     if (multi_join_) cudaEventDestroy(multi_join_);
     if (multi_stream_) cudaStreamDestroy(multi_stream_);
@@ -1092,10 +1093,11 @@ bool Solver::launch_step_kernels(int src, int dst, bool collide, bool write_macr
         // A Boundary list of one group goes first and the bulk kernel beside it.
         const bool edges = collide && !write_macro && one_group_ && !groups_.empty();
         if (edges) CK(launch::edges_exact(p, stage_group(0, src, dst, write_macro, bparity, false), arith_, s));
+        if (edges && !beside(s)) return false;
         CK(launch::step_exact(p, has_flags_, collide, block_, s, arith_, edges));
         if (edges) {
-            if (forces) CK(launch::force_reduce(d_force_slot_, 1, true, s));
-            return true;
+            if (forces) CK(launch::force_reduce(d_force_slot_, 1, true, s));  // (reads the bulk kernel's alone)
+            return join(s);
         }
     } else {
         const FastStepParams fp = fast_params(p);
@@ -1103,7 +1105,7 @@ bool Solver::launch_step_kernels(int src, int dst, bool collide, bool write_macr
         // as its programmatic follower: the grid of clean-pair blocks fills the
         // SMs around the special nodes' latency-bound blocks from the start
         // (the plain kernel of a flag-free grid steps its own odd column).
-        // What follows is an ordinary launch, so it sees both. A Boundary list
+        // What follows is an ordinary launch behind both. A Boundary list
         // of one group steps with the special nodes (near_shifted).
         const bool near = collide && !write_macro && special_launch() && one_group_ && !groups_.empty() && !wide();
         if (near)
@@ -1111,13 +1113,27 @@ bool Solver::launch_step_kernels(int src, int dst, bool collide, bool write_macr
                                     stage_group(0, src, dst, write_macro, bparity, false), false, s));
         else if (special_launch())
             CK(launch::special_shifted(fp, d_special_, nspecial_, d_.store, true, collide, false, s));
+        if (special_launch() && !beside(s)) return false;
         CK(launch::step_shifted(fp, d_.store, has_flags_, collide, block_, s, special_launch()));
+        if (special_launch() && !join(s)) return false;
         if (near) {
             if (forces) CK(launch::force_reduce(d_force_slot_, 1, false, s));
             return true;
         }
     }
     return launch_edges(src, dst, collide, write_macro, bparity, forces, d_.store == STORE_F64, s);
+}
+
+// In a captured graph: the kernel just launched on s runs beside its programmatic
+// follower, and what is launched after join(s) waits for both (pdl.cuh).
+bool Solver::beside(cudaStream_t s) {
+    if (capturing_) CK(cudaEventRecord(beside_ev_, s));
+    return true;
+}
+
+bool Solver::join(cudaStream_t s) {
+    if (capturing_) CK(cudaStreamWaitEvent(s, beside_ev_, 0));
+    return true;
 }
 
 // The Boundary list's launches of a step and its wall force, behind the kernels
@@ -1357,11 +1373,14 @@ bool Solver::capture_pair() {
         cudaGraphExecDestroy(pair_exec_);
         pair_exec_ = nullptr;
     }
+    if (!beside_ev_) CK(cudaEventCreateWithFlags(&beside_ev_, cudaEventDisableTiming));
     cudaGraph_t g = nullptr;
     CK(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
     bool okk = true;
+    capturing_ = true;
     for (int q = 0; q < kGraphPairs && okk; q++)
         okk = launch_step(cur_, 1 - cur_, true, false, parity_) && launch_step(1 - cur_, cur_, true, false, parity_ ^ 1);
+    capturing_ = false;
     cudaError_t e = cudaStreamEndCapture(stream_, &g);
     if (!okk) {
         if (g) cudaGraphDestroy(g);

@@ -279,6 +279,8 @@ class Solver {
     int nprobes_ = 0, probe_cap_ = 0;
     bool launch_collide(int b, cudaStream_t s = nullptr);
     bool capture_pair();
+    bool beside(cudaStream_t s);
+    bool join(cudaStream_t s);
     int multi_warps() const;
     bool multi_setup();
     bool launch_multi(int cur, int other, int lv);
@@ -337,6 +339,8 @@ class Solver {
     cudaGraphExec_t pair_exec_ = nullptr;
     int pair_cur_ = -1, pair_parity_ = -1;
     bool graph_valid_ = false;
+    bool capturing_ = false;
+    cudaEvent_t beside_ev_ = nullptr;
     cudaGraphExec_t multi_exec_ = nullptr;
     int multi_cur_ = -1, multi_parity_ = -1;
     bool graph_valid_multi_ = false;

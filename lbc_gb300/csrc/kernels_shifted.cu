@@ -90,7 +90,8 @@ __global__ void __launch_bounds__(256, 5) k_step_shifted_geo(const FastStepParam
 // It reads and writes nothing the clean-pair kernel touches: a case alone
 // launches it first, as an ordinary launch, with the clean pairs as its
 // programmatic follower (pdl.cuh), so their blocks fill the SMs around its
-// latency-bound ones; the launch after both is ordinary. (The trigger at the
+// latency-bound ones; the launch after both is ordinary and, in a graph, has an
+// edge from each (Solver::join). (The trigger at the
 // start lets the follower launch at once; the wait at the end is then a
 // no-op.)
 template <typename T, typename I, bool FLAGS, bool COLLIDE, bool FORCE, bool LINKS>

@@ -11,6 +11,14 @@
 // its writes are visible) before it reads or writes anything that kernel
 // touches. A kernel launched without the attribute passes through both
 // instructions unaffected.
+//
+// A follower that touches nothing of the kernel before it (the bulk kernel beside
+// the edges or special nodes launched first) does not wait and may complete
+// first. In a stream an ordinary launch comes after both all the same; in a
+// captured graph its only edge would come from the follower, so the capture adds
+// one from the kernel before (Solver::beside, Solver::join). (The follower's first
+// block waiting at its end orders them too: lid 129 x 129 FP32 4.25 us per step
+// against 3.80, the second completion in the chain.)
 #pragma once
 #include <cuda_runtime.h>
 
