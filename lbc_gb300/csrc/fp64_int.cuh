@@ -249,9 +249,29 @@ LBM_HD double from_fixed(uint64_t v, int lsb) {
 }
 // 1/d for d = D 2^-63 in [1/2, 1), as an integer of LSB 2^-63, below the true
 // value by less than 8 units: the FP32 reciprocal, then two Newton steps.
-LBM_HD uint64_t recip_fixed(uint64_t D) {
+// The FP32 number that stands for d: above d's first 24 bits by 3 2^-24 at most,
+// and so far above 1/2 that a reciprocal 2^-23 off (the bound of rcp.approx) is
+// below 2.
+LBM_HD uint32_t recip_arg(uint64_t D) {
+    return 0x3F000000u | (hi32(D << 1) >> 8 & 0x7FFFFFu) | 3u;
+}
+// yb: the bits of its reciprocal, between 1 - 2^-24 and 2.
+LBM_HD uint64_t recip_refine(uint64_t D, uint32_t yb) {
     const uint32_t dh = hi32(D) << 1 | lo32(D) >> 31, dl = lo32(D) << 1;  // LSB 2^-64
-    const uint32_t db = 0x3F000000u | ((dh >> 8) & 0x7FFFFFu) | 1u;      // above 1/2: 1/d < 2
+    // LSB 2^-31: the exponent's last bit is 2^31; 1 - 2^-24 (exponent one less,
+    // mantissa of ones) gives 2^31 - 2^8 of its own accord
+    const uint32_t y0 = yb << 8;
+    // e = 1 - d y0, |e| < 2^-20, LSB 2^-63
+    const uint64_t t = (uint64_t)dh * y0 + (((uint64_t)dl * y0) >> 32);
+    const int32_t e0 = (int32_t)((int64_t)(0x8000000000000000ull - t) >> 11);  // LSB 2^-52
+    const uint64_t y1 = ((uint64_t)y0 << 32) + (uint64_t)(((int64_t)e0 * (int64_t)(y0 >> 1)) >> 19);
+    // |1 - d y1| < 2^-40
+    const int32_t e1 = (int32_t)(uint32_t)(0x8000000000000000ull - mul_high(u64(dl, dh), y1));
+    // 4 units off keep 1/d = 2 inside 64 bits
+    return y1 + (uint64_t)(((int64_t)e1 * (int64_t)(hi32(y1) >> 1)) >> 30) - 4u;
+}
+LBM_HD uint64_t recip_fixed(uint64_t D) {
+    const uint32_t db = recip_arg(D);
     uint32_t yb;
 #ifdef __CUDA_ARCH__
     float y;
@@ -263,15 +283,7 @@ LBM_HD uint64_t recip_fixed(uint64_t D) {
     y = 1.0f / df;
     std::memcpy(&yb, &y, 4);
 #endif
-    const uint32_t y0 = (yb << 8) | 0x80000000u;  // LSB 2^-31
-    // e = 1 - d y0, |e| < 2^-20, LSB 2^-63
-    const uint64_t t = (uint64_t)dh * y0 + (((uint64_t)dl * y0) >> 32);
-    const int32_t e0 = (int32_t)((int64_t)(0x8000000000000000ull - t) >> 11);  // LSB 2^-52
-    const uint64_t y1 = ((uint64_t)y0 << 32) + (uint64_t)(((int64_t)e0 * (int64_t)(y0 >> 1)) >> 19);
-    // |1 - d y1| < 2^-40
-    const int32_t e1 = (int32_t)(uint32_t)(0x8000000000000000ull - mul_high(u64(dl, dh), y1));
-    // 4 units off keep 1/d = 2 inside 64 bits
-    return y1 + (uint64_t)(((int64_t)e1 * (int64_t)(hi32(y1) >> 1)) >> 30) - 4u;
+    return recip_refine(D, yb);
 }
 
 // a / d rounded to FP64 for a of at most 53 significant bits and d = D 2^-63
