@@ -102,10 +102,12 @@ Solver::Solver(const CaseDesc &d) : d_(d) {
     // The integer form of the FP64 step has no use for large blocks: 64 x 2
     // packs the most warps on an SM (1024^2: 74.5 us per step with 64 x 4,
     // 72.8 with 64 x 2). A grid of at most a warp per SM sub-partition takes
-    // one-warp blocks, so that no two of its warps share one.
+    // one-warp blocks, so that no two of its warps share one; a grid of more rows
+    // than a launch of 64 x 2 blocks reaches keeps 64 x 4.
     if (arith_ == ARITH_INT) {
         const long long warps = (long long)((d_.Nx + 31) / 32) * d_.Ny;
-        block_ = warps <= 4LL * launch::sm_count() ? dim3(32, 1, 1) : dim3(64, 2, 1);
+        if (warps <= 4LL * launch::sm_count()) block_ = dim3(32, 1, 1);
+        else if (block_reaches(2)) block_ = dim3(64, 2, 1);
     }
     // (a failure here shows at the launch)
     if (multi_levels() > 0 && launch::multi_load(d_.store, multi_levels(), !has_flags_, has_force()) != cudaSuccess)
@@ -1712,7 +1714,11 @@ static const int kNBlockCand = 7;
 // (after two steps that estimate K) and keeps the fastest. Returns the number
 // of steps taken (all of them steps of the run), or -1 on a CUDA error.
 int Solver::tune_online(int avail) {
-    const int nc = kNBlockCand;
+    std::vector<dim3> cand;
+    for (const int *b : kBlockCand)
+        if (block_reaches(b[1])) cand.push_back(dim3(b[0], b[1], 1));
+    const int nc = (int)cand.size();
+    if (nc == 0) return 0;
     WindowTimer est(1);
     if (!est.ok()) return -1;
     if (!est.mark(0, stream_) || !trial_step() || !trial_step() || !est.mark(1, stream_) || !est.wait()) return -1;
@@ -1725,7 +1731,7 @@ int Solver::tune_online(int avail) {
     for (int r = 0; r < 2; r++)
         for (int c = 0; c < nc; c++) {
             if (!wt.mark(r * nc + c, stream_)) return -1;
-            set_block(dim3(kBlockCand[c][0], kBlockCand[c][1], 1));
+            set_block(cand[c]);
             for (int k = 0; k < K; k++)
                 if (!trial_step()) return -1;
         }
@@ -1737,10 +1743,10 @@ int Solver::tune_online(int avail) {
         const float ms = std::min(wt.elapsed(c), wt.elapsed(nc + c));
         if (best < 0 || ms < best_ms) { best = c; best_ms = ms; }
     }
-    set_block(dim3(kBlockCand[best][0], kBlockCand[best][1], 1));
+    set_block(cand[best]);
     tuned_ = true;
     tuned_us_ = best_ms * 1e3f / K;
-    tune_store(tune_key(), kBlockCand[best][0], kBlockCand[best][1], tuned_us_);
+    tune_store(tune_key(), (int)cand[best].x, (int)cand[best].y, tuned_us_);
     return used;
 }
 

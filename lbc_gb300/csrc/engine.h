@@ -287,6 +287,8 @@ class Solver {
     bool capture_multi();
     int run_multi(int avail);
     bool trial_step();
+    // A launch of the fused step in blocks of `by` rows reaches every row.
+    bool block_reaches(int by) const { return (d_.Ny + by - 1) / by <= 65535; }
     int tune_online(int avail);
     int tune_mode_ = 0;
     bool tuned_ = false;
