@@ -35,7 +35,7 @@ __device__ __forceinline__ void pull_node(const StepParams &p, int i, int j, flo
     const int so[9] = {r0 + i, r0 + im, rm + i, r0 + ip, rp + i, rm + im, rm + ip, rp + ip, rp + im};
     const uint16_t fl = p.flags[node];
 #pragma unroll
-    for (int k = 0; k < 9; k++) g[k] = SV<T>::ld(S + (int)k * pl + so[k]);
+    for (int k = 0; k < 9; k++) g[k] = ld_src<T, false>(S + (int)k * pl + so[k]);
     if (!(fl & (NF_SPECIAL_MASK | NF_SOLID))) return;
     if (fl & NF_SOLID) {
 #pragma unroll
@@ -51,12 +51,12 @@ __device__ __forceinline__ void pull_node(const StepParams &p, int i, int j, flo
             g[k] = SV<T>::ld_plain(Old + (int)k * pl + node);
             continue;
         }
-        const float own = SV<T>::ld(S + (int)oppk(k) * pl + node);
+        const float own = ld_src<T, false>(S + (int)oppk(k) * pl + node);
         float val = own;
         if (lk) {
             const Link L = *lk++;
-            if (L.mode == LINK_IBB_LO) val = (float)L.c1 * own + (float)L.c2 * SV<T>::ld(S + (int)oppk(k) * pl + (int)L.behind);
-            else if (L.mode == LINK_IBB_HI) val = (float)L.c1 * own + (float)L.c2 * SV<T>::ld(S + (int)k * pl + (int)L.behind);
+            if (L.mode == LINK_IBB_LO) val = (float)L.c1 * own + (float)L.c2 * ld_src<T, false>(S + (int)oppk(k) * pl + (int)L.behind);
+            else if (L.mode == LINK_IBB_HI) val = (float)L.c1 * own + (float)L.c2 * ld_src<T, false>(S + (int)k * pl + (int)L.behind);
             else if (L.mode == LINK_MOVING) val = own - (float)L.c2;
         }
         g[k] = SV<T>::rnd(val);
@@ -126,7 +126,7 @@ __device__ __forceinline__ void step_segment(const FastStepParams &fp, int j, in
     if (p.py) { if (jm < 0) jm += p.Ny; if (jp >= p.Ny) jp -= p.Ny; }
     else { jm = max(jm, 0); jp = min(jp, p.Ny - 1); }
     float2 g[9];
-    load_pair_shifted<T, int>(p, i0, j, im, ip2, jm, jp, g);
+    load_pair_shifted<T, int, false>(p, i0, j, im, ip2, jm, jp, g);
     collide_store_pair_shifted<T, int, true, true>(fp, i0, j, g);
 }
 
@@ -161,7 +161,7 @@ __global__ void __launch_bounds__(128) k_near_shifted(const FastStepParams fp, c
     bool link = false;
     if (q < n) {
         const int2 ij = nodes[q];
-        if (!(ij.x & kSpecialSolid)) step_node_shifted<T, int, true, true, true, LINKS>(fp, ij.x, ij.y, mx, my, link);
+        if (!(ij.x & kSpecialSolid)) step_node_shifted<T, int, true, true, true, LINKS, false>(fp, ij.x, ij.y, mx, my, link);
     }
     if (fp.s.mem_partials)
         chunk_reduce2_store((double)mx, (double)my, link, q >> 5, fp.s.chunk_slot, fp.s.mem_partials);
@@ -203,8 +203,8 @@ __global__ void __launch_bounds__(128) k_near_batch_shifted(const FastStepParams
     float mx = 0.f, my = 0.f;
     bool link = false;
     if (e.y >= 0 && !(e.y & kSpecialSolid)) {
-        if (fp.s.flags) step_node_shifted<T, int, true, true, true, LINKS>(fp, e.y, e.z, mx, my, link);
-        else step_node_shifted<T, int, false, true, true, LINKS>(fp, e.y, e.z, mx, my, link);
+        if (fp.s.flags) step_node_shifted<T, int, true, true, true, LINKS, false>(fp, e.y, e.z, mx, my, link);
+        else step_node_shifted<T, int, false, true, true, LINKS, false>(fp, e.y, e.z, mx, my, link);
     }
 }
 

@@ -18,6 +18,7 @@ template <> struct SV<float> {
     static __device__ __forceinline__ void st(float *p, float v) { *p = v; }
     static __device__ __forceinline__ float rnd(float v) { return v; }
     static __device__ __forceinline__ float2 ld2(const float *p) { return __ldg((const float2 *)p); }
+    static __device__ __forceinline__ float2 ld2_plain(const float *p) { return *(const float2 *)p; }
     static __device__ __forceinline__ void st2(float *p, float2 v) { *(float2 *)p = v; }
 };
 template <> struct SV<__half> {
@@ -26,8 +27,20 @@ template <> struct SV<__half> {
     static __device__ __forceinline__ void st(__half *p, float v) { *p = __float2half_rn(v); }
     static __device__ __forceinline__ float rnd(float v) { return __half2float(__float2half_rn(v)); }
     static __device__ __forceinline__ float2 ld2(const __half *p) { return __half22float2(__ldg((const __half2 *)p)); }
+    static __device__ __forceinline__ float2 ld2_plain(const __half *p) { return __half22float2(*(const __half2 *)p); }
     static __device__ __forceinline__ void st2(__half *p, float2 v) { *(__half2 *)p = __float22half2_rn(v); }
 };
+
+// Loads of the populations a step pulls from. RO: nobody writes them while the
+// kernel's grid is resident, so the read-only path may serve them. Not so in a
+// chain of programmatic followers (kernels_near.cu), whose grid is resident while
+// the one before it still writes what it reads after pdl_wait().
+template <typename T, bool RO> __device__ __forceinline__ float ld_src(const T *p) {
+    return RO ? SV<T>::ld(p) : SV<T>::ld_plain(p);
+}
+template <typename T, bool RO> __device__ __forceinline__ float2 ld2_src(const T *p) {
+    return RO ? SV<T>::ld2(p) : SV<T>::ld2_plain(p);
+}
 
 // ---------------------------------------------------------------- lane math
 // The arithmetic of one node (float) or of two adjacent nodes at once (float2,

@@ -74,7 +74,7 @@ static __device__ __noinline__ float2 omega_pair(const double *omega, size_t dn)
 // records (plain bounce-back on every solid link), and the record path is
 // left out (measured: 116 -> 64 registers for the batched special-node
 // kernel, twice the resident warps).
-template <typename T, typename I, bool FLAGS, bool COLLIDE, bool FORCE, bool LINKS = true>
+template <typename T, typename I, bool FLAGS, bool COLLIDE, bool FORCE, bool LINKS = true, bool RO = true>
 __device__ __forceinline__ void step_node_shifted(const FastStepParams &fp, int i, int j,
                                                   float &mfx, float &mfy, bool &link) {
     const StepParams &p = fp.s;
@@ -104,13 +104,13 @@ __device__ __forceinline__ void step_node_shifted(const FastStepParams &fp, int 
     const uint16_t fl = FLAGS ? p.flags[node] : (uint16_t)0;
     float g[9];
 #pragma unroll
-    for (int k = 0; k < 9; k++) g[k] = SV<T>::ld(S + (I)k * pl + so[k]);
+    for (int k = 0; k < 9; k++) g[k] = ld_src<T, RO>(S + (I)k * pl + so[k]);
     int lo = 0, cb = -1, rb = -1;
     float own[9];
     bool off[9];
     if (FLAGS) {
 #pragma unroll
-        for (int k = 1; k < 9; k++) own[k] = SV<T>::ld(S + (I)oppk(k) * pl + node);
+        for (int k = 1; k < 9; k++) own[k] = ld_src<T, RO>(S + (I)oppk(k) * pl + node);
         if (LINKS && p.link_off) lo = p.link_off[node];
         // Without cut-link records, also the band bases and the stale slots
         // of off-grid sources (this node's own destination slots, written by
@@ -154,8 +154,8 @@ __device__ __forceinline__ void step_node_shifted(const FastStepParams &fp, int 
             if (off[k]) {
                 if (LINKS) g[k] = SV<T>::ld_plain(Old + (I)k * pl + node);
             } else if (has_links) {
-                if (L[k].mode == LINK_IBB_LO) behind[k] = SV<T>::ld(S + (I)oppk(k) * pl + (I)L[k].behind);
-                else if (L[k].mode == LINK_IBB_HI) behind[k] = SV<T>::ld(S + (I)k * pl + (I)L[k].behind);
+                if (L[k].mode == LINK_IBB_LO) behind[k] = ld_src<T, RO>(S + (I)oppk(k) * pl + (I)L[k].behind);
+                else if (L[k].mode == LINK_IBB_HI) behind[k] = ld_src<T, RO>(S + (I)k * pl + (I)L[k].behind);
             }
         }
 #pragma unroll
@@ -199,7 +199,7 @@ __device__ __forceinline__ void step_node_shifted(const FastStepParams &fp, int 
 // FP32 arithmetic, pair stores. im = source column of i0 - 1, ip2 of i0 + 2
 // (wrapped or clamped like the per-node path), so every load is in bounds
 // whatever the nodes' flags say.
-template <typename T, typename I>
+template <typename T, typename I, bool RO = true>
 __device__ __forceinline__ void load_pair_shifted(const StepParams &p, int i0, int j, int im, int ip2, int jm,
                                                   int jp, float2 g[9]) {
     const T *S = (const T *)p.src;
@@ -207,21 +207,21 @@ __device__ __forceinline__ void load_pair_shifted(const StepParams &p, int i0, i
     const I r0 = (I)j * (I)p.pitch + (I)i0, rm = (I)jm * (I)p.pitch, rp = (I)jp * (I)p.pitch;
     const I m0 = rm + (I)i0, p0 = rp + (I)i0;
     float2 a;
-    g[0] = SV<T>::ld2(S + r0);
-    a = SV<T>::ld2(S + pl + r0);
-    g[1] = make_float2(SV<T>::ld(S + pl + (r0 - (I)i0 + (I)im)), a.x);
-    g[2] = SV<T>::ld2(S + 2 * pl + m0);
-    a = SV<T>::ld2(S + 3 * pl + r0);
-    g[3] = make_float2(a.y, SV<T>::ld(S + 3 * pl + (r0 - (I)i0 + (I)ip2)));
-    g[4] = SV<T>::ld2(S + 4 * pl + p0);
-    a = SV<T>::ld2(S + 5 * pl + m0);
-    g[5] = make_float2(SV<T>::ld(S + 5 * pl + rm + (I)im), a.x);
-    a = SV<T>::ld2(S + 6 * pl + m0);
-    g[6] = make_float2(a.y, SV<T>::ld(S + 6 * pl + rm + (I)ip2));
-    a = SV<T>::ld2(S + 7 * pl + p0);
-    g[7] = make_float2(a.y, SV<T>::ld(S + 7 * pl + rp + (I)ip2));
-    a = SV<T>::ld2(S + 8 * pl + p0);
-    g[8] = make_float2(SV<T>::ld(S + 8 * pl + rp + (I)im), a.x);
+    g[0] = ld2_src<T, RO>(S + r0);
+    a = ld2_src<T, RO>(S + pl + r0);
+    g[1] = make_float2(ld_src<T, RO>(S + pl + (r0 - (I)i0 + (I)im)), a.x);
+    g[2] = ld2_src<T, RO>(S + 2 * pl + m0);
+    a = ld2_src<T, RO>(S + 3 * pl + r0);
+    g[3] = make_float2(a.y, ld_src<T, RO>(S + 3 * pl + (r0 - (I)i0 + (I)ip2)));
+    g[4] = ld2_src<T, RO>(S + 4 * pl + p0);
+    a = ld2_src<T, RO>(S + 5 * pl + m0);
+    g[5] = make_float2(ld_src<T, RO>(S + 5 * pl + rm + (I)im), a.x);
+    a = ld2_src<T, RO>(S + 6 * pl + m0);
+    g[6] = make_float2(a.y, ld_src<T, RO>(S + 6 * pl + rm + (I)ip2));
+    a = ld2_src<T, RO>(S + 7 * pl + p0);
+    g[7] = make_float2(a.y, ld_src<T, RO>(S + 7 * pl + rp + (I)ip2));
+    a = ld2_src<T, RO>(S + 8 * pl + p0);
+    g[8] = make_float2(ld_src<T, RO>(S + 8 * pl + rp + (I)im), a.x);
 }
 
 template <typename T, typename I, bool COLLIDE, bool FORCE>

@@ -54,3 +54,26 @@ def test_steps_wait_for_their_edges(oracle, name, storage, hist):
         oracle.run(case, st, steps)
         for fld in FIELDS:
             assert same(getattr(states[0], fld), getattr(st, fld)), fld
+
+
+@pytest.mark.parametrize("storage", ["f32", "f16"])
+def test_chained_steps_of_a_pass_see_each_other(storage):
+    """The lists beside a pass follow each other while the one before still
+    runs: buffer 2 is read by step 2 of a pass, written by step 3 and read
+    again by step 4. Many passes against steps taken one by one."""
+    from lbc_gb300 import GpuSolver, STORAGE
+    case, _ = cases.cylinder_wake(3400, 620, D=90.0, xc=500.0, yc=310.0, u_max=0.05, Re=80.0)
+    st = cases.random_state(case, 4)
+    a, b = (GpuSolver(case, STORAGE[storage]) for _ in range(2))
+    for s in (a, b):
+        s.set_state(st)
+    for n in (513, 1, 1286):
+        a.run(n)
+    for _ in range(1800):
+        b.run(1)
+    x, y = a.get_state(), b.get_state()
+    for fld in FIELDS:
+        assert same(getattr(x, fld), getattr(y, fld)), fld
+    assert a.forces() == b.forces()
+    a.close()
+    b.close()
