@@ -191,12 +191,11 @@ __global__ void k_collide_shifted(const CollideParams p) {
 #pragma unroll
     for (int k = 0; k < 9; k++) { g[k] = SV<T>::ld_plain(F + k * p.plane + node); wf[k] = (float)p.w[k]; }
     const float om = p.omega ? (float)p.omega[dn] : (float)p.omega0;
-    float dr, rho, ux, uy, Jx, Jy, jx, jy;
+    float dr, ux, uy, Jx, Jy, jx, jy;
     if (p.from_pops) {
-        moments_shifted(g, (float)(0.5 * p.Fx), (float)(0.5 * p.Fy), dr, rho, ux, uy, Jx, Jy, jx, jy);
+        moments_shifted(g, (float)(0.5 * p.Fx), (float)(0.5 * p.Fy), dr, ux, uy, Jx, Jy, jx, jy);
     } else {
         // the stored fields: rho, u = (j + F/2) / rho
-        rho = (float)p.rho[dn];
         dr = (float)(p.rho[dn] - 1.0);
         ux = (float)p.ux[dn];
         uy = (float)p.uy[dn];

@@ -51,24 +51,20 @@ __device__ __forceinline__ float v_add(float a, float b) { return __fadd_rn(a, b
 __device__ __forceinline__ float v_sub(float a, float b) { return __fsub_rn(a, b); }
 __device__ __forceinline__ float v_mul(float a, float b) { return __fmul_rn(a, b); }
 __device__ __forceinline__ float v_fma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
-// 1/a correctly rounded for 2^-126 <= a <= 2^125: the hardware's estimate and
-// one Newton step (checked against __frcp_rn on every float of that range; the
-// intrinsic itself has a branch, which keeps the compiler from interleaving the
-// steps of kernels_multi.cu).
+// The hardware's estimate of 1/a, a >= 2^-126, and max and min that keep a NaN.
 __device__ __forceinline__ float v_rcp_seed(float a) {
     float r;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a));
     return r;
 }
-__device__ __forceinline__ float v_rcp(float a) {
-    const float r = v_rcp_seed(a);
-    return __fmaf_rn(r, __fmaf_rn(-a, r, 1.0f), r);
-}
-// lbc's floor on the density (compute_macroscopic_fields.c:27), and v_rcp's
-// range above; NaN stays NaN.
-__device__ __forceinline__ float v_floor_rho(float a) {
+__device__ __forceinline__ float v_max_nan(float a, float b) {
     float r;
-    asm("max.NaN.f32 %0, %1, %2;\n\tmin.NaN.f32 %0, %0, %3;" : "=&f"(r) : "f"(a), "f"(1e-16f), "f"(0x1p125f));
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ float v_min_nan(float a, float b) {
+    float r;
+    asm("min.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
     return r;
 }
 __device__ __forceinline__ float2 v_add(float2 a, float2 b) { return __fadd2_rn(a, b); }
@@ -86,14 +82,32 @@ __device__ __forceinline__ float2 v_mul_alone(float2 a, float2 b) {
     const float nz = __uint_as_float(0x80000000u + (blockDim.z - 1u));
     return __ffma2_rn(a, b, make_float2(nz, nz));
 }
-__device__ __forceinline__ float2 v_rcp(float2 a) {
-    const float2 r = make_float2(v_rcp_seed(a.x), v_rcp_seed(a.y));
-    return __ffma2_rn(r, __ffma2_rn(make_float2(-a.x, -a.y), r, make_float2(1.0f, 1.0f)), r);
+__device__ __forceinline__ float2 v_rcp_seed(float2 a) { return make_float2(v_rcp_seed(a.x), v_rcp_seed(a.y)); }
+__device__ __forceinline__ float2 v_max_nan(float2 a, float2 b) {
+    return make_float2(v_max_nan(a.x, b.x), v_max_nan(a.y, b.y));
 }
-__device__ __forceinline__ float2 v_floor_rho(float2 a) { return make_float2(v_floor_rho(a.x), v_floor_rho(a.y)); }
+__device__ __forceinline__ float2 v_min_nan(float2 a, float2 b) {
+    return make_float2(v_min_nan(a.x, b.x), v_min_nan(a.y, b.y));
+}
+__device__ __forceinline__ float2 v_neg(float2 a) { return make_float2(-a.x, -a.y); }
+__device__ __forceinline__ float v_neg(float a) { return -a; }
 template <class V> __device__ __forceinline__ V v_splat(float x);
 template <> __device__ __forceinline__ float v_splat<float>(float x) { return x; }
 template <> __device__ __forceinline__ float2 v_splat<float2>(float x) { return make_float2(x, x); }
+
+// 1/rho, rho = 1 + dr with lbc's floor (compute_macroscopic_fields.c:27), rounded
+// as __frcp_rn rounds it: the hardware's estimate and one Newton step (that
+// intrinsic has a branch, which keeps the compiler from interleaving the steps of
+// kernels_multi.cu). The estimate is of rho / 8, so that it is a normal number for
+// every finite density and 0 for an infinite one, and an eighth of it takes the
+// Newton step. Above 2^126, where 1/rho is subnormal, within 2^-149. NaN stays NaN.
+template <class V> __device__ __forceinline__ V inv_density(V dr) {
+    const V eighth = v_splat<V>(0.125f);
+    const V a = v_max_nan(v_fma(dr, eighth, eighth), v_splat<V>(0.125f * 1e-16f));
+    const V r = v_rcp_seed(a), s = v_mul(r, eighth);
+    const V e = v_fma(v_neg(v_min_nan(a, v_splat<V>(0x1p125f))), r, v_splat<V>(1.0f));
+    return v_fma(s, e, s);
+}
 
 // h1 = fl(3 w1), h5 = (1 - 2 h1) / 4, as the host computes them.
 __device__ __forceinline__ void shifted_h(float w1, float &h1, float &h5) {
@@ -104,14 +118,13 @@ __device__ __forceinline__ void shifted_h(float w1, float &h1, float &h5) {
 // Shifted moments: delta rho = sum g, j = sum c g (sum c w = 0). Jx, Jy are the
 // momentum including half the body force (rho u of lbc); jx, jy without it.
 template <class V>
-__device__ __forceinline__ void moments_v(const V g[9], V hFx, V hFy, V &dr, V &rho, V &ux, V &uy, V &Jx,
-                                          V &Jy, V &jx, V &jy) {
+__device__ __forceinline__ void moments_v(const V g[9], V hFx, V hFy, V &dr, V &ux, V &uy, V &Jx, V &Jy, V &jx,
+                                          V &jy) {
     dr = v_add(v_add(v_add(v_add(g[0], g[1]), v_add(g[2], g[3])), v_add(v_add(g[4], g[5]), v_add(g[6], g[7]))),
                g[8]);
     jx = v_add(v_add(v_sub(g[1], g[3]), v_sub(g[5], g[6])), v_sub(g[8], g[7]));
     jy = v_sub(v_add(v_sub(g[2], g[4]), v_add(g[5], g[6])), v_add(g[7], g[8]));
-    rho = v_floor_rho(v_add(v_splat<V>(1.0f), dr));
-    const V inv = v_rcp(rho);
+    const V inv = inv_density(dr);
     Jx = v_add(jx, hFx);
     Jy = v_add(jy, hFy);
     ux = v_mul_alone(Jx, inv);

@@ -10,9 +10,8 @@ namespace lbm {
 
 // Scalar entry points used by the per-node paths.
 __device__ __forceinline__ void moments_shifted(const float g[9], float hFx, float hFy, float &dr,
-                                                float &rho, float &ux, float &uy, float &Jx,
-                                                float &Jy, float &jx, float &jy) {
-    moments_v<float>(g, hFx, hFy, dr, rho, ux, uy, Jx, Jy, jx, jy);
+                                                float &ux, float &uy, float &Jx, float &Jy, float &jx, float &jy) {
+    moments_v<float>(g, hFx, hFy, dr, ux, uy, Jx, Jy, jx, jy);
 }
 
 // Rare per-node outputs, kept out of line so the compiler cannot hoist their
@@ -181,8 +180,8 @@ __device__ __forceinline__ void step_node_shifted(const FastStepParams &fp, int 
         for (int k = 0; k < 9; k++) p.bandg[(size_t)k * p.nslots + slot] = g[k];
     }
     if (FLAGS && (fl & NF_BCW)) return;
-    float dr, rho, ux, uy, Jx, Jy, jx, jy;
-    moments_v<float>(g, fp.hFxf, fp.hFyf, dr, rho, ux, uy, Jx, Jy, jx, jy);
+    float dr, ux, uy, Jx, Jy, jx, jy;
+    moments_v<float>(g, fp.hFxf, fp.hFyf, dr, ux, uy, Jx, Jy, jx, jy);
     if (p.write_macro || slot >= 0) macro_store(p, dn, slot, dr, ux, uy);
     if (COLLIDE) {
         const float om = p.omega ? (float)p.omega[dn] : fp.omega0f;
@@ -230,8 +229,8 @@ __device__ __forceinline__ void collide_store_pair_shifted(const FastStepParams 
     T *Dst = (T *)p.dst;
     const I pl = (I)p.plane;
     const I r0 = (I)j * (I)p.pitch + (I)i0;
-    float2 dr, rho, ux, uy, Jx, Jy, jx, jy;
-    moments_v<float2>(g, v_splat<float2>(fp.hFxf), v_splat<float2>(fp.hFyf), dr, rho, ux, uy, Jx, Jy, jx, jy);
+    float2 dr, ux, uy, Jx, Jy, jx, jy;
+    moments_v<float2>(g, v_splat<float2>(fp.hFxf), v_splat<float2>(fp.hFyf), dr, ux, uy, Jx, Jy, jx, jy);
     const size_t dn = (size_t)j * (size_t)p.Nx + (size_t)i0;
     if (p.write_macro) macro_store_pair(p, dn, dr, ux, uy);
     if (COLLIDE) {
@@ -253,8 +252,8 @@ __device__ __forceinline__ void finish_pops_shifted(const FinishParams &p, int2 
         g[k] = SV<T>::rnd(f[k]);
         wf[k] = p.wf[k];
     }
-    float dr, rho, ux, uy, Jx, Jy, jx, jy;
-    moments_shifted(g, p.hFxf, p.hFyf, dr, rho, ux, uy, Jx, Jy, jx, jy);
+    float dr, ux, uy, Jx, Jy, jx, jy;
+    moments_shifted(g, p.hFxf, p.hFyf, dr, ux, uy, Jx, Jy, jx, jy);
     const size_t dn = (size_t)ij.y * p.Nx + ij.x;
     if (p.write_macro) { p.rho[dn] = 1.0 + (double)dr; p.ux[dn] = ux; p.uy[dn] = uy; }
     p.bandm_next[slot] = 1.0 + (double)dr;
