@@ -18,10 +18,11 @@
 //
 // Nothing is approximated: every operation returns the FP64 result that
 // moments_exact / collide_exact round to. The fixed-point forms hold for the
-// ranges of an ordinary flow (checked per node, the flag `ok`); any other node
-// takes moments_exact / collide_exact. Ranges: populations and equilibria in
-// [2^-8, 1) (f_1 .. f_8 below 1/2), 9/16 <= rho < 2, |c.u| < 1/4, |f - f_eq| <
-// 2^-9 (2^-6 where no f or f_eq is below 2^-6). Zeros come out with lbc's value; their sign is not kept.
+// ranges of an ordinary flow, checked per node; any other node takes
+// moments_exact and collide_exact, or the latter alone. Ranges: populations in
+// [2^-8, 1) (f_1 .. f_8 below 1/2), 9/16 <= rho < 2, |c.u| < 1/4 (the equilibria
+// are then above 2^-8), |f - f_eq| < 2^-9 (2^-6 where no f or f_eq is below 2^-6).
+// Zeros come out with lbc's value; their sign is not kept.
 //
 // The division by the density is an integer one: a 64-bit reciprocal by Newton
 // steps from the FP32 one, shared by both velocities, and the exact remainder
@@ -379,11 +380,20 @@ LBM_HD double relax(uint64_t x, uint32_t s, double om, double om_m) {
     return make_double(w.lo, w.hi ^ (~hi32(x) & 0x80000000u));
 }
 
-// One node: moments, then (COLLIDE) the collided populations in f. Returns
-// false, with f untouched, when a range check fails. Needs lbc's weights w and
-// an ordinary omega (the caller's checks).
+// How far step_node_parts got: a range check failed before the moments, after
+// them (rho, ux, uy are lbc's), or none did.
+enum Done : int { DONE_NOTHING = 0, DONE_MOMENTS = 1, DONE_ALL = 2 };
+
+// One node: moments, then (COLLIDE) the collided populations in f, which stays
+// as it was when a range check fails. Needs lbc's weights w and an ordinary
+// omega (the caller's checks). A node whose collision is out of range keeps its
+// moments, so that the FP64 pipe only collides it, and one whose populations are
+// is refused before anything else. Vortices at speeds up to 0.3, us per step: 64^2
+// 8.3, 256^2 20.7, 512^2 51, 1024^2 165 (with the moments taken again 256^2 25.7,
+// 1024^2 217; all on the FP64 pipe 12.5, 21.7, 67, 252). Density 2.5: 7.0, 20.9,
+// 66.9, 251.
 template <bool COLLIDE>
-LBM_HD bool step_node(double f[9], const double w[9], bool force, double hFx, double hFy, double om, double Fx,
+LBM_HD int step_node_parts(double f[9], const double w[9], bool force, double hFx, double hFy, double om, double Fx,
                       double Fy, double &rho, double &ux, double &uy) {
     uint32_t bad = 0, half = 0;
     uint64_t F[9];
@@ -394,12 +404,13 @@ LBM_HD bool step_node(double f[9], const double w[9], bool force, double hFx, do
         half |= hi32(F[k]);
     }
     bad |= half & 0xF0000000u;
+    if (bad > 7u) return DONE_NOTHING;
     const Moments q = moments(F, force, hFx, hFy, bad);
-    if (bad > 7u) return false;
+    if (bad > 7u) return DONE_NOTHING;
     rho = from_fixed(q.s, 61);
     ux = value_of(q.ux);
     uy = value_of(q.uy);
-    if (!COLLIDE) return true;
+    if (!COLLIDE) return DONE_ALL;
 
     const uint64_t kNinth = 0xE38E38E38E38E000ull;  // the FP64 number 1/9, LSB 2^-67
     const uint64_t wr = round53(mul_high_sticky(kNinth, q.D << 1));
@@ -432,7 +443,7 @@ LBM_HD bool step_node(double f[9], const double w[9], bool force, double hFx, do
     // Below 2^-9 as they are; below 2^-6 without their low three bits, which are
     // zero when f and f_eq are 2^-6 or more.
     const uint32_t sh = big >> 20 ? 3u : 0u;
-    if ((big >> 23) || (sh && (low & 7u)) || (far >> 31)) return false;
+    if ((big >> 23) || (sh && (low & 7u)) || (far >> 31)) return DONE_MOMENTS;
     const double om_m = make_double(words(om).lo, words(om).hi + 0x80000000u - ((9u - sh) << 20));
     double r[9];
 #pragma unroll
@@ -440,7 +451,7 @@ LBM_HD bool step_node(double f[9], const double w[9], bool force, double hFx, do
     if (!force) {
 #pragma unroll
         for (int k = 0; k < 9; k++) f[k] = add(f[k], r[k]);
-        return true;
+        return DONE_ALL;
     }
     // Guo's term (collide_exact): w (3 c.F + 9 (c.u)(c.F) - 3 u.F), in the FP64
     // sequence. The pair's product (9 c.u)(c.F) is the same for both directions;
@@ -466,7 +477,14 @@ LBM_HD bool step_node(double f[9], const double w[9], bool force, double hFx, do
         f[ka] = add(f[ka], add(r[ka], ta));
         f[kb] = add(f[kb], add(r[kb], tb));
     }
-    return true;
+    return DONE_ALL;
+}
+
+// The same, all or nothing.
+template <bool COLLIDE>
+LBM_HD bool step_node(double f[9], const double w[9], bool force, double hFx, double hFy, double om, double Fx,
+                      double Fy, double &rho, double &ux, double &uy) {
+    return step_node_parts<COLLIDE>(f, w, force, hFx, hFy, om, Fx, Fy, rho, ux, uy) == DONE_ALL;
 }
 
 }  // namespace fi

@@ -117,10 +117,11 @@ __device__ __forceinline__ void step_node_exact(const StepParams &p, int i, int 
             if (!(FLAGS && (fl & NF_BCW))) {
                 double rho, ux, uy;
                 const double om = COLLIDE ? (p.omega ? p.omega[dn] : p.omega0) : 0.0;
-                bool done = false;
+                int done = fi::DONE_NOTHING;
                 if (ARITH == ARITH_INT)
-                    done = fi::step_node<COLLIDE>(f, p.w, p.has_force != 0, p.hFx, p.hFy, om, p.Fx, p.Fy, rho, ux, uy);
-                if (!done) {
+                    done = fi::step_node_parts<COLLIDE>(f, p.w, p.has_force != 0, p.hFx, p.hFy, om, p.Fx, p.Fy, rho, ux,
+                                                        uy);
+                if (done == fi::DONE_NOTHING) {
                     if (ARITH == ARITH_FMA) moments_fma(f, p.hFx, p.hFy, p.has_force != 0, rho, ux, uy);
                     else moments_exact(f, p.hFx, p.hFy, rho, ux, uy);
                 }
@@ -130,7 +131,7 @@ __device__ __forceinline__ void step_node_exact(const StepParams &p, int i, int 
                     p.bandm_next[(size_t)p.nslots + slot] = ux;
                     p.bandm_next[2 * (size_t)p.nslots + slot] = uy;
                 }
-                if (COLLIDE && !done) {
+                if (COLLIDE && done != fi::DONE_ALL) {
                     if (ARITH == ARITH_FMA) collide_fma(f, p.w[0], p.w[1], p.w[5], rho, ux, uy, om, p.has_force != 0, p.Fx, p.Fy);
                     else collide_exact(f, p.w, rho, ux, uy, om, p.has_force != 0, p.Fx, p.Fy);
                 }
@@ -245,16 +246,17 @@ __device__ __forceinline__ void finish_pops_exact(const FinishParams &p, int2 ij
     double rho, ux, uy;
     const size_t dn = (size_t)ij.y * p.Nx + ij.x;
     const double om = COLLIDE ? (p.omega ? p.omega[dn] : p.omega0) : 0.0;
-    const bool done = arith == ARITH_INT && fi::step_node<COLLIDE>(f, p.w, p.has_force != 0, p.hFx, p.hFy, om, p.Fx, p.Fy,
-                                                                   rho, ux, uy);
-    if (!done) moments_exact(f, p.hFx, p.hFy, rho, ux, uy);
+    int done = fi::DONE_NOTHING;
+    if (arith == ARITH_INT)
+        done = fi::step_node_parts<COLLIDE>(f, p.w, p.has_force != 0, p.hFx, p.hFy, om, p.Fx, p.Fy, rho, ux, uy);
+    if (done == fi::DONE_NOTHING) moments_exact(f, p.hFx, p.hFy, rho, ux, uy);
     if (live) {
         if (p.write_macro) { p.rho[dn] = rho; p.ux[dn] = ux; p.uy[dn] = uy; }
         p.bandm_next[slot] = rho;
         p.bandm_next[(size_t)p.nslots + slot] = ux;
         p.bandm_next[2 * (size_t)p.nslots + slot] = uy;
     }
-    if (COLLIDE && !done) collide_exact(f, p.w, rho, ux, uy, om, p.has_force != 0, p.Fx, p.Fy);
+    if (COLLIDE && done != fi::DONE_ALL) collide_exact(f, p.w, rho, ux, uy, om, p.has_force != 0, p.Fx, p.Fy);
     double *D = (double *)p.dst;
     const long long node = (long long)ij.y * p.pitch + ij.x;
     if (live) {
