@@ -120,8 +120,10 @@ Solver::~Solver() {
     vtk_wait();
     if (vtk_ev_) cudaEventDestroy(vtk_ev_);
     if (h_vtk_) cudaFreeHost(h_vtk_);
-    if (pair_exec_) cudaGraphExecDestroy(pair_exec_);
-    if (multi_exec_) cudaGraphExecDestroy(multi_exec_);
+    for (int q = 0; q < 4; q++) {
+        if (pair_graph_[q].exec) cudaGraphExecDestroy(pair_graph_[q].exec);
+        if (multi_graph_[q].exec) cudaGraphExecDestroy(multi_graph_[q].exec);
+    }
     if (beside_ev_) cudaEventDestroy(beside_ev_);
     if (multi_fork_) cudaEventDestroy(multi_fork_);
     if (multi_join_) cudaEventDestroy(multi_join_);
@@ -624,7 +626,7 @@ bool Solver::upload_force_slot() {
 
 bool Solver::set_block(dim3 b) {
     block_ = b;
-    graph_valid_ = graph_valid_multi_ = false;
+    drop_graphs();
     return true;
 }
 
@@ -776,7 +778,7 @@ bool Solver::enable_force_history(int capacity) {
     hist_cap_ = capacity;
     hist_count_ptr_ = cnt;
     hist_written_ = 0;  // a new ring: its records count from its first step
-    graph_valid_ = graph_valid_multi_ = false;
+    drop_graphs();
     return upload_force_slot();
 }
 
@@ -1027,7 +1029,7 @@ bool Solver::set_impedance(int entry, const double *R, const double *m, const do
         st->imp_cos[f] = std::cos(omegas[f]);
         st->imp_sin[f] = std::sin(omegas[f]);
     }
-    graph_valid_ = graph_valid_multi_ = false;
+    drop_graphs();
     // a wall trace reads this array: its record task follows a new allocation
     return st->d_trace ? upload_records() : true;
 }
@@ -1213,7 +1215,7 @@ bool Solver::upload_records() {
         r.count = st.trace_count;
         rec_host_.push_back(r);
     }
-    graph_valid_ = graph_valid_multi_ = false;
+    drop_graphs();
     if (rec_host_.empty()) return true;
     if ((int)rec_host_.size() > rec_cap_) {
         if (!dalloc(&d_rec_, rec_host_.size())) return false;
@@ -1369,11 +1371,11 @@ void Solver::advance(int nsteps) {
 // a pair of small steps does not hide: Taylor-Green 64^2 FP32 3.10 us per step
 // with one pair per graph, 2.10 with four, 2.00 with sixteen; channel 256 x 64
 // FP64 9.25, 8.49, 8.27.
-bool Solver::capture_pair() {
-    if (graph_valid_ && pair_cur_ == cur_ && pair_parity_ == parity_) return true;
-    if (pair_exec_) {
-        cudaGraphExecDestroy(pair_exec_);
-        pair_exec_ = nullptr;
+bool Solver::capture_pair(StepGraph &sg) {
+    if (sg.valid) return true;
+    if (sg.exec) {
+        cudaGraphExecDestroy(sg.exec);
+        sg.exec = nullptr;
     }
     if (!beside_ev_) CK(cudaEventCreateWithFlags(&beside_ev_, cudaEventDisableTiming));
     cudaGraph_t g = nullptr;
@@ -1389,13 +1391,15 @@ bool Solver::capture_pair() {
         return false;
     }
     CK(e);
-    e = cudaGraphInstantiate(&pair_exec_, g, 0);
+    e = cudaGraphInstantiate(&sg.exec, g, 0);
     cudaGraphDestroy(g);
     CK(e);
-    pair_cur_ = cur_;
-    pair_parity_ = parity_;
-    graph_valid_ = true;
+    sg.valid = true;
     return true;
+}
+
+void Solver::drop_graphs() {
+    for (int q = 0; q < 4; q++) pair_graph_[q].valid = multi_graph_[q].valid = false;
 }
 
 // This case's tiles for the batched kernel (x = 0, y = x0, z = y0, w = 1 when
@@ -1654,11 +1658,11 @@ bool Solver::launch_multi(int cur, int other, int lv) {
 }
 
 // kGraphPairs / 2 double passes (cur -> other -> cur) captured once and replayed.
-bool Solver::capture_multi() {
-    if (multi_exec_ && multi_cur_ == cur_ && multi_parity_ == parity_ && graph_valid_multi_) return true;
-    if (multi_exec_) {
-        cudaGraphExecDestroy(multi_exec_);
-        multi_exec_ = nullptr;
+bool Solver::capture_multi(StepGraph &sg) {
+    if (sg.valid) return true;
+    if (sg.exec) {
+        cudaGraphExecDestroy(sg.exec);
+        sg.exec = nullptr;
     }
     cudaGraph_t g = nullptr;
     CK(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
@@ -1671,12 +1675,10 @@ bool Solver::capture_multi() {
         return false;
     }
     CK(e);
-    e = cudaGraphInstantiate(&multi_exec_, g, 0);
+    e = cudaGraphInstantiate(&sg.exec, g, 0);
     cudaGraphDestroy(g);
     CK(e);
-    multi_cur_ = cur_;
-    multi_parity_ = parity_;
-    graph_valid_multi_ = true;
+    sg.valid = true;
     return true;
 }
 
@@ -1687,10 +1689,11 @@ int Solver::run_multi(int avail) {
     if (!swap_multi(true, lv, stream_)) return -1;
     int used = 0;
     const int whole = kGraphPairs * lv;
-    if (avail >= whole) {
-        if (!capture_multi()) return -1;
+    StepGraph &g = multi_graph_[2 * cur_ + parity_];
+    if (avail >= whole && (g.valid || capture_due(g.owed, avail))) {
+        if (!capture_multi(g)) return -1;
         for (; avail - used >= whole; used += whole)
-            if (!check_cuda(cudaGraphLaunch(multi_exec_, stream_), "cudaGraphLaunch")) return -1;
+            if (!check_cuda(cudaGraphLaunch(g.exec, stream_), "cudaGraphLaunch")) return -1;
     }
     for (; avail - used >= 2 * lv; used += 2 * lv)
         if (!launch_multi(cur_, 1 - cur_, lv) || !launch_multi(1 - cur_, cur_, lv)) return -1;
@@ -1782,9 +1785,10 @@ bool Solver::run(int nsteps) {
         const int near = 1 + (one_group_ ? force : (int)groups_.size());
         launches_ += (long long)(used / lv) * (has_flags_ ? 1 + lv * near : 1) + (has_flags_ ? 2 : 0);
     }
-    if (remaining >= 2 * kGraphPairs) {
-        if (!capture_pair()) return false;
-        for (; remaining >= 2 * kGraphPairs; remaining -= 2 * kGraphPairs) CK(cudaGraphLaunch(pair_exec_, stream_));
+    StepGraph &g = pair_graph_[2 * cur_ + parity_];
+    if (remaining >= 2 * kGraphPairs && (g.valid || capture_due(g.owed, remaining))) {
+        if (!capture_pair(g)) return false;
+        for (; remaining >= 2 * kGraphPairs; remaining -= 2 * kGraphPairs) CK(cudaGraphLaunch(g.exec, stream_));
     }
     for (; remaining > 0; remaining--)
         if (!trial_step()) return false;
@@ -2386,8 +2390,11 @@ bool Batch::run(int nsteps) {
         }
         // (params_ev_ again: the passes' parameter copies are waited for too)
         if (okk) okk = check_cuda(cudaEventRecord(params_ev_, stream_), "event");
-        if (okk && pairs >= kGraphPairs) okk = capture_pair();
-        for (; okk && pairs >= kGraphPairs; pairs -= kGraphPairs) okk = check_cuda(cudaGraphLaunch(pair_exec_, stream_), "graph");
+        if (okk && pairs >= kGraphPairs && (pair_exec_ || capture_due(owed_, 2 * pairs))) {
+            okk = capture_pair();
+            for (; okk && pairs >= kGraphPairs; pairs -= kGraphPairs)
+                okk = check_cuda(cudaGraphLaunch(pair_exec_, stream_), "graph");
+        }
         for (; okk && pairs > 0; pairs--) okk = launch_batched(0) && launch_batched(1);
         if (okk && (mid & 1)) okk = launch_batched(0);
         for (Solver *c : cases_) {

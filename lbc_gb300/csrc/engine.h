@@ -91,6 +91,25 @@ struct Stage {
 
 // Step pairs per captured graph.
 constexpr int kGraphPairs = 4;
+// A graph is captured once kCaptureSteps steps have been asked for that it would
+// serve, in one run or in several (owed): capturing and instantiating eight steps
+// costs the host more than launching them. Taylor-Green 64^2 FP32, first run of 9
+// steps 68 us with a graph, 50 without; of 33 steps 119.
+constexpr int kCaptureSteps = 32;
+inline bool capture_due(int &owed, int steps) {
+    owed = std::min(owed + std::min(steps, kCaptureSteps), kCaptureSteps);
+    return owed == kCaptureSteps;
+}
+
+// A captured graph of steps from one state (the current buffer and the parity of
+// the band moments). A run of odd length leaves the other state, so each has its
+// graph (Taylor-Green 64^2 FP32, runs of 11: 68 us with a graph captured in each,
+// 48 with both kept).
+struct StepGraph {
+    cudaGraphExec_t exec = nullptr;
+    bool valid = false;
+    int owed = 0;
+};
 
 // Most probes a solver records (one block of a record launch walks them).
 constexpr int kMaxProbes = 4096;
@@ -278,13 +297,14 @@ class Solver {
     unsigned long long *probe_count_ = nullptr;
     int nprobes_ = 0, probe_cap_ = 0;
     bool launch_collide(int b, cudaStream_t s = nullptr);
-    bool capture_pair();
+    bool capture_pair(StepGraph &g);
+    void drop_graphs();
     bool beside(cudaStream_t s);
     bool join(cudaStream_t s);
     int multi_warps() const;
     bool multi_setup();
     bool launch_multi(int cur, int other, int lv);
-    bool capture_multi();
+    bool capture_multi(StepGraph &g);
     int run_multi(int avail);
     bool trial_step();
     // A launch of the fused step in blocks of `by` rows reaches every row.
@@ -338,14 +358,9 @@ class Solver {
     std::vector<short> last_host_;
     short *d_last_ = nullptr;
     dim3 block_{64, 4, 1};
-    cudaGraphExec_t pair_exec_ = nullptr;
-    int pair_cur_ = -1, pair_parity_ = -1;
-    bool graph_valid_ = false;
+    StepGraph pair_graph_[4], multi_graph_[4];  // by 2 cur_ + parity_
     bool capturing_ = false;
     cudaEvent_t beside_ev_ = nullptr;
-    cudaGraphExec_t multi_exec_ = nullptr;
-    int multi_cur_ = -1, multi_parity_ = -1;
-    bool graph_valid_multi_ = false;
     mutable NearPlan near_plan_;
     int multi_state_ = 0;                 // 0: not tried, 1: set up, -1: not for this case
     uint32_t *d_deep_ = nullptr;
@@ -462,6 +477,7 @@ class Batch {
     RecordTask *d_rec_ = nullptr;   // every case's probes and wall traces (case index set)
     int nrec_ = 0;
     cudaGraphExec_t pair_exec_ = nullptr;
+    int owed_ = 0;  // steps that runs asked for without it
     std::vector<void *> allocs_;
     // passes of several steps (multi_setup)
     int multi_state_ = 0, multi_lv_ = 4, ntasks_ = 0, nmsegs_[4] = {0, 0, 0, 0};

@@ -173,7 +173,7 @@ bool Solver::checkpoint_load(const char *path) {
     parity_ = h.parity;
     fields_are_moments_ = h.fields_are_moments != 0;
     steps_done_ = h.steps_done;
-    graph_valid_ = false;
+    drop_graphs();
     return true;
 }
 
