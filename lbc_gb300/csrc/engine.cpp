@@ -876,7 +876,6 @@ StepParams Solver::step_params(int src, int dst, bool write_macro, int bparity) 
     p.flags = d_flags_; p.link_off = d_link_off_; p.links = d_links_;
     p.seg_clean = d_seg_clean_; p.seg_words = seg_words_;
     p.omega = d_omega_; p.omega0 = omega0_;
-    p.fma = arith_ == ARITH_FMA ? 1 : 0;
     p.has_force = (d_.Fx != 0.0 || d_.Fy != 0.0);
     p.Fx = d_.Fx; p.Fy = d_.Fy; p.hFx = 0.5 * d_.Fx; p.hFy = 0.5 * d_.Fy;
     for (int k = 0; k < 9; k++) p.w[k] = d_.w[k];
@@ -1822,11 +1821,6 @@ Batch::Batch(const std::vector<Solver *> &cases) : cases_(cases) {
             return;
         }
     }
-    // One arithmetic per launch; for a mix, one kernel that asks each case
-    // (the integer form's cases take lbc's sequence there: the same bits).
-    arith_ = cases_[0]->arith();
-    for (Solver *c : cases_)
-        if (c->arith() != arith_) arith_ = ARITH_MIXED;
     // FP64 batches (FP64-issue bound, long) run at the lowest stream priority,
     // shifted-storage batches at the highest, so that when both run at once
     // (the server's lanes) free SMs go to the short, memory-bound FP32 steps
@@ -1868,13 +1862,33 @@ template <class T> static bool balloc(std::vector<void *> &allocs, T **p, size_t
 // room for the per-direction parameter arrays, which run() refreshes.
 // Tiles of 2^tws x 2^(8 - tws) threads over every case (one node per thread in
 // FP64, two adjacent nodes in shifted storage); w = 1 for tiles that contain
-// wall links (their threads store force partials).
+// wall links (their threads store force partials). FP64: the cases of one
+// arithmetic after those of another (tile_runs), in batch order within each.
 std::vector<int4> Batch::make_tiles(int tws) const {
     std::vector<int4> tiles;
-    for (int c = 0; c < (int)cases_.size(); c++)
-        for (const int4 &t : cases_[c]->tiles(tws))
-            tiles.push_back(make_int4(c, t.y, t.z, t.w));
+    for (int a = 0; a < ARITH_COUNT; a++)
+        for (int c = 0; c < (int)cases_.size(); c++) {
+            if (cases_[c]->arith() != a) continue;
+            for (const int4 &t : cases_[c]->tiles(tws)) tiles.push_back(make_int4(c, t.y, t.z, t.w));
+        }
     return tiles;
+}
+
+// One launch of the FP64 bulk kernel per arithmetic in the batch. (One kernel that
+// asks each case is compiled for the registers of them all: eight 512^2 vortices
+// beside a small case of other weights 587 us per step, XX in two launches, 164
+// without it.)
+std::vector<Batch::TileRun> Batch::tile_runs(int tws) const {
+    std::vector<TileRun> runs;
+    int first = 0;
+    for (int a = 0; a < ARITH_COUNT; a++) {
+        int n = 0;
+        for (const Solver *c : cases_)
+            if (c->arith() == a) n += (int)c->tiles(tws).size();
+        if (n) runs.push_back(TileRun{a, first, n});
+        first += n;
+    }
+    return runs;
 }
 
 bool Batch::upload_tiles(const std::vector<int4> &tiles, int4 **d) {
@@ -1891,6 +1905,7 @@ void Batch::install_tiles(int4 *d, int n, int tws, bool free_old) {
     d_tiles_ = d;
     ntiles_ = n;
     tws_ = tws;
+    runs_ = tile_runs(tws);
     grid_ = std::min(ntiles_, store_ == STORE_F64 ? launch::step_batch_exact_grid()
                                                   : launch::step_batch_shifted_grid(store_));
     if (grid_ < 1) grid_ = 1;
@@ -2109,7 +2124,7 @@ bool Batch::build() {
     // The force reductions ride in the first stage level's launch.
     int stage_launches = 0;
     for (int nb : stage_nblocks_) stage_launches += nb > 0 ? 1 : 0;
-    launches_per_step_ = 1 + (nspecial_ ? 1 : 0) + stage_launches +
+    launches_per_step_ = (store_ == STORE_F64 ? (int)runs_.size() : 1) + (nspecial_ ? 1 : 0) + stage_launches +
                          (nforce_ && max_stages_ == 0 ? 1 : 0) + (nrec_ ? 1 : 0);
     CK(cudaStreamSynchronize(stream_));
     return true;
@@ -2117,8 +2132,9 @@ bool Batch::build() {
 
 bool Batch::launch_batched(int sel) {
     if (store_ == STORE_F64) {
-        CK(launch::step_batch_exact((const StepParams *)d_sp_, d_tiles_, ntiles_, sel, tws_,
-                                    grid_, stream_, arith_));
+        for (const TileRun &r : runs_)
+            CK(launch::step_batch_exact((const StepParams *)d_sp_, d_tiles_ + r.first, r.n, sel, tws_,
+                                        std::min(grid_, r.n), stream_, r.arith));
     } else {
         // the clean pairs, then the special nodes overlapping their tail
         CK(launch::step_batch_shifted((const FastStepParams *)d_sp_, d_tiles_, ntiles_, sel, tws_,

@@ -434,6 +434,9 @@ class Batch {
     bool build();
     bool build_tiles(int tws);
     std::vector<int4> make_tiles(int tws) const;
+    // The tiles of the cases of one arithmetic (FP64 storage).
+    struct TileRun { int arith, first, n; };
+    std::vector<TileRun> tile_runs(int tws) const;
     bool upload_tiles(const std::vector<int4> &tiles, int4 **d);
     void install_tiles(int4 *d, int n, int tws, bool free_old);
     int tune_online(int avail_pairs);
@@ -448,7 +451,7 @@ class Batch {
     int run_multi(int pairs);
 
     std::vector<Solver *> cases_;
-    int store_ = STORE_F64, arith_ = ARITH_LBC;
+    int store_ = STORE_F64;
     bool ok_ = false;
     cudaStream_t stream_ = nullptr;
     long long nodes_ = 0;
@@ -476,6 +479,7 @@ class Batch {
     int nspecial_nf_ = 0;
     RecordTask *d_rec_ = nullptr;   // every case's probes and wall traces (case index set)
     int nrec_ = 0;
+    std::vector<TileRun> runs_;
     cudaGraphExec_t pair_exec_ = nullptr;
     int owed_ = 0;  // steps that runs asked for without it
     std::vector<void *> allocs_;

@@ -173,15 +173,7 @@ __global__ void __launch_bounds__(256, ARITH == ARITH_INT ? 3 : 1) k_step_batch_
         double mfx = 0.0, mfy = 0.0;
         bool link = false;
         const bool in = i < p.Nx && j < p.Ny;
-        if (ARITH == ARITH_MIXED) {
-            if (in && p.flags) {
-                if (p.fma) step_node_exact<true, true, ARITH_FMA>(p, i, j, mfx, mfy, link);
-                else step_node_exact<true, true, ARITH_LBC>(p, i, j, mfx, mfy, link);
-            } else if (in) {
-                if (p.fma) step_node_exact<false, true, ARITH_FMA>(p, i, j, mfx, mfy, link);
-                else step_node_exact<false, true, ARITH_LBC>(p, i, j, mfx, mfy, link);
-            }
-        } else if (p.flags) {
+        if (p.flags) {
             if (in) step_node_exact<true, true, ARITH>(p, i, j, mfx, mfy, link);
         } else {
             if (in) step_node_exact<false, true, ARITH>(p, i, j, mfx, mfy, link);
@@ -957,7 +949,6 @@ cudaError_t step_batch_exact(const StepParams *sp, const int4 *tiles, int ntiles
     if (tws < 5 || tws > 8) return cudaErrorInvalidValue;
     if (arith == ARITH_FMA) k_step_batch_exact<ARITH_FMA><<<grid, 256, 0, s>>>(sp, tiles, ntiles, sel, tws);
     else if (arith == ARITH_INT) k_step_batch_exact<ARITH_INT><<<grid, 256, 0, s>>>(sp, tiles, ntiles, sel, tws);
-    else if (arith == ARITH_MIXED) k_step_batch_exact<ARITH_MIXED><<<grid, 256, 0, s>>>(sp, tiles, ntiles, sel, tws);
     else k_step_batch_exact<ARITH_LBC><<<grid, 256, 0, s>>>(sp, tiles, ntiles, sel, tws);
     return cudaGetLastError();
 }

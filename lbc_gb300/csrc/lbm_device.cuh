@@ -95,7 +95,7 @@ __host__ __device__ inline bool bc_is_column(int kind) {
 }
 
 // Arithmetic of the FP64 step (step_node_exact).
-enum : int { ARITH_LBC = 0, ARITH_FMA = 1, ARITH_INT = 2, ARITH_MIXED = 3 };
+enum : int { ARITH_LBC = 0, ARITH_FMA = 1, ARITH_INT = 2, ARITH_COUNT = 3 };
 
 // Storage policies: FP64 stores f as is; FP32/FP16 store the shifted deviation
 // g_k = f_k - w_k.
@@ -558,7 +558,6 @@ struct StepParams {
     const Link *links;
     const double *omega;      // [Ny * Nx] per-node omega, or null -> omega0
     double omega0;
-    int fma;                  // batches of mixed arithmetic: this case's is ARITH_FMA, else lbc's
     int has_force;
     double Fx, Fy, hFx, hFy;  // hF = 0.5 F
     double w[9];
