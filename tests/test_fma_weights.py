@@ -49,13 +49,6 @@ def test_every_edge_case(oracle, name, omega):
         assert force_close(h[:, 1], fo[:, 0], rtol=RTOL, scale=mag), name
 
 
-def test_forced_channel(oracle):
-    case, st = _other_weights(cases.poiseuille(256, 64, 0.8, 1e-6))
-    got, _ = _run_fma(case, st, 2000)
-    oracle.run(case, st, 2000)
-    _check(case, got, st, "channel")
-
-
 @pytest.mark.parametrize("storage", ["f64", "f64fma"])
 @pytest.mark.parametrize("mixed", [False, True])
 def test_batch_equals_alone(storage, mixed):
