@@ -1490,74 +1490,8 @@ int Solver::multi_warps() const {
 // Kept per case: a server builds a batch anew whenever a request joins or leaves.
 const NearPlan &Solver::near_plan(int lv) const {
     if (near_plan_.lv == lv) return near_plan_;
-    NearPlan &plan = near_plan_;
-    plan.lv = lv;
-    const int Nx = d_.Nx, Ny = d_.Ny;
-    // Distance to the nearest special node (the larger of |dx|, |dy|), up to m,
-    // by runs of special nodes along a row.
-    const int m = 2 * lv - 1, nsp = (int)special_host_.size();
-    std::vector<uint8_t> dist((size_t)Nx * Ny, 255);
-    for (int q = 0; q < nsp;) {
-        const int y = special_host_[q].y, i0 = special_host_[q].x & ~kSpecialSolid;
-        int i1 = i0;
-        for (q++; q < nsp && special_host_[q].y == y && (special_host_[q].x & ~kSpecialSolid) == i1 + 1; q++) i1++;
-        for (int dy = -m; dy <= m; dy++) {
-            int j = y + dy;
-            if (!wrap(j, Ny, d_.py)) continue;
-            uint8_t *row = &dist[(size_t)j * Nx];
-            const uint8_t ady = (uint8_t)std::abs(dy);
-            for (int i = i0; i <= i1; i++) row[i] = std::min(row[i], ady);
-            for (int dx = 1; dx <= m; dx++) {
-                const uint8_t d = std::max(ady, (uint8_t)dx);
-                int l = i0 - dx, r = i1 + dx;
-                if (wrap(l, Nx, d_.px)) row[l] = std::min(row[l], d);
-                if (wrap(r, Nx, d_.px)) row[r] = std::min(row[r], d);
-            }
-        }
-    }
-    // Deep pairs, both nodes lv or more away: every pair of the grid, then the
-    // near ones taken out as they join the segments.
-    const int halo = multi_halo(lv), width = 64 - 2 * halo, strips = (Nx + width - 1) / width;
-    plan.deep.resize((size_t)strips * Ny);
-    for (int st = 0; st < strips; st++) {
-        uint32_t all = 0;
-        for (int c = 0; c < width && st * width + c + 1 < Nx; c += 2) all |= 1u << ((c + halo) / 2);
-        std::fill(plan.deep.begin() + (size_t)st * Ny, plan.deep.begin() + (size_t)(st + 1) * Ny, all);
-    }
-    plan.segs.assign(lv, std::vector<int4>());
-    plan.near_pairs = 0;
-    for (int j = 0; j < Ny; j++) {
-        const uint8_t *row = &dist[(size_t)j * Nx];
-        for (int s0 = 0; s0 < Nx; s0 += 64) {
-            uint32_t mask[4] = {0, 0, 0, 0};
-            bool any = false;
-            for (int l = 0; l < 32 && s0 + 2 * l < Nx; l++) {
-                const int i = s0 + 2 * l;
-                uint64_t eight;
-                if (l % 4 == 0 && i + 8 <= Nx && (std::memcpy(&eight, row + i, 8), eight == ~0ull)) {
-                    l += 3;
-                    continue;
-                }
-                if (i + 1 >= Nx) continue;  // an odd last column is special
-                const int d = std::min(row[i], row[i + 1]);
-                if (d < lv) plan.deep[(size_t)(i / width) * Ny + j] &= ~(1u << ((i % width + halo) / 2));
-                if (d == 0) continue;       // special: both nodes of the pair
-                // step q + 1 of the list needs the nodes within 2 lv - (q + 1) of
-                // a special one; the last, every pair that is not deep
-                for (int q = 0; q < lv; q++)
-                    if (q == lv - 1 ? d < lv : d < 2 * lv - q) {
-                        mask[q] |= 1u << l;
-                        any = true;
-                    }
-            }
-            for (int q = 0; any && q < lv; q++)
-                if (mask[q]) {
-                    plan.segs[q].push_back(make_int4(0, j, s0, (int)mask[q]));
-                    plan.near_pairs += __builtin_popcount(mask[q]);
-                }
-        }
-    }
-    return plan;
+    near_plan_ = make_near_plan(d_.Nx, d_.Ny, d_.px, d_.py, special_host_, ~kSpecialSolid, lv, multi_halo(lv));
+    return near_plan_;
 }
 
 bool Solver::multi_buffers(int lv) {
@@ -1589,22 +1523,33 @@ StepParams Solver::near_params(int cur, int other, int lv, int q) const {
     return p;
 }
 
+// Whether the geometry of a case with a flag word allows passes and they pay.
+bool Solver::multi_shape(int lv) {
+    const long long n = (long long)d_.Nx * d_.Ny;
+    if (nspecial_ == 0 || nspecial_ > n / 8) return false;
+    for (const Stage &st : stages_)  // these read post-collision values of the opposite edge
+        if (st.kind == BC_PERIODIC_X || st.kind == BC_PERIODIC_Y) return false;
+    // With much of the grid near walls the lists outweigh the pass (channel 16384 x
+    // 64, 16 % near: 12.9 us one step at a time, 13.7 in passes; 32768 x 64 27.8
+    // and 22.0).
+    return n >= (1LL << 21) || 16 * near_plan(lv).near_pairs <= n * lv;
+}
+
+size_t Solver::multi_need(int lv) const {
+    size_t need = 0;
+    for (int b = 2; b < (lv > 2 ? 4 : 3); b++) need += buf_[b] ? 0 : multi_bytes();
+    return need;
+}
+
 // Sets a case alone up for passes; false: not this case.
 bool Solver::multi_setup() {
     if (multi_state_) return multi_state_ > 0;
     multi_state_ = -1;
     const int lv = multi_levels();
-    if (nspecial_ == 0 || (long long)nspecial_ > (long long)d_.Nx * d_.Ny / 8) return false;
-    for (const Stage &st : stages_)  // these read post-collision values of the opposite edge
-        if (st.kind == BC_PERIODIC_X || st.kind == BC_PERIODIC_Y) return false;
+    if (!multi_shape(lv)) return false;
     size_t freeb = 0, total = 0;
-    if (cudaMemGetInfo(&freeb, &total) != cudaSuccess || freeb / 4 < (size_t)(lv > 2 ? 2 : 1) * multi_bytes()) return false;
+    if (cudaMemGetInfo(&freeb, &total) != cudaSuccess || freeb / 4 < multi_need(lv)) return false;
     const NearPlan &plan = near_plan(lv);
-    // With much of the grid near walls the lists outweigh the pass (channel 16384 x
-    // 64, 16 % near: 12.9 us one step at a time, 13.7 in passes; 32768 x 64 27.8
-    // and 22.0).
-    const long long n = (long long)d_.Nx * d_.Ny;
-    if (n < (1LL << 21) && 16 * plan.near_pairs > n * lv) return false;
     if (!dalloc(&d_deep_, plan.deep.size())) return false;
     CK(cudaMemcpyAsync(d_deep_, plan.deep.data(), plan.deep.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, stream_));
     for (int q = 0; q < lv; q++) {
@@ -1684,7 +1629,15 @@ bool Solver::capture_multi(StepGraph &sg) {
 // As many of `avail` steps as whole double passes take; -1 on an error.
 int Solver::run_multi(int avail) {
     const int lv = multi_levels();
-    if (lv == 0 || avail < 2 * lv || (has_flags_ && (avail < 8 * lv || !multi_setup()))) return 0;
+    if (lv == 0 || avail < 2 * lv) return 0;
+    if (has_flags_) {
+        if (avail < 8 * lv) return 0;
+        if (multi_state_ == 0) {
+            multi_owed_ = std::min(multi_owed_ + std::min(avail, kMultiOwed), kMultiOwed);
+            if (multi_owed_ < kMultiOwed) return 0;
+        }
+        if (!multi_setup()) return 0;
+    }
     if (!swap_multi(true, lv, stream_)) return -1;
     int used = 0;
     const int whole = kGraphPairs * lv;
@@ -2183,17 +2136,21 @@ bool Batch::capture_pair() {
 // launch of warps over strips and rows of every case, and beside it one launch
 // per step of every case's special nodes, near pairs and edges. Large batches
 // of cases whose Boundary lists are one group, without records.
+bool Batch::multi_shape() const {
+    if (store_ == STORE_F64 || nodes_ < (store_ == STORE_F32 ? (1LL << 22) : (1LL << 23)) || nrec_ || max_stages_ > 1)
+        return false;
+    for (const Solver *c : cases_)
+        if (!c->multi_case()) return false;
+    return true;
+}
+
 bool Batch::multi_setup() {
     if (multi_state_) return multi_state_ > 0;
     multi_state_ = -1;
     const int lv = multi_lv_;
-    if (store_ == STORE_F64 || nodes_ < (store_ == STORE_F32 ? (1LL << 22) : (1LL << 23)) || nrec_ || max_stages_ > 1)
-        return false;
+    if (!multi_shape()) return false;
     size_t need = 0, freeb = 0, total = 0;
-    for (Solver *c : cases_) {
-        if (!c->multi_case()) return false;
-        need += 2 * c->multi_bytes();
-    }
+    for (const Solver *c : cases_) need += c->multi_need(lv);
     if (cudaMemGetInfo(&freeb, &total) != cudaSuccess || freeb / 4 < need) return false;
     std::vector<uint32_t> deep;
     std::vector<std::vector<int4>> segs(lv);
@@ -2304,7 +2261,16 @@ bool Batch::launch_multi(int a) {
 // As many of `pairs` step pairs as whole double passes take; -1 on an error.
 int Batch::run_multi(int pairs) {
     const int lv = multi_lv_;
-    if (forces_ || pairs < 4 * lv || !multi_setup()) return 0;
+    if (forces_ || pairs < 4 * lv) return 0;
+    if (multi_state_ == 0) {
+        // Cases that have been in a batch of passes keep their plans and buffers.
+        bool fresh = false;
+        for (const Solver *c : cases_) fresh = fresh || c->multi_need(lv) > 0;
+        const int due = fresh ? kMultiOwed : 8 * lv;
+        multi_owed_ = std::min(multi_owed_ + 2 * std::min(pairs, due), due);
+        if (multi_owed_ < due) return 0;
+    }
+    if (!multi_setup()) return 0;
     if (!upload_multi()) return -1;
     for (Solver *c : cases_)
         if (!c->swap_multi(true, lv, stream_)) return -1;

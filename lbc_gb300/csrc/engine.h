@@ -11,6 +11,7 @@
 
 #include "kernels.h"
 #include "lbm_device.cuh"
+#include "near_plan.h"
 
 namespace lbm {
 
@@ -114,13 +115,9 @@ struct StepGraph {
 // Most probes a solver records (one block of a record launch walks them).
 constexpr int kMaxProbes = 4096;
 
-// A case's nodes near special ones in passes of several steps (near_plan).
-struct NearPlan {
-    int lv = 0;
-    std::vector<uint32_t> deep;
-    std::vector<std::vector<int4>> segs;
-    long long near_pairs = 0;
-};
+// Steps that runs ask for before a case or a batch is set up for passes of several
+// steps: KMULTI
+constexpr int kMultiOwed = 64;
 // Rows of a warp's task in a batch's pass (64 ducts: 126 us per step with 32, 122
 // with 64, 120.7 with 96 and 128).
 constexpr int kTaskRows = 96;
@@ -269,6 +266,8 @@ class Solver {
     }
     bool wide() const { return 9LL * plane_ >= (1LL << 31); }  // element offsets need 64 bits
     size_t multi_bytes() const { return 9 * (size_t)plane_ * esize_; }  // of one of its buffers
+    // Bytes that passes of lv steps take beside what the case holds.
+    size_t multi_need(int lv) const;
     const NearPlan &near_plan(int lv) const;
     bool multi_buffers(int lv);
     bool swap_multi(bool enter, int lv, cudaStream_t s);
@@ -302,6 +301,7 @@ class Solver {
     bool beside(cudaStream_t s);
     bool join(cudaStream_t s);
     int multi_warps() const;
+    bool multi_shape(int lv);
     bool multi_setup();
     bool launch_multi(int cur, int other, int lv);
     bool capture_multi(StepGraph &g);
@@ -362,7 +362,8 @@ class Solver {
     bool capturing_ = false;
     cudaEvent_t beside_ev_ = nullptr;
     mutable NearPlan near_plan_;
-    int multi_state_ = 0;                 // 0: not tried, 1: set up, -1: not for this case
+    int multi_state_ = 0;                 // 0: not set up, 1: set up, -1: not for this case
+    int multi_owed_ = 0;                  // steps that runs asked for without passes
     uint32_t *d_deep_ = nullptr;
     int4 *d_near_segs_[4] = {nullptr, nullptr, nullptr, nullptr};
     int near_segs_[4] = {0, 0, 0, 0};
@@ -445,6 +446,7 @@ class Batch {
     float tuned_us_ = 0.f;
     bool launch_batched(int sel);
     bool capture_pair();
+    bool multi_shape() const;
     bool multi_setup();
     bool upload_multi();
     bool launch_multi(int a);
@@ -484,6 +486,7 @@ class Batch {
     int owed_ = 0;  // steps that runs asked for without it
     std::vector<void *> allocs_;
     // passes of several steps (multi_setup)
+    int multi_owed_ = 0;
     int multi_state_ = 0, multi_lv_ = 4, ntasks_ = 0, nmsegs_[4] = {0, 0, 0, 0};
     uint32_t *d_mdeep_ = nullptr;
     MultiTask *d_mtasks_ = nullptr;
