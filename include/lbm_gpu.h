@@ -197,9 +197,11 @@ long long lbm_gpu_write_impedance_trace(lbm_gpu_solver *s, int entry, const char
 int lbm_gpu_msd_zoh(double R, double m, double K, double *A, double *b);
 
 int lbm_gpu_get_info(lbm_gpu_solver *s, lbm_gpu_info *info);
-/* The kernels this solver's runs have launched so far (those of replayed graphs
- * included), and the time steps one pass over the populations takes in a long
- * run (1, 2 or 4). */
+/* The kernels this solver's own runs have launched so far (those of replayed
+ * graphs included; steps taken in a batch or by the drop-in are not counted), and
+ * the time steps one pass over the populations takes in a long run of the case as
+ * it stands (1, 2 or 4: 1 also where its geometry or the memory left refuses
+ * passes). */
 int lbm_gpu_launch_stats(lbm_gpu_solver *s, long long *launches, int *steps_per_pass);
 /* Thread-block shape of the fused step (bx * by <= 256, bx multiple of 32).
  * No result depends on it: populations, fields and the momentum-exchange force

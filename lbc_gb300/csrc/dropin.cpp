@@ -916,7 +916,7 @@ int lbm_gpu_msd_zoh(double R, double m, double K, double *A, double *b) {
 int lbm_gpu_launch_stats(lbm_gpu_solver *s, long long *launches, int *steps_per_pass) {
     SOLVER_OR_FAIL(s);
     if (launches) *launches = s->s->launches();
-    if (steps_per_pass) *steps_per_pass = std::max(1, s->s->multi_levels());
+    if (steps_per_pass) *steps_per_pass = s->s->steps_per_pass();
     return LBM_GPU_OK;
 }
 

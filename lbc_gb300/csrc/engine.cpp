@@ -1535,6 +1535,16 @@ bool Solver::multi_shape(int lv) {
     return n >= (1LL << 21) || 16 * near_plan(lv).near_pairs <= n * lv;
 }
 
+// Steps per pass of a long run of this case as it stands.
+int Solver::steps_per_pass() {
+    const int lv = multi_levels();
+    if (lv == 0 || multi_state_ < 0) return 1;
+    if (!has_flags_ || multi_state_ > 0) return lv;
+    size_t freeb = 0, total = 0;
+    const bool room = cudaMemGetInfo(&freeb, &total) == cudaSuccess && freeb / 4 >= multi_need(lv);
+    return room && multi_shape(lv) ? lv : 1;
+}
+
 size_t Solver::multi_need(int lv) const {
     size_t need = 0;
     for (int b = 2; b < (lv > 2 ? 4 : 3); b++) need += buf_[b] ? 0 : multi_bytes();

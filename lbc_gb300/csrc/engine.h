@@ -260,6 +260,7 @@ class Solver {
     bool end_steps(cudaStream_t s);
     // Passes of several steps, for a case alone and in a batch.
     int multi_levels() const;
+    int steps_per_pass();
     bool multi_case() const {
         return d_.store != STORE_F64 && !d_omega_ && rec_host_.empty() && one_group_ && d_.Nx >= 8 && d_.Ny >= 8 &&
                !wide() && (long long)special_host_.size() <= (long long)d_.Nx * d_.Ny / 8;

@@ -78,3 +78,31 @@ def test_batch_first_steps_are_taken_one_at_a_time():
         got, want = x.get_state(), y.get_state()
         for fld in FIELDS:
             assert same(getattr(got, fld), getattr(want, fld)), fld
+
+
+def _stage_periodic():
+    # a periodic entry behind another: it reads the opposite edge after the collision
+    case, st = cases.cylinder_golden(33)[:2]
+    case.bcs = [b for b in case.bcs if not b.name.startswith("periodic")] + [cases.BC("periodic_y", 0, None, None)]
+    return case, st
+
+
+def _porous():
+    import numpy as np
+    case, st = cases.taylor_green(1200, 1000)
+    case.solid_mask[::6, ::6] = 1  # more than an eighth of the nodes beside a solid one
+    return case, st
+
+
+@pytest.mark.parametrize("name,storage,want", [
+    ("cavity", "f32", 4), ("periodic", "f32", 4), ("cavity", "f64", 1), ("edge_periodic", "f32", 1), ("porous", "f32", 1)])
+def test_launch_stats_reports_the_passes_taken(name, storage, want):
+    from lbc_gb300 import GpuSolver, STORAGE
+    case, st = {"cavity": lambda: cases.cavity_moving_wall(1500, 0.1, 300.0), "periodic": lambda: cases.taylor_green(1200, 1000),
+                "edge_periodic": _stage_periodic, "porous": _porous}[name]()
+    s = GpuSolver(case, STORAGE[storage])
+    s.set_state(st)
+    assert case.nodes >= 1 << 20 and s.launch_stats()[1] == want
+    s.run(200)
+    assert s.launch_stats()[1] == want
+    s.close()
