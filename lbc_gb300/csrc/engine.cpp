@@ -1494,14 +1494,27 @@ const NearPlan &Solver::near_plan(int lv) const {
     return near_plan_;
 }
 
-bool Solver::multi_buffers(int lv) {
+// s: the stream that uses them first (the case's or a batch's).
+bool Solver::multi_buffers(int lv, cudaStream_t s) {
     for (int b = 2; b < (lv > 2 ? 4 : 3); b++) {
         if (buf_[b]) continue;
-        char *q = nullptr;
-        if (!dalloc(&q, multi_bytes())) return false;
+        void *q = nullptr;
+        if (!device_alloc(&q, multi_bytes(), s)) return false;
+        allocs_.push_back(q);
+        dev_bytes_ += multi_bytes();
         buf_[b] = q;
     }
     return true;
+}
+
+// Steps that runs ask of a case with walls before it is set up for passes: what its
+// plan, buffers, stream and graph cost (0.45 ms and more) in steps of what passes
+// gain. us per step one at a time and in passes: cavity 1024^2 10.3 and 10.3,
+// channel 2048 x 256 7.7 and 6.5; cavity 1450^2 27.1 and 17.5; 2048^2 49.0 and 26.2
+// (set-up 1 ms), 4096^2 184 and 87 (2.3 ms).
+int Solver::multi_due() const {
+    const long long n = (long long)d_.Nx * d_.Ny;
+    return n < (5LL << 18) ? 1024 : n < (1LL << 22) ? 192 : 96;
 }
 
 // multi_swap before a run of passes (enter) and after it.
@@ -1568,7 +1581,7 @@ bool Solver::multi_setup() {
                            cudaMemcpyHostToDevice, stream_));
         near_segs_[q] = (int)plan.segs[q].size();
     }
-    if (!multi_buffers(lv)) return false;
+    if (!multi_buffers(lv, stream_)) return false;
     int lo = 0, hi = 0;
     cudaDeviceGetStreamPriorityRange(&lo, &hi);
     CK(cudaStreamCreateWithPriority(&multi_stream_, cudaStreamNonBlocking, lo));
@@ -1643,8 +1656,9 @@ int Solver::run_multi(int avail) {
     if (has_flags_) {
         if (avail < 8 * lv) return 0;
         if (multi_state_ == 0) {
-            multi_owed_ = std::min(multi_owed_ + std::min(avail, kMultiOwed), kMultiOwed);
-            if (multi_owed_ < kMultiOwed) return 0;
+            const int due = multi_due();
+            multi_owed_ = std::min(multi_owed_ + std::min(avail, due), due);
+            if (multi_owed_ < due) return 0;
         }
         if (!multi_setup()) return 0;
     }
@@ -2154,6 +2168,14 @@ bool Batch::multi_shape() const {
     return true;
 }
 
+// As Solver::multi_due: 64 ducts, 8 ms and 61 us per step. Cases that have been in
+// a batch of passes keep their plans and buffers: 2 ms.
+int Batch::multi_due() const {
+    for (const Solver *c : cases_)
+        if (c->multi_need(multi_lv_) > 0) return 160;
+    return 64;
+}
+
 bool Batch::multi_setup() {
     if (multi_state_) return multi_state_ > 0;
     multi_state_ = -1;
@@ -2185,8 +2207,15 @@ bool Batch::multi_setup() {
     // M (14 % of the node steps near) 103 -> 81, 3.2 M 50-57 either way, below
     // that slower: four list launches bound a pass.
     if (near > nodes_ * lv / 5) return false;
-    for (Solver *c : cases_)  // (allocated on the case's stream, used on this one)
-        if (!c->multi_buffers(lv) || !check_cuda(cudaStreamSynchronize(c->stream()), "multi_buffers")) return false;
+    // The pool serves a stream quickly from what that stream has freed and with a
+    // look at every other stream for each block otherwise: one block of the whole
+    // size, given back at once, makes the cases' blocks its pieces (128 buffers of
+    // 64 ducts 26 ms without it, 2 with).
+    void *all = nullptr;
+    if (need > 0 && cudaMallocAsync(&all, need, stream_) == cudaSuccess) cudaFreeAsync(all, stream_);
+    else cudaGetLastError();
+    for (Solver *c : cases_)
+        if (!c->multi_buffers(lv, stream_)) return false;
     const int nc = (int)cases_.size(), ne = max_stages_ ? stage_counts_[0] : 0;
     if (!balloc(allocs_, &d_mdeep_, deep.size(), stream_) || !balloc(allocs_, &d_mtasks_, tasks.size(), stream_) ||
         !balloc(allocs_, &d_msp_, (size_t)nc * (2 * lv + 2), stream_) || !balloc(allocs_, &d_mfin_, (size_t)nc * 2 * lv, stream_) ||
@@ -2273,10 +2302,7 @@ int Batch::run_multi(int pairs) {
     const int lv = multi_lv_;
     if (forces_ || pairs < 4 * lv) return 0;
     if (multi_state_ == 0) {
-        // Cases that have been in a batch of passes keep their plans and buffers.
-        bool fresh = false;
-        for (const Solver *c : cases_) fresh = fresh || c->multi_need(lv) > 0;
-        const int due = fresh ? kMultiOwed : 8 * lv;
+        const int due = multi_due();
         multi_owed_ = std::min(multi_owed_ + 2 * std::min(pairs, due), due);
         if (multi_owed_ < due) return 0;
     }

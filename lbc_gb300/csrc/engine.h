@@ -115,9 +115,6 @@ struct StepGraph {
 // Most probes a solver records (one block of a record launch walks them).
 constexpr int kMaxProbes = 4096;
 
-// Steps that runs ask for before a case or a batch is set up for passes of several
-// steps: KMULTI
-constexpr int kMultiOwed = 64;
 // Rows of a warp's task in a batch's pass (64 ducts: 126 us per step with 32, 122
 // with 64, 120.7 with 96 and 128).
 constexpr int kTaskRows = 96;
@@ -270,7 +267,8 @@ class Solver {
     // Bytes that passes of lv steps take beside what the case holds.
     size_t multi_need(int lv) const;
     const NearPlan &near_plan(int lv) const;
-    bool multi_buffers(int lv);
+    bool multi_buffers(int lv, cudaStream_t s);
+    int multi_due() const;
     bool swap_multi(bool enter, int lv, cudaStream_t s);
     StepParams near_params(int cur, int other, int lv, int q) const;
     // The buffer of the near nodes' state after q steps of a pass.
@@ -448,6 +446,7 @@ class Batch {
     bool launch_batched(int sel);
     bool capture_pair();
     bool multi_shape() const;
+    int multi_due() const;
     bool multi_setup();
     bool upload_multi();
     bool launch_multi(int a);

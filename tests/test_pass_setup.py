@@ -1,6 +1,7 @@
-"""When a case with walls is set up for passes of several steps: not in the first
+"""When a case with walls is set up for passes of several steps: not for the first
 few steps asked of it, which would not pay for its plan, buffers and graph, but
-after them, in one run or in several; and what lbm_gpu_launch_stats says of it."""
+after them, in one run or in several; what lbm_gpu_launch_stats says of it; and
+every kind of wall and edge in runs long enough to take the passes."""
 import pytest
 
 from conftest import same
@@ -34,7 +35,8 @@ def test_first_steps_are_taken_one_at_a_time():
     assert _launches(s, 400) <= 1.4 * 400
     s.close()
     s = _cavity()
-    for _ in range(4):
+    assert _launches(s, 34) >= 2 * 33
+    for _ in range(5):
         s.run(34)
     assert _launches(s, 34) <= 1.6 * 34
     s.close()
@@ -67,13 +69,13 @@ def test_batch_first_steps_are_taken_one_at_a_time():
         return out
 
     together, alone = solvers(), solvers()
-    for runs in ((40, 90, 200), (60,)):
+    for runs in ((40, 90, 200), (80,)):
         b = GpuBatch(together)
         for n in runs:
             b.run(n)
         b.close()
     for x, y in zip(together, alone):
-        for _ in range(390):
+        for _ in range(410):
             y.run(1)
         got, want = x.get_state(), y.get_state()
         for fld in FIELDS:
@@ -106,3 +108,99 @@ def test_launch_stats_reports_the_passes_taken(name, storage, want):
     s.run(200)
     assert s.launch_stats()[1] == want
     s.close()
+
+
+# (nodes from 2^18 on with 1024 steps asked for, from 1.3 M with 192)
+LONG = [("box_one_omega", "f32", 1060), ("boxblock_one_omega", "f32", 1060), ("blocks", "f32", 1060), ("duct", "f32", 1060), ("open_large", "f32", 1060),
+        ("golden_large", "f32", 1060), ("wake4", "f32", 230), ("wake4", "f16", 230), ("cavity4", "f32", 230), ("cavity_f16", "f16", 230)]
+
+
+@pytest.mark.parametrize("hist", [False, True])
+@pytest.mark.parametrize("name,storage,first", LONG)
+def test_walls_and_edges_in_long_runs(name, storage, first, hist):
+    """As test_multi_step's cases: passes entered and left twice, against single steps."""
+    import numpy as np
+    from lbc_gb300 import GpuSolver, STORAGE, impedance as imp
+    from test_multi_step import _walls
+    duct = None
+    if name == "open_large":
+        case, st = cases.cylinder_wake(1500, 760, D=40.0, xc=300.0, yc=200.0, u_max=0.05, Re=60.0)
+        case.solid_mask[0] = case.solid_mask[-1] = 0
+    elif name.endswith("_one_omega"):  # several groups of edges
+        (case, st), _ = _walls(name[:-10])
+        case.omega_eff[:] = 1 / 0.8
+    elif name == "golden_large":
+        case, st = cases.cylinder_golden(33)[:2]
+        st = cases.random_state(case, 7)
+    elif name == "cavity_f16":
+        case, st = cases.cavity_moving_wall(1690, 0.1, 300.0)
+    else:
+        (case, st), duct = _walls(name)
+        st = st if duct else cases.random_state(case, 7)
+    if hist and (duct is not None or not case.solid_mask.any()):
+        pytest.skip("no force to record")
+    pair = []
+    for _ in range(2):
+        s = GpuSolver(case, STORAGE[storage])
+        if duct is not None:
+            s.set_impedance_wall(imp.LINER_ENTRY, *imp.liner_arrays(duct), imp.TRACKED_OMEGAS, 1.0, imp.MEAN_RATE, 500)
+        if hist:
+            s.enable_force_history(1200)
+        s.set_state(st)
+        pair.append(s)
+    a, b = pair
+    assert a.launch_stats()[1] > 1
+    for n in (first, 2, 91):
+        a.run(n)
+    for _ in range(first + 93):
+        b.run(1)
+    assert a.launch_stats()[0] < 0.8 * b.launch_stats()[0]
+    x, y = a.get_state(), b.get_state()
+    assert np.isfinite(x.rho[case.solid_mask == 0]).all()
+    for fld in FIELDS:
+        assert same(getattr(x, fld), getattr(y, fld)), fld
+    assert a.forces() == b.forces()
+    if hist:
+        assert np.array_equal(a.force_history(1200), b.force_history(1200))
+    if duct is not None:
+        for p, q in zip(a.impedance_readback(imp.LINER_ENTRY), b.impedance_readback(imp.LINER_ENTRY)):
+            assert np.array_equal(p, q)
+    a.close()
+    b.close()
+
+
+@pytest.mark.parametrize("name", ["ducts", "mix"])
+def test_batch_passes_in_long_runs(name):
+    """As test_multi_step's batches: passes taken in the first and the second run."""
+    import numpy as np
+    from lbc_gb300 import F32_SHIFTED, GpuBatch, GpuSolver, impedance as imp
+    from test_multi_step import _batch_cases
+    built = _batch_cases(name)
+
+    def solvers():
+        out = []
+        for (case, st), duct in built:
+            s = GpuSolver(case, F32_SHIFTED)
+            if duct is not None:
+                s.set_impedance_wall(imp.LINER_ENTRY, *imp.liner_arrays(duct), imp.TRACKED_OMEGAS, 1.0, imp.MEAN_RATE, 500)
+            s.set_state(st)
+            out.append(s)
+        return out
+
+    together, alone = solvers(), solvers()
+    held = sum(s.info().device_bytes for s in together)
+    b = GpuBatch(together)
+    b.run(170)
+    assert sum(s.info().device_bytes for s in together) > 1.2 * held  # the buffers of passes
+    b.run(38)
+    for n, (x, y, (_, duct)) in enumerate(zip(together, alone, built)):
+        for _ in range(208):
+            y.run(1)
+        got, want = x.get_state(), y.get_state()
+        for fld in FIELDS:
+            assert same(getattr(got, fld), getattr(want, fld)), (n, fld)
+        assert same(np.array(x.forces()), np.array(y.forces()))
+        if duct is not None:
+            for p, q in zip(x.impedance_readback(imp.LINER_ENTRY), y.impedance_readback(imp.LINER_ENTRY)):
+                assert np.array_equal(p, q)
+    b.close()
