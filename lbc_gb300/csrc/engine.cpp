@@ -1447,8 +1447,8 @@ void Solver::set_autotune(int mode) {
 // 512^2 4.01, 3.34, 3.88; 1024 x 768 6.43, 6.42, 5.65; 1024^2 8.21, 7.98, 6.75;
 // 2048^2 46.4, 31.6, 20.3; 4096^2 173.5, 111.5, 71.4: small grids have too few
 // warps to hide the dependent collisions of a row. FP16's one-step kernel moves
-// half the bytes: 1500 x 1100 11.1 against 12.0 with four levels, 2048^2 31.0
-// against 24.6, 4096^2 112.5 against 80.4.
+// half the bytes: 1500 x 1100 11.1 against 12.0 with four levels, 4096^2 112.5
+// against 80.4.
 int Solver::multi_levels() const {
     const long long n = (long long)d_.Nx * d_.Ny;
     if (d_.store == STORE_F64 || d_omega_ || !rec_host_.empty()) return 0;
@@ -1457,15 +1457,33 @@ int Solver::multi_levels() const {
     // step at a time, 8.9 in passes; 120 x 4000 7.9 and 5.8).
     if (n < (1LL << 22) && (d_.Nx + 55) / 56 * 320 > 8 * d_.Nx) return 0;
     // With a flag word the nodes near walls and edges go step by step beside the
-    // pass, a chain of launches that bounds small grids. FP32: cylinder 1024 x
-    // 256 8.30 against 7.78 with two levels and 8.00 with four, 2048 x 512 10.9,
-    // 10.2, 10.2; cavity 1024^2 10.6, 9.85, 9.07, 2048^2 49.1, 35.7, 25.4, 4096^2
-    // 184, 131, 85. FP16: cavity 1024^2 9.6, 10.5, 9.6, 2048^2 34.2, 27.7, 26.5;
-    // channel 3000 x 750 21.0, 20.2, 22.3.
-    if (has_flags_ && d_.store == STORE_F16) return n < (1LL << 21) ? 0 : n < (3LL << 20) ? 2 : 4;
-    if (has_flags_) return n < (1LL << 18) ? 0 : n < (1LL << 20) ? 2 : 4;
-    if (d_.store == STORE_F16) return n >= (1LL << 21) ? 4 : 0;
-    return n < (1LL << 18) ? 0 : n < (1LL << 19) ? 2 : 4;
+    // pass, a chain of launches that bounds small grids, more so with cut links
+    // and moving walls. FP32 without them: channel 2048 x 128 5.44 against 4.65,
+    // 2048 x 256 7.68 and 6.52, 2048 x 512 12.7 and 11.9. With: cavity 520^2 6.69
+    // and 6.89, 724^2 7.2 and 8.0, 1024^2 10.3 and 10.3, 1150^2 14.3 and 12.0,
+    // 2048^2 49.0 and 26.2, 2900^2 94 and 45; cylinder 1024 x 256 7.70 and 7.49,
+    // 1500 x 375 8.48 and 8.31, 2048 x 512 10.55 and 10.35, 3000 x 750 28.0 and
+    // 19.4: below 2^20 nodes the few per cent do not return the set-up.
+    int lv = 0;
+    if (d_.store == STORE_F16) lv = n < (2LL << 20) ? 0 : has_flags_ && n < (3LL << 20) ? 2 : 4;
+    else if (has_flags_) lv = n < (has_links_ ? (1LL << 20) : (1LL << 18)) ? 0 : n < (1LL << 20) ? 2 : 4;
+    else lv = n < (1LL << 18) ? 0 : n < (1LL << 19) ? 2 : 4;
+    // Where the strips leave more lanes idle than the one-step kernel's blocks do,
+    // passes pay on larger grids only. FP32 128 columns wide (share 0.76): 0.42 M
+    // nodes 4.44 against 5.16, 1.1 M 8.4 and 9.5 (channel 12.9 and 18.8), 1.6 M 15.3
+    // and 12.3 (20.6 and 23.4), 2.2 M 28.9 and 27.3; 256 and 512 (0.91): 0.58 M 5.2
+    // and 5.57, 1.1 M 8.5 and 8.2 (13.6 and 15.2), 1.6 M 15.6 and 10.4 (21.1 and
+    // 20.5). FP16 256 (0.91): 3.1 M 22.2 and 25.0, 4.2 M 29.8 and 30.7; 1024 and more
+    // (0.96): 2.2 M 14.6 and 15.3-16.5, 3.1 M 22.3 and 20.0-22.7, 4.2 M 30.1 and
+    // 24.4-26.2; 100 (1.14): 2.2 M 20.4 and 18.3; with walls cavity 2.1 M 15.9 and
+    // 16.4, 2.9 M 24.4 and 21.9.
+    const double share = lv ? lane_share(64 - 2 * multi_halo(lv)) : 1.0;
+    if (d_.store == STORE_F16) {
+        if (share < 1.1 && n < (share < 0.95 ? (5LL << 20) : has_flags_ ? (5LL << 19) : (7LL << 19))) return 0;
+    } else if (lv == 2 ? share < 0.8 : share < 0.95 && n < (share < 0.8 ? (2LL << 20) : (5LL << 18))) {
+        return 0;
+    }
+    return lv;
 }
 
 // Warps a pass is split into: 8 per SM while the state is in the L2 cache
@@ -2189,6 +2207,15 @@ bool Batch::multi_setup() {
     std::vector<MultiTask> tasks;
     long long near = 0;
     const int halo = multi_halo(lv), width = 64 - 2 * halo;
+    long long strip_rows = 0;
+    double wanted = 0, walked = 0;  // lanes of the one-step kernel's blocks and of the strips
+    for (const Solver *c : cases_) {
+        strip_rows += (long long)((c->Nx() + width - 1) / width) * c->Ny();
+        walked += (double)c->Nx() * c->Ny();
+        wanted += (double)c->Nx() * c->Ny() * c->lane_share(width);
+    }
+    const double share = wanted / walked;
+    const int rows = (int)std::min<long long>(kTaskRows, std::max<long long>(24, strip_rows / (launch::sm_count() * 12)));
     for (size_t c = 0; c < cases_.size(); c++) {
         const NearPlan &plan = cases_[c]->near_plan(lv);
         near += 2 * plan.near_pairs;
@@ -2196,8 +2223,10 @@ bool Batch::multi_setup() {
             for (int4 e : plan.segs[q]) segs[q].push_back(make_int4((int)c, e.y, e.z, e.w));
         // Chunks of about kTaskRows rows: enough tasks to even out cases of
         // different height, few enough rows walked twice (2 (lv - 1) per chunk).
+        // Fewer where that leaves warps of the chip without one (16 channels of 512^2
+        // 67.2 -> 59.6 us per step, 65 vortices of 512 x 128 42.3 -> 31.5).
         const int Nx = cases_[c]->Nx(), Ny = cases_[c]->Ny(), strips = (Nx + width - 1) / width;
-        const int chunks = std::max(1, (Ny + kTaskRows / 2) / kTaskRows), h = (Ny + chunks - 1) / chunks;
+        const int chunks = std::max(1, (Ny + rows / 2) / rows), h = (Ny + chunks - 1) / chunks;
         for (int y = 0; y < Ny; y += h)
             for (int st = 0; st < strips; st++)
                 tasks.push_back(MultiTask{(int)c, st, y, std::min(Ny, y + h), (long long)deep.size()});
@@ -2205,8 +2234,17 @@ bool Batch::multi_setup() {
     }
     // Measured, one step at a time against passes: 13.5 M nodes 198 -> 125 us, 6.7
     // M (14 % of the node steps near) 103 -> 81, 3.2 M 50-57 either way, below
-    // that slower: four list launches bound a pass.
-    if (near > nodes_ * lv / 5) return false;
+    // that slower: four list launches bound a pass. 65 channels of 1024 x 64 (16 %)
+    // 66.2 and 69.1 us, 137 of them 139 and 125. Idle lanes (lane_share) count as
+    // for a case alone: 65 channels of 128 x 512 (0.76, 2 % near) 67 and 77 us, 512
+    // x 128 (0.91, 8 %) 66 and 69, 137 of them 137 and 152; 256 x 256 (0.91, 4 %) 67
+    // and 64, 137 of them 136 and 122; 137 vortices of 128 x 512 122 and 72. FP16: 16
+    // channels of 1024^2 159 and 148, 61 of 256 x 1024 176 and 191, eight of 1024^2
+    // 88 and 90.
+    const long long near_steps = 100 * near, steps = nodes_ * lv;
+    if (near_steps > steps * (nodes_ < (1LL << 23) ? 15 : 20)) return false;
+    if (near > 0 && share < 0.93 && (share < 0.9 || near_steps > 6 * steps)) return false;
+    if (near > 0 && store_ == STORE_F16 && (share < 0.95 || nodes_ < (15LL << 20))) return false;
     // The pool serves a stream quickly from what that stream has freed and with a
     // look at every other stream for each block otherwise: one block of the whole
     // size, given back at once, makes the cases' blocks its pieces (128 buffers of

@@ -258,6 +258,11 @@ class Solver {
     // Passes of several steps, for a case alone and in a batch.
     int multi_levels() const;
     int steps_per_pass();
+    // Lanes that step a node of the case in a pass whose strips keep `width` columns,
+    // against the one-step kernel's blocks of 128.
+    double lane_share(int width) const {
+        return (double)((d_.Nx + 127) / 128 * 128) / ((d_.Nx + width - 1) / width * width);
+    }
     bool multi_case() const {
         return d_.store != STORE_F64 && !d_omega_ && rec_host_.empty() && one_group_ && d_.Nx >= 8 && d_.Ny >= 8 &&
                !wide() && (long long)special_host_.size() <= (long long)d_.Nx * d_.Ny / 8;

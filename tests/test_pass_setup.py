@@ -204,3 +204,19 @@ def test_batch_passes_in_long_runs(name):
             for p, q in zip(x.impedance_readback(imp.LINER_ENTRY), y.impedance_readback(imp.LINER_ENTRY)):
                 assert np.array_equal(p, q)
     b.close()
+
+
+@pytest.mark.parametrize("storage,kind,nx,ny,want", [
+    ("f32", "vortex", 128, 4505, 1), ("f32", "vortex", 512, 1126, 1), ("f32", "vortex", 2048, 281, 4), ("f32", "vortex", 256, 1638, 2),
+    ("f32", "vortex", 128, 3276, 1), ("f32", "vortex", 256, 6144, 4), ("f32", "vortex", 100, 5767, 4), ("f32", "channel", 256, 2252, 2),
+    ("f32", "channel", 512, 2150, 1), ("f32", "cavity", 724, 724, 1), ("f16", "vortex", 256, 8601, 1), ("f16", "vortex", 1024, 2150, 1),
+    ("f16", "vortex", 4096, 1024, 4), ("f16", "cavity", 1450, 1450, 1)])
+def test_shapes_that_leave_lanes_idle(storage, kind, nx, ny, want):
+    """Passes only where their strips fill about as many lanes as the one-step
+    kernel's blocks, or the grid is large enough not to mind."""
+    from lbc_gb300 import GpuSolver, STORAGE
+    case = {"vortex": lambda: cases.taylor_green(nx, ny), "channel": lambda: cases.poiseuille(nx, ny, 0.8, 1e-6),
+            "cavity": lambda: cases.cavity_moving_wall(nx, 0.1, 300.0)}[kind]()[0]
+    s = GpuSolver(case, STORAGE[storage])
+    assert s.launch_stats()[1] == want
+    s.close()
