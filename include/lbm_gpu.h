@@ -270,8 +270,10 @@ int lbm_gpu_batch_destroy(lbm_gpu_batch *b);
  * lbm_gpu_server_set_reserve) and less the requests taken but not set up yet:
  * memory that anything else takes after the server starts holds admissions
  * back. budget_bytes > 0 also caps the estimated bytes of the active requests
- * (0: no cap). When nothing is active one request is let in regardless, so a
- * request larger than the memory left runs alone or fails cleanly. */
+ * (0: no cap), the further buffers of passes of several steps included: a batch
+ * without room for those steps one at a time. When nothing is active one request
+ * is let in regardless, so a request larger than the memory left runs alone or
+ * fails cleanly. */
 typedef struct lbm_gpu_server lbm_gpu_server;
 int lbm_gpu_server_create(size_t budget_bytes, int max_active, int chunk_steps, lbm_gpu_server **out);
 /* Returns the request id (> 0) or a negative code. f = f_new = NULL: the

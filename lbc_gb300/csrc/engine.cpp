@@ -60,6 +60,24 @@ void use_retaining_pool() {
     cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
 }
 
+size_t device_available() {
+    size_t fr = 0, tot = 0, slack = 0;
+    if (cudaMemGetInfo(&fr, &tot) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    int dev = 0;
+    cudaMemPool_t pool;
+    if (cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetDefaultMemPool(&pool, dev) == cudaSuccess) {
+        unsigned long long reserved = 0, used = 0;  // cuuint64_t
+        if (cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved) == cudaSuccess &&
+            cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) == cudaSuccess && reserved > used)
+            slack = (size_t)(reserved - used);
+    }
+    cudaGetLastError();
+    return fr + slack;
+}
+
 bool device_alloc(void **q, size_t bytes, cudaStream_t s) {
     return check_cuda(cudaMallocAsync(q, bytes, s), "cudaMallocAsync");
 }
@@ -1571,9 +1589,7 @@ int Solver::steps_per_pass() {
     const int lv = multi_levels();
     if (lv == 0 || multi_state_ < 0) return 1;
     if (!has_flags_ || multi_state_ > 0) return lv;
-    size_t freeb = 0, total = 0;
-    const bool room = cudaMemGetInfo(&freeb, &total) == cudaSuccess && freeb / 4 >= multi_need(lv);
-    return room && multi_shape(lv) ? lv : 1;
+    return device_available() / 4 >= multi_need(lv) && multi_shape(lv) ? lv : 1;
 }
 
 size_t Solver::multi_need(int lv) const {
@@ -1582,14 +1598,17 @@ size_t Solver::multi_need(int lv) const {
     return need;
 }
 
-// Sets a case alone up for passes; false: not this case.
+// Sets a case alone up for passes; false: not this case, or not enough memory now.
 bool Solver::multi_setup() {
     if (multi_state_) return multi_state_ > 0;
-    multi_state_ = -1;
     const int lv = multi_levels();
-    if (!multi_shape(lv)) return false;
-    size_t freeb = 0, total = 0;
-    if (cudaMemGetInfo(&freeb, &total) != cudaSuccess || freeb / 4 < multi_need(lv)) return false;
+    const bool shape = multi_shape(lv);
+    if (shape && device_available() / 4 < multi_need(lv)) {
+        multi_owed_ = 0;  // asked again after as many steps
+        return false;
+    }
+    multi_state_ = -1;
+    if (!shape) return false;
     const NearPlan &plan = near_plan(lv);
     if (!dalloc(&d_deep_, plan.deep.size())) return false;
     CK(cudaMemcpyAsync(d_deep_, plan.deep.data(), plan.deep.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, stream_));
@@ -2194,14 +2213,24 @@ int Batch::multi_due() const {
     return 64;
 }
 
+size_t Batch::multi_need() const {
+    size_t need = 0;
+    if (multi_state_ == 0 && multi_shape())
+        for (const Solver *c : cases_) need += c->multi_need(multi_lv_);
+    return need;
+}
+
 bool Batch::multi_setup() {
     if (multi_state_) return multi_state_ > 0;
-    multi_state_ = -1;
     const int lv = multi_lv_;
-    if (!multi_shape()) return false;
-    size_t need = 0, freeb = 0, total = 0;
-    for (const Solver *c : cases_) need += c->multi_need(lv);
-    if (cudaMemGetInfo(&freeb, &total) != cudaSuccess || freeb / 4 < need) return false;
+    const bool shape = multi_shape();
+    const size_t need = multi_need();
+    if (shape && (need > pass_limit_ || device_available() / 4 < need)) {
+        multi_owed_ = 0;
+        return false;
+    }
+    multi_state_ = -1;
+    if (!shape) return false;
     std::vector<uint32_t> deep;
     std::vector<std::vector<int4>> segs(lv);
     std::vector<MultiTask> tasks;

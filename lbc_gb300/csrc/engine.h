@@ -21,6 +21,8 @@ bool check_cuda(cudaError_t e, const char *what);
 // Stream-ordered device allocation from the device's default pool (set up to
 // retain freed memory), freed with cudaFreeAsync on the owner's stream.
 bool device_alloc(void **q, size_t bytes, cudaStream_t s);
+// Device memory that can be had now: free, and held unused by the pool.
+size_t device_available();
 void use_retaining_pool();
 
 // Rows of lbc's FP64 AoS arrays (72 B per node) that set_state / get_state
@@ -269,8 +271,10 @@ class Solver {
     }
     bool wide() const { return 9LL * plane_ >= (1LL << 31); }  // element offsets need 64 bits
     size_t multi_bytes() const { return 9 * (size_t)plane_ * esize_; }  // of one of its buffers
-    // Bytes that passes of lv steps take beside what the case holds.
+    // Bytes that passes of lv steps take beside what the case holds, and those that
+    // it holds for them.
     size_t multi_need(int lv) const;
+    size_t multi_held() const { return ((buf_[2] ? 1 : 0) + (buf_[3] ? 1 : 0)) * multi_bytes(); }
     const NearPlan &near_plan(int lv) const;
     bool multi_buffers(int lv, cudaStream_t s);
     int multi_due() const;
@@ -434,6 +438,10 @@ class Batch {
     bool tuned() const { return tuned_; }
     float tuned_us() const { return tuned_us_; }
     std::string tune_key() const;
+    // Bytes that setting its cases up for passes of several steps would take, and a
+    // limit on them for the next runs (above it the steps are taken one at a time).
+    size_t multi_need() const;
+    void limit_passes(size_t bytes) { pass_limit_ = bytes; }
 
   private:
     bool build();
@@ -492,6 +500,7 @@ class Batch {
     std::vector<void *> allocs_;
     // passes of several steps (multi_setup)
     int multi_owed_ = 0;
+    size_t pass_limit_ = ~(size_t)0;
     int multi_state_ = 0, multi_lv_ = 4, ntasks_ = 0, nmsegs_[4] = {0, 0, 0, 0};
     uint32_t *d_mdeep_ = nullptr;
     MultiTask *d_mtasks_ = nullptr;

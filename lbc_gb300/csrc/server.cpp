@@ -70,7 +70,8 @@ struct Request {
     ImpSpec imp;
     std::vector<double> spectra;
     std::unique_ptr<Solver> solver;
-    size_t est_bytes = 0;
+    size_t est_bytes = 0;   // pass_bytes included
+    size_t pass_bytes = 0;  // held for passes of several steps
     double t_submit = 0, t_admit = 0, t_done = 0;
     std::string error;
 };
@@ -205,28 +206,11 @@ static bool retire(Request *r) {
     return okk;
 }
 
-// Device memory a new request may take now: the device's free memory plus
-// what the stream-ordered pool holds unused (freed by retired requests and
-// kept for reuse), less the reserve. Read live, so memory taken by anything
-// else in or outside this process after the server started holds admissions
-// back.
-static size_t device_available(const lbm_gpu_server *S) {
-    size_t fr = 0, tot = 0;
-    if (cudaMemGetInfo(&fr, &tot) != cudaSuccess) {
-        cudaGetLastError();
-        return 0;
-    }
-    size_t slack = 0;
-    int dev = 0;
-    cudaMemPool_t pool;
-    if (cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetDefaultMemPool(&pool, dev) == cudaSuccess) {
-        unsigned long long reserved = 0, used = 0;  // cuuint64_t
-        if (cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved) == cudaSuccess &&
-            cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) == cudaSuccess && reserved > used)
-            slack = (size_t)(reserved - used);
-    }
-    cudaGetLastError();
-    const size_t have = fr + slack;
+// Device memory a new request may take now: what can be had (device_available)
+// less the reserve. Read live, so memory taken by anything else in or outside
+// this process after the server started holds admissions back.
+static size_t available_less_reserve(const lbm_gpu_server *S) {
+    const size_t have = device_available();
     return have > S->reserve ? have - S->reserve : 0;
 }
 
@@ -242,7 +226,7 @@ static size_t device_available(const lbm_gpu_server *S) {
 // behind them.
 static std::vector<Request *> take_admissions(lbm_gpu_server *S, Lane &L) {
     std::vector<Request *> out;
-    const size_t avail = device_available(S);
+    const size_t avail = available_less_reserve(S);
     std::lock_guard<std::mutex> lk(S->mu);
     int cap = S->max_active;
     if (L.storage == LBM_GPU_F64 || L.storage == LBM_GPU_F64_FMA) {
@@ -300,8 +284,26 @@ static int lane_round(lbm_gpu_server *S, Lane &L) {
             L.batch_ids = ids;
             t_b = now_s() - tb;
         }
+        // Passes of several steps take further buffers per case: only within the
+        // budget, and counted while the request is active.
+        size_t granted = 0;
+        if (L.batch->ok()) {
+            const size_t need = L.batch->multi_need();
+            std::lock_guard<std::mutex> lk(S->mu);
+            if (S->budget == 0 || S->in_use + need <= S->budget) granted = need;
+            S->in_use += granted;
+        }
+        L.batch->limit_passes(granted);
         okk = L.batch->ok() && L.batch->run(n);
         launched = true;
+        std::lock_guard<std::mutex> lk(S->mu);
+        S->in_use -= granted;
+        for (Request *r : L.active) {
+            const size_t more = r->solver->multi_held() - r->pass_bytes;
+            r->pass_bytes += more;
+            r->est_bytes += more;
+            S->in_use += more;
+        }
     }
     // Admissions overlap the chunk on the device.
     const double t_adm0 = now_s();
@@ -598,7 +600,7 @@ int lbm_gpu_server_available(lbm_gpu_server *S, size_t *bytes) {
         set_error("bad arguments");
         return LBM_GPU_ERR_ARG;
     }
-    const size_t a = device_available(S);
+    const size_t a = available_less_reserve(S);
     std::lock_guard<std::mutex> lk(S->mu);
     *bytes = a > S->pending ? a - S->pending : 0;
     return LBM_GPU_OK;
