@@ -33,10 +33,12 @@ __device__ __forceinline__ void pdl_launch_dependents() {
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // Launch k<<<g, b, 0, s>>>(args...), with programmatic stream serialization
-// when after_bulk is set (the previous kernel in s is a bulk step kernel).
+// when after_bulk is set (the previous kernel in s is a bulk step kernel). Blocks
+// are one deep (v_mul_alone in shifted_math.cuh counts on it).
 template <typename... K, typename... A>
 inline cudaError_t launch_follower(bool after_bulk, void (*k)(K...), dim3 g, dim3 b, cudaStream_t s,
                                    A &&...args) {
+    if (b.z != 1) return cudaErrorInvalidConfiguration;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = g;
     cfg.blockDim = b;
