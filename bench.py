@@ -495,7 +495,7 @@ def run_ours(a, ws, rank, pg):
                      "vs_serial_fp64": round(mlups / ser_mlups, 2),
                      "stream": f"{len(stream)} requests, rate {a.serve_rate * ws}/s, steps x{a.serve_scale} "
                                "of U_log[5000, 50000], 80/20 FP32-shifted/FP64",
-                     "fp64_requests": ("FP64 storage, fused multiply-add step (within 1e-12 of lbc)"
+                     "fp64_requests": ("F64_FMA storage (lbc's results to rounding; with lbc's weights its bits)"
                                        if a.serve_f64 == "fma" else "FP64 storage, lbc's arithmetic bit for bit")}
     clocks = clk.stop()
     res["f16"] = {"mlups": ws * N * a.steps / (ms16 / 1e3) / 1e6, "ms_per_step": ms16 / a.steps,

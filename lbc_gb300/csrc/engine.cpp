@@ -737,7 +737,7 @@ bool Solver::dropin_step_direct(double *f, double *f_new, double *rho, double *u
     CK(launch::collide_aos_exact(c, stream_));
     // Old content of f_new is needed only where the step leaves it: at solid
     // nodes and in slots whose source is off the grid, so only flagged nodes
-    // cross the link (1000 x 400 cylinder: 734 -> 600 us per call without the
+    // cross the link (1000 x 400 cylinder: 770 -> 614 us per call without the
     // other nodes' 29 MB).
     if (needs_old_dst_) {
         if (!d_old_nodes_) {

@@ -10,11 +10,12 @@
 // 64-bit fixed point, its round-to-nearest-even included, and a product of two
 // 53-bit mantissas about twenty. In this form a force-free node takes 24 FP64
 // instructions (the relaxation's product and the final additions, u.u and the
-// diagonal velocities) beside 1040 ALU and 580 multiply-add instructions:
-// 72.8 us per step, 14.4 GLUPS, with the FP64 pipe 57 % and the ALU 77 % busy,
+// diagonal velocities) beside 1020 ALU and 580 multiply-add instructions:
+// 71.5 us per step, 14.7 GLUPS, with the FP64 pipe 57 % and the ALU 77 % busy,
 // so that neither alone bounds it. (80 registers, three blocks of 256 threads
-// or six of 128 per SM: 64 registers 74.5 us, 99 registers 77.2. Additions
-// moved to the multiply-add pipe by hand, as multiplications by 1: 81.6.)
+// or six of 128 per SM; in an earlier form of 72.8 us 64 registers took 74.5, 99
+// registers 77.2, and additions moved to the multiply-add pipe by hand, as
+// multiplications by 1, 81.6.)
 //
 // Nothing is approximated: every operation returns the FP64 result that
 // moments_exact / collide_exact round to. The fixed-point forms hold for the

@@ -307,7 +307,7 @@ __device__ __forceinline__ void stage_dispatch(const StageParams &p, const Finis
 //
 // When the whole Boundary list is one group, an entry's thread pulls the node
 // that its BC reads itself and needs nothing of the bulk kernel's step
-// (near_shifted in kernels_shifted.cu does the same). The edge launch then goes
+// (near_shifted in kernels_near.cu does the same). The edge launch then goes
 // first and the bulk kernel runs beside it: a BC and its finish are a chain of
 // a few hundred FP64 instructions, 64 cycles each, which the bulk kernel's
 // blocks hide. Cylinder 1024 x 256 41.1 -> 26.7 us per step, 1000 x 400 with
