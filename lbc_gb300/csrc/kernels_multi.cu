@@ -77,9 +77,9 @@ template <> struct PairOf<__half> {
 // Collides two nodes and returns their populations as stored.
 template <typename T, bool FORCE>
 __device__ __forceinline__ void collide_pair(const FastStepParams &fp, float2 g[9], typename PairOf<T>::P out[9]) {
-    float2 dr, ux, uy, Jx, Jy, jx, jy;
-    moments_v<float2>(g, v_splat<float2>(fp.hFxf), v_splat<float2>(fp.hFyf), dr, ux, uy, Jx, Jy, jx, jy);
-    collide_v<float2, FORCE>(g, fp.wf, fp.h1f, fp.h5f, dr, ux, uy, Jx, Jy, jx, jy, v_splat<float2>(fp.omega0f),
+    float2 dr, u8x, u8y, Jx, Jy, jx, jy;
+    moments_v<float2>(g, v_splat<float2>(fp.hFxf), v_splat<float2>(fp.hFyf), dr, u8x, u8y, Jx, Jy, jx, jy);
+    collide_v<float2, FORCE>(g, fp.wf, fp.h1f, fp.h5f, dr, u8x, u8y, Jx, Jy, jx, jy, v_splat<float2>(fp.omega0f),
                              fp.s.has_force != 0, fp.Fxf, fp.Fyf);
 #pragma unroll
     for (int k = 0; k < 9; k++) out[k] = PairOf<T>::pack(g[k]);

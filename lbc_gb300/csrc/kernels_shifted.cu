@@ -191,14 +191,14 @@ __global__ void k_collide_shifted(const CollideParams p) {
 #pragma unroll
     for (int k = 0; k < 9; k++) { g[k] = SV<T>::ld_plain(F + k * p.plane + node); wf[k] = (float)p.w[k]; }
     const float om = p.omega ? (float)p.omega[dn] : (float)p.omega0;
-    float dr, ux, uy, Jx, Jy, jx, jy;
+    float dr, u8x, u8y, Jx, Jy, jx, jy;
     if (p.from_pops) {
-        moments_shifted(g, (float)(0.5 * p.Fx), (float)(0.5 * p.Fy), dr, ux, uy, Jx, Jy, jx, jy);
+        moments_shifted(g, (float)(0.5 * p.Fx), (float)(0.5 * p.Fy), dr, u8x, u8y, Jx, Jy, jx, jy);
     } else {
         // the stored fields: rho, u = (j + F/2) / rho
         dr = (float)(p.rho[dn] - 1.0);
-        ux = (float)p.ux[dn];
-        uy = (float)p.uy[dn];
+        u8x = 8.0f * (float)p.ux[dn];
+        u8y = 8.0f * (float)p.uy[dn];
         Jx = (float)(p.rho[dn] * p.ux[dn]);
         Jy = (float)(p.rho[dn] * p.uy[dn]);
         jx = (float)(p.rho[dn] * p.ux[dn] - 0.5 * p.Fx);
@@ -206,9 +206,9 @@ __global__ void k_collide_shifted(const CollideParams p) {
     }
     float h1, h5;
     shifted_h(wf[1], h1, h5);
-    if (p.has_force) collide_v<float, true>(g, wf, h1, h5, dr, ux, uy, Jx, Jy, jx, jy, om, true, (float)p.Fx,
+    if (p.has_force) collide_v<float, true>(g, wf, h1, h5, dr, u8x, u8y, Jx, Jy, jx, jy, om, true, (float)p.Fx,
                                             (float)p.Fy);
-    else collide_v<float, false>(g, wf, h1, h5, dr, ux, uy, Jx, Jy, jx, jy, om, false, 0.f, 0.f);
+    else collide_v<float, false>(g, wf, h1, h5, dr, u8x, u8y, Jx, Jy, jx, jy, om, false, 0.f, 0.f);
 #pragma unroll
     for (int k = 0; k < 9; k++) SV<T>::st(F + k * p.plane + node, g[k]);
 }

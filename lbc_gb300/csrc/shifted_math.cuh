@@ -97,18 +97,17 @@ template <class V> __device__ __forceinline__ V v_splat(float x);
 template <> __device__ __forceinline__ float v_splat<float>(float x) { return x; }
 template <> __device__ __forceinline__ float2 v_splat<float2>(float x) { return make_float2(x, x); }
 
-// 1/rho, rho = 1 + dr with lbc's floor (compute_macroscopic_fields.c:27), rounded
-// as __frcp_rn rounds it: the hardware's estimate and one Newton step (that
-// intrinsic has a branch, which keeps the compiler from interleaving the steps of
-// kernels_multi.cu). The estimate is of rho / 8, so that it is a normal number for
-// every finite density and 0 for an infinite one, and an eighth of it takes the
-// Newton step. Above 2^126, where 1/rho is subnormal, within 2^-149. NaN stays NaN.
-template <class V> __device__ __forceinline__ V inv_density(V dr) {
+// 8/rho, rho = 1 + dr with lbc's floor (compute_macroscopic_fields.c:27): an
+// eighth of it is 1/rho as __frcp_rn rounds it. The hardware's estimate of the
+// reciprocal and one Newton step (that intrinsic has a branch, which keeps the
+// compiler from interleaving the steps of kernels_multi.cu), both on rho / 8, whose
+// reciprocal is a normal number for every finite density; 0 for an infinite one.
+// NaN stays NaN.
+template <class V> __device__ __forceinline__ V eight_over_density(V dr) {
     const V eighth = v_splat<V>(0.125f);
     const V a = v_max_nan(v_fma(dr, eighth, eighth), v_splat<V>(0.125f * 1e-16f));
-    const V r = v_rcp_seed(a), s = v_mul(r, eighth);
-    const V e = v_fma(v_neg(v_min_nan(a, v_splat<V>(0x1p125f))), r, v_splat<V>(1.0f));
-    return v_fma(s, e, s);
+    const V r = v_rcp_seed(a);
+    return v_fma(r, v_fma(v_neg(v_min_nan(a, v_splat<V>(0x1p125f))), r, v_splat<V>(1.0f)), r);
 }
 
 // h1 = fl(3 w1), h5 = (1 - 2 h1) / 4, as the host computes them.
@@ -118,30 +117,32 @@ __device__ __forceinline__ void shifted_h(float w1, float &h1, float &h5) {
 }
 
 // Shifted moments: delta rho = sum g, j = sum c g (sum c w = 0). Jx, Jy are the
-// momentum including half the body force (rho u of lbc); jx, jy without it.
+// momentum including half the body force (rho u of lbc); jx, jy without it. u8x,
+// u8y: eight times the velocity (eight_over_density); the factor goes into the
+// constants of collide_v, and powers of two change no bits.
 template <class V>
-__device__ __forceinline__ void moments_v(const V g[9], V hFx, V hFy, V &dr, V &ux, V &uy, V &Jx, V &Jy, V &jx,
+__device__ __forceinline__ void moments_v(const V g[9], V hFx, V hFy, V &dr, V &u8x, V &u8y, V &Jx, V &Jy, V &jx,
                                           V &jy) {
     dr = v_add(v_add(v_add(v_add(g[0], g[1]), v_add(g[2], g[3])), v_add(v_add(g[4], g[5]), v_add(g[6], g[7]))),
                g[8]);
     jx = v_add(v_add(v_sub(g[1], g[3]), v_sub(g[5], g[6])), v_sub(g[8], g[7]));
     jy = v_sub(v_add(v_sub(g[2], g[4]), v_add(g[5], g[6])), v_add(g[7], g[8]));
-    const V inv = inv_density(dr);
+    const V inv8 = eight_over_density(dr);
     Jx = v_add(jx, hFx);
     Jy = v_add(jy, hFy);
-    ux = v_mul_alone(Jx, inv);
-    uy = v_mul_alone(Jy, inv);
+    u8x = v_mul_alone(Jx, inv8);
+    u8y = v_mul_alone(Jy, inv8);
 }
 
-// One pair of directions (k, opposite) of the equilibrium: X = w (dr + 4.5 J c
+// One pair of directions (k, opposite) of the equilibrium (c8: 8 c.u): X = w (dr + 4.5 J c
 // - rt) is the even part, h o the odd part, added to X with one rounding
 // (X +- h o as FMAs: rounding h o first doubles the FP32 velocity error of a
 // Taylor-Green run against FP64). The odd part takes the momentum without
 // the half force, o = c.j; the force enters the odd part separately (see
 // collide_v).
 template <class V>
-__device__ __forceinline__ void geq_pair(float w, float h, V dr, V c, V J, V o, V nrt, V &a, V &b) {
-    const V X = v_mul(v_splat<V>(w), v_add(dr, v_fma(v_mul(v_splat<V>(4.5f), J), c, nrt)));
+__device__ __forceinline__ void geq_pair(float w, float h, V dr, V c8, V J, V o, V nrt, V &a, V &b) {
+    const V X = v_mul(v_splat<V>(w), v_add(dr, v_fma(v_mul(v_splat<V>(4.5f / 8), J), c8, nrt)));
     a = v_fma(v_splat<V>(h), o, X);
     b = v_fma(v_splat<V>(-h), o, X);
 }
@@ -164,9 +165,9 @@ __device__ __forceinline__ void geq_pair(float w, float h, V dr, V c, V J, V o, 
 // a single rounding. Channel 256 x 64 against FP64 after 20,000 steps: u L2
 // error 5.0e-7 (6.6e-5 before).
 template <class V, bool FORCE>
-__device__ __forceinline__ void collide_v(V g[9], const float w[9], float h1, float h5, V dr, V ux, V uy,
+__device__ __forceinline__ void collide_v(V g[9], const float w[9], float h1, float h5, V dr, V u8x, V u8y,
                                           V Jx, V Jy, V jx, V jy, V om, bool force, float Fx, float Fy) {
-    const V nrt = v_mul(v_splat<V>(-1.5f), v_fma(Jx, ux, v_mul(Jy, uy)));  // -rho * 1.5 u.u
+    const V nrt = v_mul(v_splat<V>(-1.5f / 8), v_fma(Jx, u8x, v_mul(Jy, u8y)));  // -rho * 1.5 u.u
     // Without a body force j = J exactly: one set of momenta stays live.
     const bool forced = FORCE && force;
     if (!FORCE) {
@@ -174,10 +175,10 @@ __device__ __forceinline__ void collide_v(V g[9], const float w[9], float h1, fl
         jy = Jy;
     }
     V geq[9];
-    geq_pair(w[1], h1, dr, ux, Jx, jx, nrt, geq[1], geq[3]);
-    geq_pair(w[2], h1, dr, uy, Jy, jy, nrt, geq[2], geq[4]);
-    geq_pair(w[5], h5, dr, v_add(ux, uy), v_add(Jx, Jy), v_add(jx, jy), nrt, geq[5], geq[7]);
-    geq_pair(w[6], h5, dr, v_sub(uy, ux), v_sub(Jy, Jx), v_sub(jy, jx), nrt, geq[6], geq[8]);
+    geq_pair(w[1], h1, dr, u8x, Jx, jx, nrt, geq[1], geq[3]);
+    geq_pair(w[2], h1, dr, u8y, Jy, jy, nrt, geq[2], geq[4]);
+    geq_pair(w[5], h5, dr, v_add(u8x, u8y), v_add(Jx, Jy), v_add(jx, jy), nrt, geq[5], geq[7]);
+    geq_pair(w[6], h5, dr, v_sub(u8y, u8x), v_sub(Jy, Jx), v_sub(jy, jx), nrt, geq[6], geq[8]);
     geq[0] = v_sub(dr, v_add(v_add(v_add(geq[1], geq[3]), v_add(geq[2], geq[4])),
                              v_add(v_add(geq[5], geq[7]), v_add(geq[6], geq[8]))));
     if (!forced) {
@@ -190,16 +191,16 @@ __device__ __forceinline__ void collide_v(V g[9], const float w[9], float h1, fl
     }
     const V Fxv = v_splat<V>(Fx), Fyv = v_splat<V>(Fy);
     const V gf = v_fma(v_splat<V>(-0.5f), om, v_splat<V>(1.0f));
-    const V n3uF = v_mul(v_splat<V>(-3.0f), v_fma(ux, Fxv, v_mul(uy, Fyv)));  // -3 u.F
+    const V n3uF = v_mul(v_splat<V>(-3.0f / 8), v_fma(u8x, Fxv, v_mul(u8y, Fyv)));  // -3 u.F
     g[0] = v_add(g[0], v_fma(om, v_sub(geq[0], g[0]), v_mul(gf, v_mul(v_splat<V>(w[0]), n3uF))));
-    const V cu[4] = {ux, uy, v_add(ux, uy), v_sub(uy, ux)};
+    const V c8u[4] = {u8x, u8y, v_add(u8x, u8y), v_sub(u8y, u8x)};
     const float cFs[4] = {Fx, Fy, Fx + Fy, Fy - Fx};
     const float hs[4] = {h1, h1, h5, h5};
     const int ka[4] = {1, 2, 5, 6}, kb[4] = {3, 4, 7, 8};
 #pragma unroll
     for (int q = 0; q < 4; q++) {
         const V cF = v_splat<V>(cFs[q]);
-        const V S = v_fma(v_mul(v_splat<V>(9.0f), cu[q]), cF, n3uF);
+        const V S = v_fma(v_mul(v_splat<V>(9.0f / 8), c8u[q]), cF, n3uF);
         const V E = v_mul_alone(gf, v_mul(v_splat<V>(w[ka[q]]), S));
         const V O = v_splat<V>(hs[q] * cFs[q]);
         const int a = ka[q], b = kb[q];

@@ -10,8 +10,8 @@ namespace lbm {
 
 // Scalar entry points used by the per-node paths.
 __device__ __forceinline__ void moments_shifted(const float g[9], float hFx, float hFy, float &dr,
-                                                float &ux, float &uy, float &Jx, float &Jy, float &jx, float &jy) {
-    moments_v<float>(g, hFx, hFy, dr, ux, uy, Jx, Jy, jx, jy);
+                                                float &u8x, float &u8y, float &Jx, float &Jy, float &jx, float &jy) {
+    moments_v<float>(g, hFx, hFy, dr, u8x, u8y, Jx, Jy, jx, jy);
 }
 
 // Rare per-node outputs, kept out of line so the compiler cannot hoist their
@@ -180,12 +180,12 @@ __device__ __forceinline__ void step_node_shifted(const FastStepParams &fp, int 
         for (int k = 0; k < 9; k++) p.bandg[(size_t)k * p.nslots + slot] = g[k];
     }
     if (FLAGS && (fl & NF_BCW)) return;
-    float dr, ux, uy, Jx, Jy, jx, jy;
-    moments_v<float>(g, fp.hFxf, fp.hFyf, dr, ux, uy, Jx, Jy, jx, jy);
-    if (p.write_macro || slot >= 0) macro_store(p, dn, slot, dr, ux, uy);
+    float dr, u8x, u8y, Jx, Jy, jx, jy;
+    moments_v<float>(g, fp.hFxf, fp.hFyf, dr, u8x, u8y, Jx, Jy, jx, jy);
+    if (p.write_macro || slot >= 0) macro_store(p, dn, slot, dr, 0.125f * u8x, 0.125f * u8y);
     if (COLLIDE) {
         const float om = p.omega ? (float)p.omega[dn] : fp.omega0f;
-        collide_v<float, FORCE>(g, fp.wf, fp.h1f, fp.h5f, dr, ux, uy, Jx, Jy, jx, jy, om, p.has_force != 0,
+        collide_v<float, FORCE>(g, fp.wf, fp.h1f, fp.h5f, dr, u8x, u8y, Jx, Jy, jx, jy, om, p.has_force != 0,
                                 fp.Fxf, fp.Fyf);
     }
 #pragma unroll
@@ -229,13 +229,14 @@ __device__ __forceinline__ void collide_store_pair_shifted(const FastStepParams 
     T *Dst = (T *)p.dst;
     const I pl = (I)p.plane;
     const I r0 = (I)j * (I)p.pitch + (I)i0;
-    float2 dr, ux, uy, Jx, Jy, jx, jy;
-    moments_v<float2>(g, v_splat<float2>(fp.hFxf), v_splat<float2>(fp.hFyf), dr, ux, uy, Jx, Jy, jx, jy);
+    float2 dr, u8x, u8y, Jx, Jy, jx, jy;
+    moments_v<float2>(g, v_splat<float2>(fp.hFxf), v_splat<float2>(fp.hFyf), dr, u8x, u8y, Jx, Jy, jx, jy);
     const size_t dn = (size_t)j * (size_t)p.Nx + (size_t)i0;
-    if (p.write_macro) macro_store_pair(p, dn, dr, ux, uy);
+    if (p.write_macro)
+        macro_store_pair(p, dn, dr, make_float2(0.125f * u8x.x, 0.125f * u8x.y), make_float2(0.125f * u8y.x, 0.125f * u8y.y));
     if (COLLIDE) {
         const float2 om = p.omega ? omega_pair(p.omega, dn) : v_splat<float2>(fp.omega0f);
-        collide_v<float2, FORCE>(g, fp.wf, fp.h1f, fp.h5f, dr, ux, uy, Jx, Jy, jx, jy, om, p.has_force != 0,
+        collide_v<float2, FORCE>(g, fp.wf, fp.h1f, fp.h5f, dr, u8x, u8y, Jx, Jy, jx, jy, om, p.has_force != 0,
                                  fp.Fxf, fp.Fyf);
     }
 #pragma unroll
@@ -252,9 +253,10 @@ __device__ __forceinline__ void finish_pops_shifted(const FinishParams &p, int2 
         g[k] = SV<T>::rnd(f[k]);
         wf[k] = p.wf[k];
     }
-    float dr, ux, uy, Jx, Jy, jx, jy;
-    moments_shifted(g, p.hFxf, p.hFyf, dr, ux, uy, Jx, Jy, jx, jy);
+    float dr, u8x, u8y, Jx, Jy, jx, jy;
+    moments_shifted(g, p.hFxf, p.hFyf, dr, u8x, u8y, Jx, Jy, jx, jy);
     const size_t dn = (size_t)ij.y * p.Nx + ij.x;
+    const float ux = 0.125f * u8x, uy = 0.125f * u8y;
     if (p.write_macro) { p.rho[dn] = 1.0 + (double)dr; p.ux[dn] = ux; p.uy[dn] = uy; }
     p.bandm_next[slot] = 1.0 + (double)dr;
     p.bandm_next[(size_t)p.nslots + slot] = ux;
@@ -263,8 +265,8 @@ __device__ __forceinline__ void finish_pops_shifted(const FinishParams &p, int2 
         const float om = p.omega ? (float)p.omega[dn] : p.omega0f;
         float h1, h5;
         shifted_h(wf[1], h1, h5);
-        if (p.has_force) collide_v<float, true>(g, wf, h1, h5, dr, ux, uy, Jx, Jy, jx, jy, om, true, p.Fxf, p.Fyf);
-        else collide_v<float, false>(g, wf, h1, h5, dr, ux, uy, Jx, Jy, jx, jy, om, false, 0.f, 0.f);
+        if (p.has_force) collide_v<float, true>(g, wf, h1, h5, dr, u8x, u8y, Jx, Jy, jx, jy, om, true, p.Fxf, p.Fyf);
+        else collide_v<float, false>(g, wf, h1, h5, dr, u8x, u8y, Jx, Jy, jx, jy, om, false, 0.f, 0.f);
     }
     T *D = (T *)p.dst;
     const long long node = (long long)ij.y * p.pitch + ij.x;
