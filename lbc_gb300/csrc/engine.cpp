@@ -1475,16 +1475,19 @@ int Solver::multi_levels() const {
     // step at a time, 8.9 in passes; 120 x 4000 7.9 and 5.8).
     if (n < (1LL << 22) && (d_.Nx + 55) / 56 * 320 > 8 * d_.Nx) return 0;
     // With a flag word the nodes near walls and edges go step by step beside the
-    // pass, a chain of launches that bounds small grids, more so with cut links
-    // and moving walls. FP32 without them: channel 2048 x 128 5.44 against 4.65,
-    // 2048 x 256 7.68 and 6.52, 2048 x 512 12.7 and 11.9. With: cavity 520^2 6.69
-    // and 6.89, 724^2 7.2 and 8.0, 1024^2 10.3 and 10.3, 1150^2 14.3 and 12.0,
-    // 2048^2 49.0 and 26.2, 2900^2 94 and 45; cylinder 1024 x 256 7.70 and 7.49,
-    // 1500 x 375 8.48 and 8.31, 2048 x 512 10.55 and 10.35, 3000 x 750 28.0 and
-    // 19.4: below 2^20 nodes the few per cent do not return the set-up.
+    // pass, a chain of launches that bounds small grids, more so with edges, cut
+    // links or moving walls. FP32 without them: channel 2048 x 128 5.44 against 4.65,
+    // 2048 x 256 7.68 and 6.52, 2048 x 512 12.7 and 11.9. With edges: liner duct 1400
+    // x 200 6.69 and 7.21, 2048 x 400 8.59 and 8.86, 4000 x 270 10.7 and 9.6; lid
+    // 533^2 4.73 and 4.91, 746^2 6.54 and 7.23, 1050^2 11.1 and 11.0. With links:
+    // cylinder 1068 x 267 7.71 and 7.23, 1492 x 373 8.24 and 8.29, 1832 x 458 9.01 and
+    // 9.57, 2100 x 525 11.1 and 10.5; cavity 533^2 6.69 and 6.61, 746^2 7.42 and 7.51,
+    // 916^2 8.77 and 9.38, 1050^2 11.2 and 10.9, 1168^2 15.5 and 12.0.
+    const bool edges = has_links_ || !groups_.empty();
     int lv = 0;
     if (d_.store == STORE_F16) lv = n < (2LL << 20) ? 0 : has_flags_ && n < (3LL << 20) ? 2 : 4;
-    else if (has_flags_) lv = n < (has_links_ ? (1LL << 20) : (1LL << 18)) ? 0 : n < (1LL << 20) ? 2 : 4;
+    else if (edges && n < (1LL << 20)) lv = has_links_ && n >= (1LL << 18) && n < (7LL << 16) ? 2 : 0;
+    else if (has_flags_) lv = n < (1LL << 18) ? 0 : n < (1LL << 20) ? 2 : 4;
     else lv = n < (1LL << 18) ? 0 : n < (1LL << 19) ? 2 : 4;
     // Where the strips leave more lanes idle than the one-step kernel's blocks do,
     // passes pay on larger grids only. FP32 128 columns wide (share 0.76): 0.42 M

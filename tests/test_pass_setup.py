@@ -110,9 +110,10 @@ def test_launch_stats_reports_the_passes_taken(name, storage, want):
     s.close()
 
 
-# (nodes from 2^18 on with 1024 steps asked for, from 1.3 M with 192)
-LONG = [("box_one_omega", "f32", 1060), ("boxblock_one_omega", "f32", 1060), ("blocks", "f32", 1060), ("duct", "f32", 1060), ("open_large", "f32", 1060),
-        ("golden_large", "f32", 1060), ("wake4", "f32", 230), ("wake4", "f16", 230), ("cavity4", "f32", 230), ("cavity_f16", "f16", 230)]
+# (with 1024 steps asked for below 1.3 M nodes, with 192 above)
+LONG = [(n, "f32", 1060) for n in ("wake", "cavity", "golden", "open", "blocks", "box_large", "boxblock_large", "duct_large",
+                                   "open_large", "golden_large")]
+LONG += [("wake4", "f32", 230), ("wake4", "f16", 230), ("cavity4", "f32", 230), ("cavity_f16", "f16", 230)]
 
 
 @pytest.mark.parametrize("hist", [False, True])
@@ -123,20 +124,26 @@ def test_walls_and_edges_in_long_runs(name, storage, first, hist):
     from lbc_gb300 import GpuSolver, STORAGE, impedance as imp
     from test_multi_step import _walls
     duct = None
-    if name == "open_large":
-        case, st = cases.cylinder_wake(1500, 760, D=40.0, xc=300.0, yc=200.0, u_max=0.05, Re=60.0)
+    if name.startswith("open"):
+        case, st = cases.cylinder_wake(*((1500, 760) if name == "open_large" else (900, 400)), D=40.0, xc=300.0, yc=200.0,
+                                       u_max=0.05, Re=60.0)
         case.solid_mask[0] = case.solid_mask[-1] = 0
-    elif name.endswith("_one_omega"):  # several groups of edges
-        (case, st), _ = _walls(name[:-10])
+    elif name in ("box_large", "boxblock_large"):  # several groups of edges
+        case, st = cases.all_regularized_box(1210, 900)
         case.omega_eff[:] = 1 / 0.8
+        if name == "boxblock_large":
+            case.solid_mask[200:240, 300:360] = 1
+    elif name == "duct_large":
+        duct = imp.LinerParams(2100, 520, 0.2, 1.0 * imp.CS, 5e-3, 0.05)
+        case, st = imp.liner_duct(duct)
     elif name == "golden_large":
         case, st = cases.cylinder_golden(33)[:2]
         st = cases.random_state(case, 7)
     elif name == "cavity_f16":
         case, st = cases.cavity_moving_wall(1690, 0.1, 300.0)
     else:
-        (case, st), duct = _walls(name)
-        st = st if duct else cases.random_state(case, 7)
+        (case, st), _ = _walls(name)
+        st = cases.random_state(case, 7)
     if hist and (duct is not None or not case.solid_mask.any()):
         pytest.skip("no force to record")
     pair = []
@@ -209,14 +216,16 @@ def test_batch_passes_in_long_runs(name):
 @pytest.mark.parametrize("storage,kind,nx,ny,want", [
     ("f32", "vortex", 128, 4505, 1), ("f32", "vortex", 512, 1126, 1), ("f32", "vortex", 2048, 281, 4), ("f32", "vortex", 256, 1638, 2),
     ("f32", "vortex", 128, 3276, 1), ("f32", "vortex", 256, 6144, 4), ("f32", "vortex", 100, 5767, 4), ("f32", "channel", 256, 2252, 2),
-    ("f32", "channel", 512, 2150, 1), ("f32", "cavity", 724, 724, 1), ("f16", "vortex", 256, 8601, 1), ("f16", "vortex", 1024, 2150, 1),
+    ("f32", "channel", 512, 2150, 1), ("f32", "cavity", 724, 724, 1), ("f32", "cavity", 533, 533, 2), ("f32", "lid", 533, 533, 1),
+    ("f32", "lid", 1050, 1050, 4), ("f32", "cylinder", 1068, 267, 2), ("f32", "cylinder", 1492, 373, 1), ("f16", "vortex", 256, 8601, 1), ("f16", "vortex", 1024, 2150, 1),
     ("f16", "vortex", 4096, 1024, 4), ("f16", "cavity", 1450, 1450, 1)])
 def test_shapes_that_leave_lanes_idle(storage, kind, nx, ny, want):
     """Passes only where their strips fill about as many lanes as the one-step
     kernel's blocks, or the grid is large enough not to mind."""
     from lbc_gb300 import GpuSolver, STORAGE
     case = {"vortex": lambda: cases.taylor_green(nx, ny), "channel": lambda: cases.poiseuille(nx, ny, 0.8, 1e-6),
-            "cavity": lambda: cases.cavity_moving_wall(nx, 0.1, 300.0)}[kind]()[0]
+            "cavity": lambda: cases.cavity_moving_wall(nx, 0.1, 300.0), "lid": lambda: cases.cavity_zouhe(nx, 0.1, 300.0),
+            "cylinder": lambda: cases.cylinder_wake(nx, ny, D=ny / 8, xc=nx / 4, yc=ny / 2)}[kind]()[0]
     s = GpuSolver(case, STORAGE[storage])
     assert s.launch_stats()[1] == want
     s.close()
